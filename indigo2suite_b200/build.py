@@ -20,7 +20,13 @@ LIB = PKG / "libi2b200.so"
 
 SOURCES = [
     "engine.cu",
-    "resident.cu",
+    "relax_bfs.cu",
+    "relax_sssp.cu",
+    "relax_cc.cu",
+    "relax_mis.cu",
+    "resident_bfs.cu",
+    "resident_sssp.cu",
+    "resident_cc.cu",
     "selector.cu",
     "batch.cu",
     "gen_device.cu",

@@ -8,7 +8,7 @@
 // mode (I2_LOOP_GRAPH) the whole sequence is one CUDA graph whose WHILE
 // conditional node holds one cooperative relax launch that runs every
 // iteration itself, its blocks meeting at a bounded barrier between
-// iterations (relax_resident, resident.cu). I2_LOOP_RELAUNCH keeps one launch
+// iterations (relax_resident, relax.cuh). I2_LOOP_RELAUNCH keeps one launch
 // per iteration inside the graph: the fixed style's kernel, or the dispatch
 // kernel whose blocks branch on the style picked for this iteration. Either
 // way the last block of an iteration picks the next style and sets the loop
@@ -337,40 +337,30 @@ __global__ void k_cc_labels(const int* __restrict__ copy_label, const int* __res
 // ---------------------------------------------------------------------------
 // Kernel tables.
 
-typedef void (*KernelFn)(Ctx);
-
-template <int ALG>
-static KernelFn relax_fn(int v) {
-  switch (v) {
-    case kVPThread: return relax_push<ALG, kVPThread>;
-    case kVPWarp: return relax_push<ALG, kVPWarp>;
-    case kVPCta: return relax_edge_balanced<ALG>;
-    case kVPBlock: return relax_push<ALG, kVPBlock>;
-    case kPullFrontier: return relax_pull<ALG, true>;
-    case kPullTopo: return relax_pull<ALG, false>;
-    case kEdgeTopo: return relax_edge_topo<ALG>;
-    case kPushTopo: return relax_push_topo<ALG>;
-    case kUnionFind:
-      if constexpr (ALG == kCC) return relax_union<ALG>;
-      return nullptr;
-  }
-  return nullptr;
-}
-
 // The selectors' per-iteration kernel; `wide`: the form compiled for the fixed
 // styles' resident blocks per SM (graphs of kWideSelectorNodes vertices or more).
 static KernelFn dispatch_kernel(int algo, bool wide) {
-  if (algo == kBFS) return wide ? relax_dispatch<kBFS, I2_EB_MIN_BLOCKS> : relax_dispatch<kBFS>;
-  if (algo == kSSSP) return wide ? relax_dispatch<kSSSP, I2_EB_MIN_BLOCKS> : relax_dispatch<kSSSP>;
-  return wide ? relax_dispatch<kCC, I2_EB_MIN_BLOCKS> : relax_dispatch<kCC>;  // MIS never dispatches
+  if (algo == kBFS) return dispatch_fn<kBFS>(wide);
+  if (algo == kSSSP) return dispatch_fn<kSSSP>(wide);
+  return dispatch_fn<kCC>(wide);  // MIS never dispatches
 }
 
 KernelFn relax_kernel(int algo, int v, bool near_far) {
-  if (near_far && algo == kSSSP && v == kVPCta) return relax_near_far;
+  if (near_far && algo == kSSSP && v == kVPCta) return near_far_kernel(false);
   if (algo == kBFS) return relax_fn<kBFS>(v);
   if (algo == kSSSP) return relax_fn<kSSSP>(v);
   if (algo == kCC) return relax_fn<kCC>(v);
-  return relax_mis;  // one style
+  return mis_kernel(false);  // one style
+}
+
+// Kernel of a resident traversal: fixed style v (mode 0) or the per-iteration
+// pick (v < 0; `wide`: the form compiled for more resident blocks).
+static KernelFn resident_kernel(int algo, int v, bool near_far, bool wide) {
+  if (algo == kMIS) return mis_kernel(true);  // one style
+  if (near_far && algo == kSSSP && v == kVPCta) return near_far_kernel(true);
+  if (algo == kBFS) return resident_fn<kBFS>(v, wide);
+  if (algo == kSSSP) return resident_fn<kSSSP>(v, wide);
+  return resident_fn<kCC>(v, wide);
 }
 
 static KernelFn fill_kernel(int algo) {

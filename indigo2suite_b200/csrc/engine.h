@@ -10,11 +10,20 @@ typedef void (*KernelFn)(Ctx);
 
 int cuda_status(cudaError_t e);
 int grid_for(KernelFn fn, int max_per_sm);
-KernelFn relax_kernel(int algo, int variant, bool near_far = false);
-// Resident traversal kernel: fixed style `variant`, or the per-iteration pick
-// when variant < 0, in the form compiled for more resident blocks when `wide`
-// (resident.cu).
-KernelFn resident_kernel(int algo, int variant, bool near_far, bool wide = false);
+// Relax kernels of one algorithm, each set instantiated in a translation unit
+// of its own (relax_*.cu, resident_*.cu: they compile in parallel).
+// relax_fn: one launch per iteration in style v; dispatch_fn: one launch per
+// iteration in the style the selectors picked; resident_fn: every iteration in
+// one launch, in style v or (v < 0) the selectors' per-iteration pick. `wide`:
+// the selectors' form compiled for the fixed styles' resident blocks per SM.
+template <int ALG>
+KernelFn relax_fn(int v);
+template <int ALG>
+KernelFn dispatch_fn(bool wide);
+template <int ALG>
+KernelFn resident_fn(int v, bool wide);
+KernelFn near_far_kernel(bool resident);  // SSSP with the near/far ordering (relax_sssp.cu, resident_sssp.cu)
+KernelFn mis_kernel(bool resident);       // maximal independent set (relax_mis.cu)
 const float* mlp_device_params();
 int mlp_install(const float* params, int count);
 

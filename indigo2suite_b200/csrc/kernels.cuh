@@ -1,0 +1,53 @@
+// Kernel tables: the bodies of relax_fn, dispatch_fn and resident_fn
+// (engine.h). Each is instantiated for one algorithm per translation unit.
+#pragma once
+#include "engine.h"
+#include "mlp.cuh"
+#include "relax.cuh"
+#include "iteration.cuh"
+
+namespace i2 {
+
+template <int ALG>
+KernelFn relax_fn(int v) {
+  switch (v) {
+    case kVPThread: return relax_push<ALG, kVPThread>;
+    case kVPWarp: return relax_push<ALG, kVPWarp>;
+    case kVPCta: return relax_edge_balanced<ALG>;
+    case kVPBlock: return relax_push<ALG, kVPBlock>;
+    case kPullFrontier: return relax_pull<ALG, true>;
+    case kPullTopo: return relax_pull<ALG, false>;
+    case kEdgeTopo: return relax_edge_topo<ALG>;
+    case kPushTopo: return relax_push_topo<ALG>;
+    case kUnionFind:
+      if constexpr (ALG == kCC) return relax_union<ALG>;
+      return nullptr;
+  }
+  return nullptr;
+}
+
+template <int ALG>
+KernelFn dispatch_fn(bool wide) {
+  return wide ? relax_dispatch<ALG, I2_EB_MIN_BLOCKS> : relax_dispatch<ALG>;
+}
+
+template <int ALG>
+KernelFn resident_fn(int v, bool wide) {
+  switch (v) {
+    case kVPThread: return relax_resident<ALG, kVPThread>;
+    case kVPWarp: return relax_resident<ALG, kVPWarp>;
+    case kVPCta: return relax_resident<ALG, kVPCta>;
+    case kVPBlock: return relax_resident<ALG, kVPBlock>;
+    case kPullFrontier: return relax_resident<ALG, kPullFrontier>;
+    case kPullTopo: return relax_resident<ALG, kPullTopo>;
+    case kEdgeTopo: return relax_resident<ALG, kEdgeTopo>;
+    case kPushTopo: return relax_resident<ALG, kPushTopo>;
+    case kUnionFind:
+      if constexpr (ALG == kCC) return relax_resident<ALG, kUnionFind>;
+      return nullptr;
+  }
+  // per-iteration pick
+  return wide ? relax_resident<ALG, -1, false, I2_EB_MIN_BLOCKS> : relax_resident<ALG, -1>;
+}
+
+}  // namespace i2

@@ -1,0 +1,9 @@
+// CC kernels launched once per iteration (every style, and the selectors' dispatch).
+#include "kernels.cuh"
+
+namespace i2 {
+
+template KernelFn relax_fn<kCC>(int);
+template KernelFn dispatch_fn<kCC>(bool);
+
+}  // namespace i2

@@ -1,0 +1,8 @@
+// CC kernels that run a whole traversal in one launch.
+#include "kernels.cuh"
+
+namespace i2 {
+
+template KernelFn resident_fn<kCC>(int, bool);
+
+}  // namespace i2
