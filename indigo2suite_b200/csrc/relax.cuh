@@ -1524,73 +1524,263 @@ __device__ __forceinline__ bool body_union(const Ctx& c, Stage& s) {
 }
 
 // ---------------------------------------------------------------------------
-// Maximal independent set (kMIS; one style). A warp per frontier vertex v
-// still undecided: its lanes scan v's neighbours for ones that outrank v. If one
-// of them is in the set, v is out; if none is undecided (all out, or there are
-// none), v is in; otherwise v waits. A vertex that decides pushes its undecided
-// neighbours into the next frontier, so a waiting vertex is examined again as
-// soon as a neighbour that outranks it decides. Decisions depend only on
-// outranking vertices, whose decisions are final, so the set is the greedy one
-// in decreasing rank whatever the order of the updates.
-__device__ __forceinline__ bool body_mis(const Ctx& c, EBShared& sh) {
-  EpiStage& s = sh.s;
+// Maximal independent set (kMIS; one style). A frontier entry is an undecided
+// vertex v with a cursor into its adjacency: every neighbour before the cursor
+// is known not to block v (it does not outrank v, or it is out). An iteration
+// moves the cursor on to the first neighbour that outranks v and is undecided,
+// and v waits there; one that is in the set makes v out; past the end v joins
+// the set and writes its neighbours out, which the waiting ones find when their
+// turn comes. Decisions depend only on outranking vertices, whose decisions are
+// final, so the set is the greedy one in decreasing rank whatever the order of
+// the updates; a vertex in the set outranks all its undecided neighbours, and
+// those that outrank it are out already, so its writes are right without
+// looking.
+//
+// Each adjacency list is scanned once over the whole run and mostly not past
+// its second entry (a random neighbour outranks v half the time), so the work
+// is far below the graph's edges: random status reads bound it. One thread
+// scans the first kMisProbe entries, a warp goes on, and lists of
+// kMisBlockDegree entries or more take the whole block. (A warp per vertex
+// rescanning the list in every iteration left a hub to one warp: RMAT 2^20 took
+// 2,642 us, 2,122 of them in the first iteration; now 482 and 186.)
+constexpr int kMisProbe = 16;          // entries a thread scans (or writes) by itself
+constexpr int kMisBlockDegree = 2048;  // entries from which the whole block does
+
+// Outcome of `count` (<= 4) consecutive entries from k on, loaded together:
+// bit r of *wait: entry r outranks v and is undecided; returns whether one
+// that outranks v is in the set.
+__device__ __forceinline__ bool mis_probe(const Ctx& c, int v, int pv, const int* k, int count, unsigned* wait) {
+  volatile int* st = c.dist;
+  const int* __restrict__ nl = c.g.nlist;
+  int u[4], su[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) u[r] = r < count ? ld_adj(nl + k[r]) : v;
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+    su[r] = (u[r] != v && mis_outranks(u[r], mis_priority(u[r]), v, pv)) ? (int)st[u[r]] : (int)kMisOut;
+  unsigned w = 0;
+  bool in = false;
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    in |= su[r] == kMisIn;
+    w |= su[r] == kMisUndecided ? 1u << r : 0u;
+  }
+  *wait = w;
+  return in;
+}
+
+// Publish the staged waiting vertices (block-uniform call): s.q the vertices,
+// s.qd their cursors, s.m their entries still to scan.
+__device__ __forceinline__ void mis_flush(const Ctx& c, Stage& s, int nxt) {
+  __syncthreads();
+  const int n = s.n;
+  if (n == 0) return;
+  if (threadIdx.x == 0)
+    s.base = atomicAdd(&c.ctl->slot[nxt].packed, ((unsigned long long)n << 32) | (unsigned)s.m);
+  __syncthreads();
+  const int b = (int)(s.base >> 32);
+  for (int j = threadIdx.x; j < n; j += kBlock) {
+    c.wl[nxt][b + j] = s.q[j];
+    c.woff[nxt][b + j] = (unsigned)s.qd[j];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s.n = 0;
+    s.m = 0;
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ bool body_mis(const Ctx& c, Stage& s) {
   block_prologue(c);
   const int i = c.ctl->iter;
   const int cur = i % 3, nxt = (i + 1) % 3, old = (i + 2) % 3;
   const int n = slot_size(c.ctl->slot[cur].packed);
-  const int active = active_blocks(c, old, ((long long)n + kWarpsPerBlock - 1) / kWarpsPerBlock);
+  const int active = (int)min((long long)gridDim.x, ((long long)n + kBlock - 1) / kBlock);
   if (blockIdx.x >= active) return idle_epilogue(c, s, i, cur, nxt, old);
-  if (threadIdx.x == 0) s.last = 0;
+  stage_init(s);
+  if (threadIdx.x == 0) s.m = 0;
   Acc a;
   acc_init(a);
-  clear_old(c, old, active);
-  const int lane = threadIdx.x & 31;
-  WarpStage& ws = sh.wss[threadIdx.x >> 5];
-  if (lane == 0) ws.n = 0;
-  __syncwarp();
+  __syncthreads();
   const int* wl = c.wl[cur];
+  const unsigned* cursor = c.woff[cur];
   volatile int* st = c.dist;
   const int* __restrict__ nl = c.g.nlist;
-  const long long stride = (long long)active * kWarpsPerBlock;
-  for (long long k = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); k < n; k += stride) {
-    const int v = wl[k];
-    if (st[v] != kMisUndecided) continue;  // warp-uniform
-    const int pv = mis_priority(v);
-    const int b = c.g.nindex[v], e = c.g.nindex[v + 1];
-    bool in_set = false, waiting = false;
-    for (int base = b; base < e; base += kWarp) {
-      const int j = base + lane;
-      if (j < e) {
-        const int u = ld_adj(nl + j);
-        if (u != v && mis_outranks(u, mis_priority(u), v, pv)) {
-          const int su = st[u];
-          in_set |= su == kMisIn;
-          waiting |= su == kMisUndecided;
+  const int lane = threadIdx.x & 31;
+  for (long long base = (long long)blockIdx.x * kBlock; base < n; base += (long long)active * kBlock) {
+    const long long idx = base + threadIdx.x;
+    enum { kNone, kWait, kIn, kOut, kMore };
+    int state = kNone, v = 0, pv = 0, k = 0, end = 0;
+    if (idx < n) {
+      v = wl[idx];
+      state = kMore;
+      if (st[v] != kMisUndecided) {  // a neighbour joined the set meanwhile
+        state = kNone;
+        a.visited++;
+      } else {
+        k = i == 0 ? c.g.nindex[v] : (int)cursor[idx];
+        end = c.g.nindex[v + 1];
+        pv = mis_priority(v);
+        for (int t = 0; t < kMisProbe && state == kMore; t += 4) {
+          const int cnt = min(4, end - k);
+          const int ks[4] = {k, k + 1, k + 2, k + 3};
+          unsigned w = 0;
+          if (cnt <= 0) {
+            state = kIn;
+          } else if (mis_probe(c, v, pv, ks, cnt, &w)) {
+            state = kOut;
+          } else if (w) {
+            k += __ffs(w) - 1;
+            state = kWait;
+          } else {
+            k += cnt;
+          }
+        }
+        if (state == kMore && k >= end) state = kIn;
+      }
+    }
+    // longer lists: the block's (deferred to after the pass), else the warp's
+    bool mine = state == kMore;
+    if (mine && end - k >= kMisBlockDegree) {
+      const int p = atomicAdd(&s.hn, 1);
+      if (p < kHQueue) {
+        s.hq[p] = v;
+        s.ht[p] = k;
+        state = kNone;
+        mine = false;
+      }
+    }
+    for (unsigned todo = __ballot_sync(0xffffffffu, mine); todo; todo &= todo - 1) {
+      const int l = __ffs(todo) - 1;
+      const int wv = __shfl_sync(0xffffffffu, v, l), wpv = __shfl_sync(0xffffffffu, pv, l);
+      const int we = __shfl_sync(0xffffffffu, end, l);
+      int wk = __shfl_sync(0xffffffffu, k, l), out = kIn;
+      for (; wk < we; wk += 4 * kWarp) {
+        int ks[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) ks[r] = wk + r * kWarp + lane;
+        const int cnt = we - wk > lane ? min(4, (we - wk - lane + kWarp - 1) / kWarp) : 0;
+        unsigned w = 0;
+        const bool in = mis_probe(c, wv, wpv, ks, cnt, &w);
+        if (__any_sync(0xffffffffu, in)) {
+          out = kOut;
+          break;
+        }
+        const int first = __reduce_min_sync(0xffffffffu, w ? (__ffs(w) - 1) * kWarp + lane : INT_MAX);
+        if (first != INT_MAX) {
+          wk += first;
+          out = kWait;
+          break;
         }
       }
-      if (__any_sync(0xffffffffu, in_set)) break;  // v is out whatever the rest holds
+      if (lane == l) {
+        state = out;
+        k = wk;
+      }
     }
-    const bool out = __any_sync(0xffffffffu, in_set);
-    const bool wait = !out && __any_sync(0xffffffffu, waiting);
-    if (wait) continue;
-    if (lane == 0) st[v] = out ? kMisOut : kMisIn;
-    a.visited += lane == 0;
-    for (int base = b; base < e; base += kWarp) {
-      const int j = base + lane;
-      if (j < e) {
+    if (state == kOut) {
+      st[v] = kMisOut;
+      a.visited++;
+    }
+    // joined: neighbours are out
+    bool wide = false;
+    if (state == kIn) {
+      st[v] = kMisIn;
+      a.visited++;
+      const int b = c.g.nindex[v];
+      if (end - b <= kMisProbe) {
+        for (int j = b; j < end; ++j) {
+          const int u = ld_adj(nl + j);
+          if (u != v) st[u] = kMisOut;
+        }
+      } else {
+        k = b;
+        wide = true;
+      }
+    }
+    for (unsigned todo = __ballot_sync(0xffffffffu, wide); todo; todo &= todo - 1) {
+      const int l = __ffs(todo) - 1;
+      const int wv = __shfl_sync(0xffffffffu, v, l), we = __shfl_sync(0xffffffffu, end, l);
+#pragma unroll 4
+      for (int j = __shfl_sync(0xffffffffu, k, l) + lane; j < we; j += kWarp) {
         const int u = ld_adj(nl + j);
-        if (u != v && st[u] == kMisUndecided) {
-          const unsigned bit = 1u << (u & 31);
-          unsigned* w = &c.bm[nxt][u >> 5];
-          if (!(*(volatile unsigned*)w & bit) && !(atomicOr(w, bit) & bit))
-            warp_stage_entry(c, ws, a, nxt, u, c.g.nindex[u + 1] - c.g.nindex[u]);
+        if (u != wv) st[u] = kMisOut;
+      }
+    }
+    // waiting vertices into the block's queue
+    const unsigned waiting = __ballot_sync(0xffffffffu, state == kWait);
+    if (waiting) {
+      const int left = __reduce_add_sync(0xffffffffu, state == kWait ? end - k : 0);
+      int p = 0;
+      if (lane == 0) {
+        p = atomicAdd(&s.n, __popc(waiting));
+        atomicAdd(&s.m, left);
+      }
+      p = __shfl_sync(0xffffffffu, p, 0) + __popc(waiting & ((1u << lane) - 1u));
+      if (state == kWait) {
+        s.q[p] = v;
+        s.qd[p] = k;
+      }
+    }
+    __syncthreads();
+    // lists for the whole block
+    const int nb = min(s.hn, kHQueue);
+    for (int x = 0; x < nb; ++x) {
+      const int bv = s.hq[x], be = c.g.nindex[bv + 1], bpv = mis_priority(bv);
+      int bk = s.ht[x], out = kIn;
+      for (; bk < be; bk += 4 * kBlock) {
+        if (threadIdx.x == 0) {
+          s.j0 = INT_MAX;
+          s.chunk = 0;
+        }
+        __syncthreads();
+        int ks[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) ks[r] = bk + r * kBlock + threadIdx.x;
+        const int t = threadIdx.x;
+        const int cnt = be - bk > t ? min(4, (be - bk - t + kBlock - 1) / kBlock) : 0;
+        unsigned w = 0;
+        if (mis_probe(c, bv, bpv, ks, cnt, &w)) s.chunk = 1;
+        if (w) atomicMin(&s.j0, (__ffs(w) - 1) * kBlock + t);
+        __syncthreads();
+        const int found = s.chunk, first = s.j0;
+        __syncthreads();  // read before the next step resets them
+        if (found) {
+          out = kOut;
+          break;
+        }
+        if (first != INT_MAX) {
+          bk += first;
+          out = kWait;
+          break;
         }
       }
-      __syncwarp();
-      if (ws.n >= kWarpQueue / 2) warp_flush(c, ws, nxt);
+      if (out == kIn) {
+        for (int j = c.g.nindex[bv] + (int)threadIdx.x; j < be; j += kBlock) {
+          const int u = ld_adj(nl + j);
+          if (u != bv) st[u] = kMisOut;
+        }
+      }
+      if (threadIdx.x == 0) {
+        if (out == kWait) {
+          s.q[s.n] = bv;
+          s.qd[s.n] = bk;
+          s.n += 1;
+          s.m += be - bk;
+        } else {
+          st[bv] = out == kIn ? kMisIn : kMisOut;
+          a.visited++;
+        }
+      }
     }
+    __syncthreads();
+    if (threadIdx.x == 0) s.hn = 0;
+    // a pass adds at most kBlock entries
+    if (s.n > kQueue - kBlock) mis_flush(c, s, nxt);
+    __syncthreads();
   }
-  warp_flush(c, ws, nxt);
+  mis_flush(c, s, nxt);
   __syncthreads();
   return block_epilogue(c, s, a, i, cur, nxt, old, active);
 }
@@ -1610,8 +1800,8 @@ __global__ void __launch_bounds__(kBlock, I2_EB_MIN_BLOCKS) relax_edge_balanced(
 }
 
 static __global__ void __launch_bounds__(kBlock, I2_EB_MIN_BLOCKS) relax_mis(Ctx c) {
-  __shared__ EBShared sh;
-  body_mis(c, sh);
+  __shared__ Stage s;
+  body_mis(c, s);
 }
 
 // Edge-balanced SSSP push with near/far ordering (Ctl::delta != 0).
@@ -1682,7 +1872,7 @@ __device__ __forceinline__ void grid_wait(Ctl* ctl, unsigned gen) {
 template <int ALG, int VAR, bool DEFER>
 __device__ __forceinline__ bool run_body(const Ctx& c, AnyShared<DEFER>& sh) {
   if constexpr (ALG == kMIS) {
-    return body_mis(c, sh.eb);  // one style
+    return body_mis(c, sh.st);  // one style
   } else {
     const int v = VAR >= 0 ? VAR : *(volatile int*)&c.ctl->variant;  // uniform: written before the release
     switch (v) {

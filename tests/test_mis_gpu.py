@@ -72,3 +72,22 @@ def test_mis_edge_cases_and_refusals(gpu):
     np.testing.assert_array_equal(st, oracle.mis(g))
     np.testing.assert_array_equal(prio, [oracle.mis_priority(v) for v in range(g.nodes)])
     dg.free()
+
+
+@pytest.mark.parametrize("degree", [1, 15, 16, 17, 143, 144, 145, 2047, 2063, 2064, 2065, 3089, 70001])
+def test_mis_stars_around_the_list_lengths_where_threads_warps_and_blocks_take_over(gpu, degree):
+    n = degree + 1
+    order = np.argsort(i2.mis_priority(np.arange(n)).astype(np.int64) * n + np.arange(n))
+    for hub in {int(order[-1]), int(order[-2]), int(order[0]), int(order[n // 2])}:
+        # a star of n vertices, and beside it a path through every second leaf
+        leaves = np.array([v for v in range(n) if v != hub], np.int32)
+        u = np.concatenate([np.full(degree, hub, np.int32), leaves, leaves[:-1:2], leaves[1::2]])
+        v = np.concatenate([leaves, np.full(degree, hub, np.int32), leaves[1::2], leaves[:-1:2]])
+        o = np.lexsort((v, u))
+        ni = np.zeros(n + 1, np.int32)
+        np.cumsum(np.bincount(u, minlength=n), out=ni[1:])
+        g = i2.ECLGraph(n, len(u), ni, np.ascontiguousarray(v[o]), np.ones(len(u), np.int32))
+        dg = i2.DeviceGraph.upload(g)
+        for loop in (i2.I2_LOOP_GRAPH, i2.I2_LOOP_HOST):
+            np.testing.assert_array_equal(dg.mis(loop=loop)[0], oracle.mis(g), err_msg=f"hub {hub} loop {loop}")
+        dg.free()
