@@ -216,7 +216,7 @@ __device__ __forceinline__ void hist_far(const Hists& hs, int val, int deg) {
 // Defer v (new value val, at or above the threshold) to the current far pile.
 // The pile's bitmap keeps one live entry per vertex: a vertex already on the
 // pile only lowers the pile's minimum. Vertices without edges are never
-// deferred. With a warp stage the entry is staged (published by warp_flush
+// deferred. With a warp stage the entry is staged (published by warp_publish
 // with one atomic per flush); without one it is appended at once. False when
 // the pile is full: the caller then pushes v into the next frontier, which is
 // always valid. With the edge budget (hs) new entries are histogrammed.
@@ -683,16 +683,15 @@ __device__ __forceinline__ bool body_push(const Ctx& c, Stage& s) {
 // warp scan and one packed atomic. No vertex is too big or too small: work is
 // split by edges, as in the reference's edge-centric codes.
 constexpr int kWarpTile = kWarp * kEdgesPerThread;  // edges per warp tile
-// Warp staging capacity (overflow appends directly); a warp flushes once it
-// holds half of it, and a tile pushes at most kWarpTile entries. 192 rather
+// Warp queue capacity; a tile queues at most kWarpTile vertices, and the queue
+// is resolved when the next tile's might not fit. 192 rather
 // than 256: the 5 KB less shared memory per block is L1 for the random value
 // and bitmap reads (RMAT-22 SSSP 4% faster; 128 loses on grids).
 #ifndef I2_WARP_QUEUE
 #define I2_WARP_QUEUE 192
 #endif
 constexpr int kWarpQueue = I2_WARP_QUEUE;
-static_assert(kWarpQueue % kWarp == 0 && kWarpQueue / 2 + kWarpTile <= kWarpQueue,
-              "a tile's pushes must fit after a half-full queue");
+static_assert(kWarpQueue % kWarp == 0 && kWarpTile <= kWarpQueue, "a tile's vertices must fit");
 constexpr int kWarpsPerBlock = kBlock / kWarp;
 
 struct WarpStage {
@@ -718,7 +717,7 @@ __device__ __forceinline__ void warp_stage_entry(const Ctx& c, WarpStage& ws, Ac
 }
 
 // Stage a far-pile entry of the near/far ordering: kept in the warp's queue
-// as ~v (negative) beside its degree, and published by warp_flush<true>.
+// as ~v (negative) beside its degree, and published by warp_publish<true>.
 // Without room in the queue it is appended at once.
 __device__ __forceinline__ bool stage_far(const Ctx& c, WarpStage* ws, int v, int deg) {
   const int p = atomicAdd(&ws->n, 1);
@@ -730,45 +729,22 @@ __device__ __forceinline__ bool stage_far(const Ctx& c, WarpStage* ws, int v, in
   return pile_append(c, c.ctl->pcur, v, deg);
 }
 
-template <bool DEFER>
-__device__ __forceinline__ void warp_push_vertex(const Ctx& c, WarpStage& ws, Acc& a, int nxt, int v, int val,
-                                                 int old, int thr, const Hists& hs) {
-  if (old == kInf) a.visited++;
-  if (DEFER && val >= thr && defer_vertex(c, a, v, val, &ws, hs.h ? &hs : nullptr)) return;
-  if (DEFER && hs.h) unpile(c, v);
-  a.mindist = min(a.mindist, val);
-  const unsigned bit = 1u << (v & 31);
-  unsigned* w = &c.bm[nxt][v >> 5];
-  if (*(volatile unsigned*)w & bit) return;
-  if (atomicOr(w, bit) & bit) return;
-  const int deg = c.g.nindex[v + 1] - c.g.nindex[v];
-  if (deg == 0) {
-    atomicAnd(w, ~bit);
-    return;
-  }
-  if (DEFER && hs.h) hist_near(hs, val, deg);
-  warp_stage_entry(c, ws, a, nxt, v, deg);
-}
-
-// Publish the warp's staged entries (warp-uniform call): one packed atomic
+// Publish the warp's resolved queue entries [0, n) (warp-uniform call): q[j] a
+// vertex and qd[j] its degree, 0 where the entry was dropped. One packed atomic
 // reserves positions and edge offsets in the next frontier for all of them.
-// DEFER: the queue also holds far-pile entries (negative, ~v); they go onto
-// the current pile with one more atomic, and the frontier entries are
-// compacted. Far entries that find the pile full join the next frontier.
+// DEFER: negative entries (~v) are far-pile entries; they go onto the current
+// pile with one more atomic. Far entries that find the pile full join the next
+// frontier. Lane l owns the entries l, l + 32, ...
 template <bool DEFER = false>
-__device__ __forceinline__ void warp_flush(const Ctx& c, WarpStage& ws, int nxt) {
+__device__ __forceinline__ void warp_publish(const Ctx& c, WarpStage& ws, int nxt, int n) {
   constexpr int kPer = kWarpQueue / kWarp;
-  __syncwarp();
-  const int n = min(ws.n, kWarpQueue);
-  __syncwarp();
-  if (n == 0) return;
   const int lane = threadIdx.x & 31;
   if constexpr (DEFER) {
     int nf = 0;
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
-      const int j = lane * kPer + i;
-      nf += (j < n && ws.q[j] < 0) ? 1 : 0;
+      const int j = lane + i * kWarp;
+      nf += (j < n && ws.q[j] < 0 && ws.qd[j] > 0) ? 1 : 0;
     }
     int fincl = nf;
     for (int o = 1; o < 32; o <<= 1) {
@@ -783,8 +759,8 @@ __device__ __forceinline__ void warp_flush(const Ctx& c, WarpStage& ws, int nxt)
       pb = __shfl_sync(0xffffffffu, pb, 0);
       unsigned k = pb + (unsigned)(fincl - nf);
       for (int i = 0; i < kPer; ++i) {
-        const int j = lane * kPer + i;
-        if (j < n && ws.q[j] < 0) {
+        const int j = lane + i * kWarp;
+        if (j < n && ws.q[j] < 0 && ws.qd[j] > 0) {
           const int v = ~ws.q[j];
           if (k < c.pile_cap && k >= pb) {
             c.pile[p][k] = v;
@@ -804,94 +780,150 @@ __device__ __forceinline__ void warp_flush(const Ctx& c, WarpStage& ws, int nxt)
       __syncwarp();
     }
   }
-  if constexpr (!DEFER) {
-    int d[kPer];
-    int sum = 0;
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-      const int j = lane * kPer + i;
-      d[i] = sum;
-      sum += j < n ? ws.qd[j] : 0;
-    }
-    int incl = sum;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
-    }
-    const int excl = incl - sum;
-    const int tot = __shfl_sync(0xffffffffu, incl, 31);
-    unsigned long long base = 0;
-    if (lane == 0) {
-      base = atomicAdd(&c.ctl->slot[nxt].packed, ((unsigned long long)n << 32) | (unsigned)tot);
-      ws.n = 0;
-    }
-    base = __shfl_sync(0xffffffffu, base, 0);
-    const int b = (int)(base >> 32);
-    const unsigned eb = (unsigned)(base & 0xffffffffu);
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-      const int j = lane * kPer + i;
-      if (j < n) {
-        c.wl[nxt][b + j] = ws.q[j];
-        c.woff[nxt][b + j] = eb + (unsigned)(excl + d[i]);
-      }
-    }
-    __syncwarp();
-    return;
-  }
   // frontier entries: count and degree prefix in one 64-bit scan
-  unsigned long long d[kPer];
   unsigned long long sum = 0;
 #pragma unroll
   for (int i = 0; i < kPer; ++i) {
-    const int j = lane * kPer + i;
-    d[i] = sum;
-    if (j < n && ws.q[j] >= 0) sum += (1ull << 32) | (unsigned)ws.qd[j];
+    const int j = lane + i * kWarp;
+    if (j < n && (!DEFER || ws.q[j] >= 0) && ws.qd[j] > 0) sum += (1ull << 32) | (unsigned)ws.qd[j];
   }
   unsigned long long incl = sum;
   for (int o = 1; o < 32; o <<= 1) {
     const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += y;
   }
-  const unsigned long long excl = incl - sum;
-  const unsigned long long tot = __shfl_sync(0xffffffffu, incl, 31);
   unsigned long long base = 0;
-  if (lane == 0) {
-    if (tot) base = atomicAdd(&c.ctl->slot[nxt].packed, tot);
-    ws.n = 0;
-  }
-  base = __shfl_sync(0xffffffffu, base, 0);
-  const int b = (int)(base >> 32);
-  const unsigned eb = (unsigned)(base & 0xffffffffu);
+  if (lane == 31 && incl) base = atomicAdd(&c.ctl->slot[nxt].packed, incl);
+  base = __shfl_sync(0xffffffffu, base, 31) + incl - sum;
 #pragma unroll
   for (int i = 0; i < kPer; ++i) {
-    const int j = lane * kPer + i;
-    if (j < n && ws.q[j] >= 0) {
-      const unsigned long long x = excl + d[i];
-      c.wl[nxt][b + (int)(x >> 32)] = ws.q[j];
-      c.woff[nxt][b + (int)(x >> 32)] = eb + (unsigned)(x & 0xffffffffu);
+    const int j = lane + i * kWarp;
+    if (j < n && (!DEFER || ws.q[j] >= 0) && ws.qd[j] > 0) {
+      c.wl[nxt][slot_size(base)] = ws.q[j];
+      c.woff[nxt][slot_size(base)] = slot_edges(base);
+      base += (1ull << 32) | (unsigned)ws.qd[j];
     }
   }
   __syncwarp();
 }
 
+// Resolve and publish the warp's queue of n lowered vertices (warp-uniform
+// call). An entry is a vertex whose value a relaxation lowered; the frontier
+// bitmap decides here, for up to kPart entries per lane at once, whether it is
+// pushed, so the chain of dependent bitmap read, atomicOr and degree reads is
+// paid once per queue and not for each edge of every tile that lowers a value
+// (ER 2M SSSP 1,651 -> 1,558 us, RMAT-22 SSSP 2,314 -> 2,205, grid 2000^2 BFS
+// 2,580 -> 2,337, a batch of 32 graphs 6,476 -> 5,952).
+// BFS (visited counted here; level `val`): entries may repeat.
+// DEFER: negative entries (~v) are values at or above the threshold, bound for
+// the far pile; qd holds the values. One whose vertex has meanwhile fallen
+// below the threshold is dropped: the fall queued it as near.
+// A vertex without edges keeps its bitmap bit and is dropped: it has nothing
+// to relax in any style, and the bit keeps its visit counted once.
 template <int ALG, bool DEFER>
-__device__ __forceinline__ void warp_relax_batch(const Ctx& c, WarpStage& ws, Acc& a, int nxt, const int* du,
-                                                 const int* nv, const int* wv, const bool* ok, int thr,
-                                                 const Hists& hs) {
-  int cand[kEdgesPerThread], cur[kEdgesPerThread];
+__device__ __forceinline__ void warp_resolve(const Ctx& c, WarpStage& ws, Acc& a, int nxt, int n, int thr,
+                                             const Hists& hs) {
+  constexpr int kPer = kWarpQueue / kWarp;
+  constexpr int kPart = 3;
+  static_assert(kPer % kPart == 0, "whole parts");
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  for (int part = 0; part < kPer && part * kWarp < n; part += kPart) {
+    int v[kPart], deg[kPart];
+    unsigned w[kPart];
+    bool live[kPart], far[kPart];
+#pragma unroll
+    for (int r = 0; r < kPart; ++r) {
+      const int j = (part + r) * kWarp + lane;
+      const int e = j < n ? ws.q[j] : 0;
+      live[r] = j < n;
+      far[r] = DEFER && e < 0;
+      v[r] = far[r] ? ~e : e;
+      unsigned* word = (far[r] ? c.fbm : c.bm[nxt]) + (v[r] >> 5);
+      w[r] = live[r] ? *(volatile unsigned*)word : ~0u;
+      if (DEFER && far[r] && live[r] && *(volatile int*)&c.dist[v[r]] < thr) {
+        live[r] = false;
+        w[r] = ~0u;
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < kPart; ++r) {
+      const unsigned bit = 1u << (v[r] & 31);
+      deg[r] = 0;
+      if (!(w[r] & bit)) {
+        deg[r] = c.g.nindex[v[r] + 1] - c.g.nindex[v[r]];
+        w[r] = atomicOr((far[r] ? c.fbm : c.bm[nxt]) + (v[r] >> 5), bit);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < kPart; ++r) {
+      const unsigned bit = 1u << (v[r] & 31);
+      const int j = (part + r) * kWarp + lane;
+      const bool won = live[r] && !(w[r] & bit);
+      if (ALG == kBFS && won) a.visited++;
+      if (DEFER && live[r]) {
+        const int val = ws.qd[j];
+        if (far[r]) {
+          if (won && deg[r] == 0) {
+            atomicAnd(&c.fbm[v[r] >> 5], ~bit);  // never on the pile
+          } else {
+            a.fmin = min(a.fmin, val);
+            if (won && hs.h) hist_far(hs, val, deg[r]);
+          }
+        } else {
+          if (hs.h) unpile(c, v[r]);
+          if (won && deg[r] && hs.h) hist_near(hs, val, deg[r]);
+        }
+      }
+      if (won && deg[r] && !far[r]) {
+        a.maxdeg = max(a.maxdeg, deg[r]);
+        if (deg[r] >= c.heavy)
+          direct_append(&c.ctl->slot[nxt].hpacked, c.hwl[nxt], c.htoff[nxt], v[r], heavy_tiles(deg[r]));
+      }
+      if (j < n) ws.qd[j] = won ? deg[r] : 0;
+    }
+  }
+  warp_publish<DEFER>(c, ws, nxt, n);
+}
+
+// Relax this lane's candidate edges and queue the vertices whose values fell:
+// all dist[] loads first, then all atomicMins, then the queue (its length qn
+// is warp-uniform and returned). BFS runs level by level in every style, so an
+// unreached neighbour takes the level with a plain store (every writer of the
+// iteration writes the same one).
+template <int ALG, bool DEFER>
+__device__ __forceinline__ int warp_relax_batch(const Ctx& c, WarpStage& ws, Acc& a, const int* du, const int* nv,
+                                                const int* wv, const bool* ok, int thr, int qn) {
+  int cand[kEdgesPerThread], old[kEdgesPerThread];
+  const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int r = 0; r < kEdgesPerThread; ++r) {
     cand[r] = ok[r] ? Op<ALG>::cand(du[r], wv[r]) : kInf;
-    cur[r] = ok[r] ? c.dist[nv[r]] : kInf;
+    old[r] = ok[r] ? c.dist[nv[r]] : kInf;
   }
 #pragma unroll
   for (int r = 0; r < kEdgesPerThread; ++r) {
-    if (cand[r] < cur[r]) {
-      const int old = atomicMin(&c.dist[nv[r]], cand[r]);
-      if (cand[r] < old) warp_push_vertex<DEFER>(c, ws, a, nxt, nv[r], cand[r], old, thr, hs);
+    if (ALG == kBFS) {
+      if (cand[r] < old[r]) c.dist[nv[r]] = cand[r];
+    } else if (cand[r] < old[r]) {
+      old[r] = atomicMin(&c.dist[nv[r]], cand[r]);
     }
   }
+#pragma unroll
+  for (int r = 0; r < kEdgesPerThread; ++r) {
+    const bool fell = cand[r] < old[r];
+    const unsigned m = __ballot_sync(0xffffffffu, fell);
+    if (fell) {
+      const int p = qn + __popc(m & ((1u << lane) - 1u));
+      const bool far = DEFER && cand[r] >= thr;
+      ws.q[p] = far ? ~nv[r] : nv[r];
+      if (DEFER) ws.qd[p] = cand[r];
+      if (ALG != kBFS && old[r] == kInf) a.visited++;
+      if (!far) a.mindist = min(a.mindist, cand[r]);
+    }
+    qn += __popc(m);
+  }
+  return qn;
 }
 
 struct EpiStage {
@@ -942,6 +974,18 @@ __device__ __forceinline__ void block_hist_end(const unsigned* h, unsigned long 
   const unsigned x = h[threadIdx.x], y = h[kHistBins + threadIdx.x];
   if (x) atomicAdd(&dst[threadIdx.x], (unsigned long long)x);
   if (y) atomicAdd(&dst[kHistBins + threadIdx.x], (unsigned long long)y);
+}
+
+// Publish a split launch's staged entries once there are `least` of them
+// (warp-uniform call).
+__device__ __forceinline__ void split_flush(const Ctx& c, WarpStage& ws, int nxt, int least) {
+  __syncwarp();
+  const int n = min(ws.n, kWarpQueue);
+  __syncwarp();
+  if (n < least) return;
+  warp_publish<true>(c, ws, nxt, n);
+  if ((threadIdx.x & 31) == 0) ws.n = 0;
+  __syncwarp();
 }
 
 // Launches of the SSSP near/far ordering other than relaxations (Ctl::split):
@@ -1093,10 +1137,9 @@ __device__ __forceinline__ bool body_split(const Ctx& c, EBSharedFar& sh, int i,
       }
       __syncthreads();  // s_keep and s_kbase are rewritten by the next pass
     }
-    __syncwarp();
-    if (ws.n >= kWarpQueue - kR * kWarp) warp_flush<true>(c, ws, nxt);
+    split_flush(c, ws, nxt, kWarpQueue - kR * kWarp);
   }
-  warp_flush<true>(c, ws, nxt);
+  split_flush(c, ws, nxt, 1);
   if (budget) block_hist_end(sh.hist, c.hist);
   __syncthreads();
   return block_epilogue(c, s, a, i, cur, nxt, old, active);
@@ -1134,8 +1177,7 @@ __device__ __forceinline__ bool body_edge_balanced(const Ctx& c, EBSharedT<DEFER
   clear_old(c, old, active);
   const int lane = threadIdx.x & 31;
   WarpStage& ws = sh.wss[threadIdx.x >> 5];
-  if (lane == 0) ws.n = 0;
-  __syncwarp();
+  int qn = 0;  // queued vertices of this warp
   const int* wl = c.wl[cur];
   const unsigned* woff = c.woff[cur];
   const int* __restrict__ nl = c.g.nlist;
@@ -1166,7 +1208,7 @@ __device__ __forceinline__ bool body_edge_balanced(const Ctx& c, EBSharedT<DEFER
         const int below = __popc(__ballot_sync(0xffffffffu, w < e1));
         if (lane < below) {  // offsets ascend: the entries below e1 are a prefix
           ws.beg[m + lane] = c.g.nindex[v];
-          ws.du[m + lane] = c.dist[v];
+          if (ALG != kBFS) ws.du[m + lane] = c.dist[v];
         }
         m += below;
         if (below < kWarp) break;
@@ -1188,18 +1230,21 @@ __device__ __forceinline__ bool body_edge_balanced(const Ctx& c, EBSharedT<DEFER
           const int e = ws.beg[o] + (int)(x - ws.off[o]);
           nv[r] = ld_adj(nl + e);
           if (Op<ALG>::kWeighted) wv[r] = ld_adj(ew + e);
-          du[r] = ws.du[o];
+          du[r] = ALG == kBFS ? i : ws.du[o];  // BFS: F_i is level i
           ok[r] = Op<ALG>::valid(du[r]);
         }
       }
-      warp_relax_batch<ALG, DEFER>(c, ws, a, nxt, du, nv, wv, ok, thr, hs);
+      qn = warp_relax_batch<ALG, DEFER>(c, ws, a, du, nv, wv, ok, thr, qn);
       // the next tile starts at e1: its first entry is the last one with offset <= e1
       j += (ws.off[m] == e1) ? m : m - 1;
       __syncwarp();
-      if (ws.n >= kWarpQueue / 2) warp_flush<DEFER>(c, ws, nxt);
+      if (qn > kWarpQueue - kWarpTile) {  // the next tile's might not fit
+        warp_resolve<ALG, DEFER>(c, ws, a, nxt, qn, thr, hs);
+        qn = 0;
+      }
     }
   }
-  warp_flush<DEFER>(c, ws, nxt);
+  if (qn) warp_resolve<ALG, DEFER>(c, ws, a, nxt, qn, thr, hs);
   if (DEFER && hs.h) block_hist_end(hs.h, c.hist);
   __syncthreads();
   return block_epilogue(c, s, a, i, cur, nxt, old, active);
@@ -1334,6 +1379,8 @@ __device__ __forceinline__ bool body_pull(const Ctx& c, Stage& s) {
           if (FRONTIER && !((bmc[u >> 5] >> (u & 31)) & 1u)) continue;
           const int du = c.dist[u];
           if (!Op<ALG>::valid(du)) continue;
+          // BFS stays level by level: a neighbour reached in this iteration waits
+          if (ALG == kBFS && !FRONTIER && du > i) continue;
           const int cd = Op<ALG>::cand(du, Op<ALG>::kWeighted ? ld_adj(ew + k) : 0);
           if (cd < best) {
             best = cd;

@@ -402,3 +402,34 @@ def test_pooled_memory_reuse_and_trim(gpu):
         if k == 1:
             i2.trim_device_memory()
     i2.trim_device_memory()
+
+
+@pytest.mark.parametrize("mid,leaves", [(1, 63), (1, 64), (1, 65), (2, 32), (3, 43), (64, 1), (65, 3), (129, 2),
+                                        (192, 1), (193, 5), (700, 64)])
+def test_queued_vertices_around_tile_and_queue_sizes(gpu, mid, leaves):
+    # source -> mid vertices -> leaves each: every edge lowers a value. The first
+    # half of each vertex's leaves are shared by all (repeats in one warp's
+    # queue), have no edges themselves (directed: never in a frontier) but for
+    # one chain that continues from the last leaf.
+    shared = leaves // 2
+    own = leaves - shared
+    n = 1 + mid + shared + mid * own + 3
+    u, v = [np.zeros(mid, np.int64)], [np.arange(1, 1 + mid)]
+    for k in range(mid):
+        u.append(np.full(leaves, 1 + k))
+        v.append(np.concatenate([1 + mid + np.arange(shared), 1 + mid + shared + k * own + np.arange(own)]))
+    last = n - 4
+    u.append(np.array([last, n - 3, n - 2]))
+    v.append(np.array([n - 3, n - 2, n - 1]))
+    u, v = np.concatenate(u), np.concatenate(v).astype(np.int32)
+    ni = np.zeros(n + 1, np.int32)
+    np.cumsum(np.bincount(u, minlength=n), out=ni[1:])
+    w = (1 + (np.arange(len(v)) * 7919) % 251).astype(np.int32)
+    g = i2.ECLGraph(n, len(v), ni, v, w)
+    dg = i2.DeviceGraph.upload(g)
+    for loop in (i2.I2_LOOP_GRAPH, i2.I2_LOOP_HOST):
+        np.testing.assert_array_equal(dg.bfs(0, loop=loop)[0], oracle.bfs(g, 0))
+        for budget in (0, 40):
+            np.testing.assert_array_equal(dg.sssp(0, loop=loop, budget=budget)[0], oracle.sssp(g, 0))
+        np.testing.assert_array_equal(dg.sssp(0, loop=loop, delta=60)[0], oracle.sssp(g, 0))
+    dg.free()
