@@ -107,7 +107,8 @@ typedef struct {
   int sssp_budget;  /* SSSP with I2_VP_CTA only, when sssp_delta <= 0: budgeted
                        near/far ordering. Each iteration relaxes only the frontier
                        vertices below a distance threshold that the engine sets on
-                       the device so that about `sssp_budget` edges lie below it
+                       the device so that about `sssp_budget` edges lie below it, or
+                       2 edges per entry of a large far pile,
                        (from distance histograms of the frontier, and of the far
                        pile when the frontier runs dry); the rest wait on the far
                        pile. 0: off; > 0: this many edges;

@@ -110,7 +110,7 @@ struct GStats {
 // atomicAdd hands out consistent positions in wl[] and offsets in woff[]; a
 // frontier holds each vertex at most once, so edges <= E < 2^31 never carries
 // into the entry count. The heavy list pairs entries with tiles the same way.
-struct Slot {
+struct alignas(128) Slot {    // a line of its own: every flush adds to `packed`
   unsigned long long packed;  // entries << 32 | edges
   unsigned long long hpacked; // heavy entries << 32 | heavy tiles
   int maxdeg;
@@ -120,19 +120,23 @@ struct Slot {
 __host__ __device__ __forceinline__ int slot_size(unsigned long long p) { return (int)(p >> 32); }
 __host__ __device__ __forceinline__ unsigned slot_edges(unsigned long long p) { return (unsigned)(p & 0xffffffffu); }
 
-struct Ctl {
-  Slot slot[3];
+// Control block of a traversal. Its head is the state of the current iteration.
+// Every block copies the head to shared memory in one coalesced read when the
+// iteration begins and takes all its decisions from the copy; the block that
+// finishes the iteration reads it once more (now with the accumulated counts),
+// advances it in shared memory and writes it back. (Read field by field from
+// global memory, the chain of dependent L2 reads cost about 8 us per iteration
+// between the last relaxation and the next start: grid 2000^2 BFS, 117
+// iterations, took 2,337 us and takes 1,735; SSSP on RMAT with 3,001 vertices,
+// 11 iterations, 213 and 163.)
+// Fields that blocks change with atomics during an iteration lie on lines of
+// their own behind the state; in the copy they are only good where this
+// iteration does not change them (slot[cur], slot[old], the pile that a move
+// reads).
+struct CtlHead {
   int iter;                 // index of the next relax launch
   int iter_cap;
-  int status;               // error bits, see kStatus*
   int variant;              // variant to run at the next launch
-  unsigned done;            // blocks finished in the current launch
-  int chunk;                // dynamic work counter of the current launch
-  int htile;                // dynamic heavy-tile counter of the current launch
-  int pad0;
-  unsigned long long tstart;// earliest block start of the current launch (globaltimer ns)
-  long long visited;        // vertices reached so far
-  int hist[kMaxVariants];   // launches per variant
   int mode;                 // 0 fixed, 1 heuristic, 2 learned, 3 fixed switch (then_at)
   int fixed_variant;
   int allowed;              // bitmask of variants allowed on this graph
@@ -163,23 +167,34 @@ struct Ctl {
   int hshift;               // histogram bin width 2^hshift (budget)
   int hbase;                // frontier histogram base of the current launch (budget)
   int pbase;                // pile histogram base (budget)
-  int pad2;
-  int pcur;
-  unsigned psize[2];
-  int pmin[2];              // lower bound of the values on each pile
+  int pcur;                 // current far pile
   int uf_phase;             // union-find CC: 1 after the hook launch (the compress launch follows)
+  int uf_giant;             // union-find CC: root of the sampled largest tree
   int then_at;              // mode 3: iteration from which then_variant runs
   int then_variant;
-  int uf_giant;             // union-find CC: root of the sampled largest tree
-  // Resident launches (one launch runs every iteration, the grid meeting at
-  // a barrier between them).
-  unsigned bar_gen;         // barrier generation, bumped once per iteration
   int go;                   // 1 while another iteration follows
   int hold;                 // test hook: the first release is withheld
-  int pad1;
   unsigned long long stall_ns;  // longest wait at the barrier before giving up
   unsigned long long relax_ns;  // sum of relax launch durations
   float feat[kFeatures];    // features of the frontier the next launch consumes
+  Slot slot[3];
+  // counts of the traversal, added to once per block
+  alignas(128) long long visited;  // vertices reached so far
+  unsigned long long tstart;// start of the current launch (globaltimer ns)
+  unsigned psize[2];        // entries of the far piles
+  int pmin[2];              // lower bound of the values on each pile
+  int chunk;                // dynamic work counter of the current launch
+  alignas(128) unsigned done;  // blocks finished in the current launch
+};
+constexpr int kHeadWords = sizeof(CtlHead) / 4;
+static_assert(kHeadWords <= kBlock, "one word of the head per thread");
+
+struct Ctl : CtlHead {
+  // Resident launches (one launch runs every iteration, the grid meeting at
+  // a barrier between them): the waiting blocks poll this line alone.
+  alignas(128) unsigned bar_gen;  // barrier generation, bumped once per iteration
+  int status;               // error bits, see kStatus*
+  int hist[kMaxVariants];   // launches per variant
 };
 
 // Union-find CC pays on graphs of 2^19 vertices or more, or of average degree
@@ -191,8 +206,8 @@ __host__ __device__ inline bool union_find_pays(long long nodes, float avgdeg) {
   return nodes >= (1LL << 19) || avgdeg < 6.f;
 }
 
-// Graphs on which the selectors' kernel is compiled for the fixed styles'
-// resident blocks per SM rather than I2_SEL_MIN_BLOCKS (relax.cuh).
+// Graphs on which the selectors' kernel is compiled for
+// I2_FIXED_MIN_BLOCKS resident blocks per SM rather than I2_SEL_MIN_BLOCKS (relax.cuh).
 constexpr long long kWideSelectorNodes = 1LL << 25;
 
 enum : int {

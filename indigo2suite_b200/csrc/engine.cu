@@ -112,7 +112,19 @@ __global__ void __launch_bounds__(kBlock) k_seed(Ctx c) {
   }
   __threadfence();
   __syncthreads();
-  select_next(c, 0, 0, true, -1);
+  // the head with the seeded frontier: its features, and the first style
+  __shared__ CtlHead S;
+  load_head(c, S);
+  __syncthreads();
+  if (threadIdx.x < kFeatures) {
+    const Slot& f = S.slot[0];
+    S.feat[threadIdx.x] = frontier_feature(threadIdx.x, c.gs, S.algo, 0, slot_size(f.packed), slot_size(f.hpacked),
+                                           slot_edges(f.packed), f.maxdeg, S.visited);
+  }
+  __syncthreads();
+  select_next(c, S, 0, 0, true, -1);
+  __syncthreads();
+  store_head(c, S);
 }
 
 // Per-run parameters, passed by value to k_reset so that queued runs never
@@ -123,9 +135,10 @@ struct RunParams {
 };
 
 __global__ void k_reset(Ctl* ctl, RunParams p) {
-  if (threadIdx.x != 0) return;
   unsigned* w = reinterpret_cast<unsigned*>(ctl);
-  for (unsigned k = 0; k < sizeof(Ctl) / sizeof(unsigned); ++k) w[k] = 0u;
+  for (unsigned k = threadIdx.x; k < sizeof(Ctl) / sizeof(unsigned); k += blockDim.x) w[k] = 0u;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
   for (int k = 0; k < 3; ++k) ctl->slot[k].mindist = kInf;
   ctl->tstart = ~0ull;
   ctl->iter_cap = p.iter_cap;

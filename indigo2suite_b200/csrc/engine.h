@@ -15,7 +15,7 @@ int grid_for(KernelFn fn, int max_per_sm);
 // relax_fn: one launch per iteration in style v; dispatch_fn: one launch per
 // iteration in the style the selectors picked; resident_fn: every iteration in
 // one launch, in style v or (v < 0) the selectors' per-iteration pick. `wide`:
-// the selectors' form compiled for the fixed styles' resident blocks per SM.
+// the selectors' form compiled for more resident blocks per SM (I2_FIXED_MIN_BLOCKS).
 template <int ALG>
 KernelFn relax_fn(int v);
 template <int ALG>

@@ -42,10 +42,12 @@ static __device__ int heuristic_pick(const GStats& gs, int algo, int allowed, in
   return ok(kVPCta) ? kVPCta : kVPThread;
 }
 
-// Executed by every thread of one block. Computes the features of the frontier
-// in slot `nxt`, picks the variant for the next launch and sets the loop
-// condition of the graph. `cond` tells whether another launch will happen;
-// `force` >= 0 overrides the pick (the compress launch of union-find CC).
+// Executed by every thread of one block, on the head S in shared memory: picks
+// the variant for the next launch from the frontier in slot `nxt`, whose
+// features the caller has put into S.feat, and sets go (and, when the
+// traversal ends, the loop condition of the graph). `cond` tells whether
+// another launch will happen; `force` >= 0 overrides the pick (the compress
+// launch of union-find CC).
 // The learned selector is re-evaluated when the frontier's entries or edges
 // moved by more than a factor 1.5 since its last evaluation, or 16 iterations
 // passed; otherwise the previous choice stands (long tails of small, similar
@@ -53,62 +55,62 @@ static __device__ int heuristic_pick(const GStats& gs, int algo, int allowed, in
 // than any it was trained on it defers to the frequency rule (no inference):
 // measured on RMAT-24 and RMAT-26 BFS, its picks there cost 1.08-1.38x the
 // rule's time even with the size features clamped to the training range.
-static __device__ void select_next(const Ctx& c, int next_iter, int nxt, bool cond, int force) {
-  __shared__ float x[kFeatures], h1[kHidden], h2[kHidden], y[kOut];
-  __shared__ int s_eval;
-  Ctl* ctl = c.ctl;
-  if (threadIdx.x == 0) {
-    volatile Slot* sl = &ctl->slot[nxt];
-    const unsigned long long p = sl->packed;
-    const int n = slot_size(p);
-    const unsigned e = slot_edges(p);
-    frontier_features(c.gs, ctl->algo, next_iter, n, slot_size(sl->hpacked), e, sl->maxdeg,
-                      *(volatile long long*)&ctl->visited, x);
-    for (int k = 0; k < kFeatures; ++k) ctl->feat[k] = x[k];
-    const long long sn = ctl->sel_n, se = ctl->sel_e;
-    s_eval = next_iter == 0 || 2LL * n > 3LL * sn || 3LL * n < 2LL * sn || 2LL * e > 3LL * se ||
-             3LL * e < 2LL * se || next_iter - ctl->sel_iter >= 16;
-  }
-  __syncthreads();
-  const int mode = ctl->mode;
+static __device__ void select_next(const Ctx& c, CtlHead& S, int next_iter, int nxt, bool cond, int force) {
+  __shared__ float h1[kHidden], h2[kHidden], y[kOut];
+  const unsigned long long p = S.slot[nxt].packed;
+  const int n = slot_size(p);
+  const unsigned e = slot_edges(p);
+  const int mode = S.mode;
   const bool learned = c.mlp && c.gs.nodes <= kMaxTrainedNodes;
-  const bool infer = mode == 2 && learned && cond && s_eval && force < 0;
-  if (infer) mlp_forward_block(c.mlp, x, h1, h2, y);
+  const long long sn = S.sel_n, se = S.sel_e;
+  const bool moved = next_iter == 0 || 2LL * n > 3LL * sn || 3LL * n < 2LL * sn || 2LL * e > 3LL * se ||
+                     3LL * e < 2LL * se || next_iter - S.sel_iter >= 16;
+  const bool infer = mode == 2 && learned && cond && moved && force < 0;
+  if (infer) mlp_forward_block(c.mlp, S.feat, h1, h2, y);
   if (threadIdx.x == 0) {
-    int v = ctl->fixed_variant;
+    int v = S.fixed_variant;
     if (mode == 3) {
-      v = next_iter >= ctl->then_at ? ctl->then_variant : ctl->fixed_variant;
-    } else if ((mode == 1 || mode == 2) && union_find_first(c.gs, ctl->algo, ctl->allowed, next_iter)) {
+      v = next_iter >= S.then_at ? S.then_variant : S.fixed_variant;
+    } else if ((mode == 1 || mode == 2) && union_find_first(c.gs, S.algo, S.allowed, next_iter)) {
       v = kUnionFind;
     } else if (mode == 1 || (mode == 2 && !learned)) {
-      volatile Slot* sl = &ctl->slot[nxt];
-      const unsigned long long p = sl->packed;
-      v = heuristic_pick(c.gs, ctl->algo, ctl->allowed, slot_size(p), slot_edges(p));
+      v = heuristic_pick(c.gs, S.algo, S.allowed, n, e);
     } else if (mode == 2) {
-      v = ctl->variant;
+      v = S.variant;
       if (infer) {
-        volatile Slot* sl = &ctl->slot[nxt];
-        const unsigned long long p = sl->packed;
-        const int h = heuristic_pick(c.gs, ctl->algo, ctl->allowed, slot_size(p), slot_edges(p));
+        const int h = heuristic_pick(c.gs, S.algo, S.allowed, n, e);
         float best = 3.0e38f;
         int bv = -1;
         for (int k = 0; k < kOut; ++k)  // per-iteration styles only (see union_find_first)
-          if (k != kUnionFind && ((ctl->allowed >> k) & 1) && y[k] < best) {
+          if (k != kUnionFind && ((S.allowed >> k) & 1) && y[k] < best) {
             best = y[k];
             bv = k;
           }
         v = (bv >= 0 && best + kLearnedMargin < y[h]) ? bv : h;
-        ctl->sel_n = slot_size(p);
-        ctl->sel_e = slot_edges(p);
-        ctl->sel_iter = next_iter;
+        S.sel_n = n;
+        S.sel_e = e;
+        S.sel_iter = next_iter;
       }
     }
     if (force >= 0) v = force;
-    ctl->variant = v;
-    if (cond) ctl->hist[v] += 1;
-    ctl->go = cond ? 1 : 0;
-    if (c.use_loop) cudaGraphSetConditional((cudaGraphConditionalHandle)c.loop_h, cond ? 1u : 0u);
+    S.variant = v;
+    if (cond) atomicAdd(&c.ctl->hist[v], 1);
+    S.go = cond ? 1 : 0;
+    // the graph's loop condition starts at 1 and keeps its value between launches
+    if (c.use_loop && !cond) cudaGraphSetConditional((cudaGraphConditionalHandle)c.loop_h, 0u);
   }
+}
+
+// Edges that the next near set should carry: the budget, or more where the
+// far pile is large. A move reads the whole pile, about 20 ps an entry, which
+// is the time of 2 relaxed edges; near sets of fewer edges than that spend
+// most of the traversal in moves. RMAT-25 ordered (12 M entries on the pile),
+// ms: no growth 16.7 (25 moves, 5.6 ms), 1 edge per entry 14.7, 2 14.1,
+// 3 15.8; RMAT-22 (2 M entries), where the budget is the larger: 2.07 with all.
+constexpr long long kMoveEdgesPerEntry = 2;
+static __device__ __forceinline__ long long near_budget(const CtlHead& S) {
+  const int np = S.split == 1 ? 1 - S.pcur : S.pcur;  // the pile the next move reads
+  return max(-(long long)S.delta, kMoveEdgesPerEntry * (long long)S.psize[np]);
 }
 
 // Edge budget of the SSSP near/far ordering (whole block; kBlock bins): the
@@ -116,10 +118,10 @@ static __device__ void select_next(const Ctx& c, int next_iter, int nxt, bool co
 // (kHistBins if it never does): [0] the next frontier's, [1] the pile's. The
 // next frontier's histogram is then cleared for the next launch's pushes.
 static_assert(kHistBins == kBlock, "one histogram bin per thread");
-static __device__ void budget_quantiles(const Ctx& c, int* q) {
+static __device__ void budget_quantiles(const Ctx& c, const CtlHead& S, int* q) {
   __shared__ unsigned long long part[kBlock / kWarp];
   __shared__ int sq[2];
-  const unsigned long long B = (unsigned long long)(-(long long)c.ctl->delta);
+  const unsigned long long B = (unsigned long long)near_budget(S);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   for (int which = 0; which < 2; ++which) {
     unsigned long long* h = c.hist + which * kHistBins;
@@ -145,134 +147,147 @@ static __device__ void budget_quantiles(const Ctx& c, int* q) {
 // `q` are the histogram quantiles, `n`/`e` the next frontier's entries and
 // edges. Returns whether another launch follows; *clear_pile is set when the
 // pile histogram must be cleared (a move rebuilds it from the entries it keeps).
-static __device__ int budget_next(const Ctx& c, const int* q, long long n, unsigned e, int nxt, int* clear_pile) {
-  Ctl* ctl = c.ctl;
-  const long long B = -(long long)ctl->delta;
-  const int shift = ctl->hshift;
-  const int was = ctl->split;
-  const int p = ctl->pcur;
+static __device__ int budget_next(CtlHead& S, const int* q, long long n, unsigned e, int nxt, int* clear_pile) {
+  const long long B = -(long long)S.delta, near = near_budget(S);
+  const int shift = S.hshift;
+  const int was = S.split;
+  const int p = S.pcur;
   int cond = n > 0;
   *clear_pile = 0;
   if (was == 1) {  // the move emptied pile p onto the other one
-    ctl->psize[p] = 0;
-    ctl->pmin[p] = kInf;
-    ctl->pcur = 1 - p;
+    S.psize[p] = 0;
+    S.pmin[p] = kInf;
+    S.pcur = 1 - p;
   }
-  ctl->split = 0;
-  const int np = ctl->pcur;
+  S.split = 0;
+  const int np = S.pcur;
   // move next when the frontier is empty, or so small that its last
   // iterations would cost more launches than edges (it is carried along)
-  if (*(volatile unsigned*)&ctl->psize[np] > 0 && (n == 0 || (was == 0 && (long long)e * 16 < B))) {
+  if (S.psize[np] > 0 && (n == 0 || (was == 0 && (long long)e * 16 < B))) {
     // at the budget's quantile of the pile (and above the pile's lower bound,
     // so that a live entry moves, or the move learns the bound)
-    const int pm = *(volatile int*)&ctl->pmin[np];
-    long long T = q[1] < kHistBins ? (long long)ctl->pbase + ((long long)(q[1] + 1) << shift) : (long long)kInf;
+    const int pm = S.pmin[np];
+    long long T = q[1] < kHistBins ? (long long)S.pbase + ((long long)(q[1] + 1) << shift) : (long long)kInf;
     if (pm != kInf) T = max(T, (long long)pm + 1);
     T = min(T, (long long)kInf);
-    ctl->prev_threshold = ctl->threshold;
-    ctl->threshold = (int)T;
-    int lo = pm != kInf ? pm : ctl->pbase;  // the smallest value the move can carry
-    if (n > 0) lo = min(lo, *(volatile int*)&ctl->slot[nxt].mindist);
-    ctl->hbase = lo;
-    ctl->pbase = (int)T;                       // kept values are at or above T
-    ctl->split = 1;
+    S.prev_threshold = S.threshold;
+    S.threshold = (int)T;
+    int lo = pm != kInf ? pm : S.pbase;  // the smallest value the move can carry
+    if (n > 0) lo = min(lo, S.slot[nxt].mindist);
+    S.hbase = lo;
+    S.pbase = (int)T;                       // kept values are at or above T
+    S.split = 1;
     *clear_pile = 1;
     return 1;
   }
-  if (n > 0 && was != 3 && (long long)e > 2 * B && q[0] < kHistBins) {
-    const long long T = (long long)ctl->hbase + ((long long)(q[0] + 1) << shift);
-    if (T < (long long)ctl->threshold) {  // trim the next frontier to about B edges
-      ctl->threshold = (int)T;
-      ctl->split = 3;
+  if (n > 0 && was != 3 && (long long)e > 2 * near && q[0] < kHistBins) {
+    const long long T = (long long)S.hbase + ((long long)(q[0] + 1) << shift);
+    if (T < (long long)S.threshold) {  // trim the next frontier to about that many edges
+      S.threshold = (int)T;
+      S.split = 3;
     }
   }
-  ctl->hbase = *(volatile int*)&ctl->slot[nxt].mindist;
+  S.hbase = S.slot[nxt].mindist;
   return cond;
 }
 
 // Last block of a relax launch: record the launch, advance the iteration and
-// decide whether the loop continues.
-static __device__ void finish_iteration(const Ctx& c, int i, int cur, int nxt, int old) {
+// decide whether the loop continues. The head is read once (with the counts
+// that every block has added), advanced in shared memory by thread 0 while the
+// second warp writes the record and computes the next frontier's features, and
+// written back with one store per thread.
+static __device__ __forceinline__ void finish_iteration(const Ctx& c, CtlHead& S, int i, int cur, int nxt, int old) {
   __shared__ int s_cond, s_force, s_clear;
   __shared__ int s_q[2];
-  Ctl* ctl = c.ctl;
-  if (ctl->variant == kUnionFind && ctl->uf_phase == 0) uf_sample_giant(c);  // whole block
+  const unsigned long long t1 = globaltimer();
+  load_head(c, S);
   if (threadIdx.x == 0) s_clear = 0;
-  if (ctl->delta < 0) {
+  __syncthreads();
+  if (S.variant == kUnionFind && S.uf_phase == 0) uf_sample_giant(c, S);  // whole block
+  if (S.delta < 0) {
     int q[2];
-    budget_quantiles(c, q);
+    budget_quantiles(c, S, q);
     if (threadIdx.x == 0) {
       s_q[0] = q[0];
       s_q[1] = q[1];
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    const unsigned long long t1 = globaltimer();
-    const unsigned long long dt = t1 - ctl->tstart;
-    ctl->relax_ns += dt;
-    volatile Slot* sc = &ctl->slot[cur];
+  const unsigned long long dt = t1 - S.tstart;
+  if (threadIdx.x / kWarp == 1) {
+    const int lane = threadIdx.x % kWarp;
     if (c.recs && i < c.rec_cap) {
       IterRec& r = c.recs[i];
-      r.iter = i;
-      r.variant = ctl->variant;
-      r.size = slot_size(sc->packed);
-      r.hsize = slot_size(sc->hpacked);
-      r.edges = slot_edges(sc->packed);
-      r.maxdeg = sc->maxdeg;
-      r.mindist = sc->mindist;
-      r.visited = *(volatile long long*)&ctl->visited;
-      r.t_ns = dt;
-      for (int k = 0; k < kFeatures; ++k) r.feat[k] = ctl->feat[k];
-      r.kind = ctl->split;
-      r.threshold = ctl->threshold;
-      r.pile = ctl->delta != 0 ? *(volatile unsigned*)&ctl->psize[ctl->split == 1 ? 1 - ctl->pcur : ctl->pcur] : 0u;
+      if (lane == 0) {
+        const Slot& f = S.slot[cur];
+        r.iter = i;
+        r.variant = S.variant;
+        r.size = slot_size(f.packed);
+        r.hsize = slot_size(f.hpacked);
+        r.edges = slot_edges(f.packed);
+        r.maxdeg = f.maxdeg;
+        r.mindist = f.mindist;
+        r.visited = S.visited;
+        r.t_ns = dt;
+        r.kind = S.split;
+        r.threshold = S.threshold;
+        r.pile = S.delta != 0 ? S.psize[S.split == 1 ? 1 - S.pcur : S.pcur] : 0u;
+      }
+      if (lane < kFeatures) r.feat[lane] = S.feat[lane];
     }
-    Slot& so = ctl->slot[old];
+    if (lane < kFeatures) {
+      const Slot& f = S.slot[nxt];
+      S.feat[lane] = frontier_feature(lane, c.gs, S.algo, i + 1, slot_size(f.packed), slot_size(f.hpacked),
+                                      slot_edges(f.packed), f.maxdeg, S.visited);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    S.relax_ns += dt;
+    Slot& so = S.slot[old];
     so.packed = 0;
     so.hpacked = 0;
     so.maxdeg = 0;
     so.mindist = kInf;
-    ctl->done = 0;
-    ctl->chunk = 0;
-    ctl->htile = 0;
-    ctl->tstart = ~0ull;
-    ctl->iter = i + 1;
-    volatile Slot* sn = &ctl->slot[nxt];
-    const long long n = slot_size(sn->packed);
+    S.done = 0;
+    S.chunk = 0;
+    S.tstart = ~0ull;
+    S.iter = i + 1;
+    const Slot& sn = S.slot[nxt];
+    const long long n = slot_size(sn.packed);
     int cond = n > 0;
-    if (ctl->delta < 0) {
-      cond = budget_next(c, s_q, n, slot_edges(sn->packed), nxt, &s_clear);
-    } else if (ctl->delta > 0) {
-      if (ctl->split) {  // this launch emptied pile pcur onto the other one
-        const int p = ctl->pcur;
-        ctl->psize[p] = 0;
-        ctl->pmin[p] = kInf;
-        ctl->pcur = 1 - p;
-        ctl->split = 0;
+    if (S.delta < 0) {
+      cond = budget_next(S, s_q, n, slot_edges(sn.packed), nxt, &s_clear);
+    } else if (S.delta > 0) {
+      if (S.split) {  // this launch emptied pile pcur onto the other one
+        const int p = S.pcur;
+        S.psize[p] = 0;
+        S.pmin[p] = kInf;
+        S.pcur = 1 - p;
+        S.split = 0;
       }
-      const int p = ctl->pcur;
-      if (n == 0 && *(volatile unsigned*)&ctl->psize[p] > 0) {
+      const int p = S.pcur;
+      if (n == 0 && S.psize[p] > 0) {
         // next launch splits the pile at a raised threshold
-        const long long lo = max((long long)ctl->threshold, (long long)*(volatile int*)&ctl->pmin[p]);
-        ctl->prev_threshold = ctl->threshold;
-        ctl->threshold = (int)min(lo + (long long)ctl->delta, (long long)kInf);
-        ctl->split = 1;
+        const long long lo = max((long long)S.threshold, (long long)S.pmin[p]);
+        S.prev_threshold = S.threshold;
+        S.threshold = (int)min(lo + (long long)S.delta, (long long)kInf);
+        S.split = 1;
         cond = 1;
       }
     }
     int force = -1;
-    if (ctl->variant == kUnionFind) {
-      if (ctl->uf_phase < 2) {  // the next union-find launch follows
-        ctl->uf_phase += 1;
+    if (S.variant == kUnionFind) {
+      if (S.uf_phase < 2) {  // the next union-find launch follows
+        S.uf_phase += 1;
         force = kUnionFind;
         cond = 1;
       } else {
-        ctl->uf_phase = 0;  // labels final; nothing was pushed
+        S.uf_phase = 0;  // labels final; nothing was pushed
       }
     }
-    if (cond && i + 1 >= ctl->iter_cap) {
-      ctl->status |= kStatusIterCap;
+    if (cond && i + 1 >= S.iter_cap) {
+      atomicOr(&c.ctl->status, kStatusIterCap);
       cond = 0;
     }
     s_cond = cond;
@@ -280,7 +295,9 @@ static __device__ void finish_iteration(const Ctx& c, int i, int cur, int nxt, i
   }
   __syncthreads();
   if (s_clear) c.hist[kHistBins + threadIdx.x] = 0ull;  // read above; the move rebuilds it
-  select_next(c, i + 1, nxt, s_cond != 0, s_force);
+  select_next(c, S, i + 1, nxt, s_cond != 0, s_force);
+  __syncthreads();
+  store_head(c, S);
 }
 
 }  // namespace i2

@@ -28,7 +28,7 @@ KernelFn relax_fn(int v) {
 
 template <int ALG>
 KernelFn dispatch_fn(bool wide) {
-  return wide ? relax_dispatch<ALG, I2_EB_MIN_BLOCKS> : relax_dispatch<ALG>;
+  return wide ? relax_dispatch<ALG, I2_FIXED_MIN_BLOCKS> : relax_dispatch<ALG>;
 }
 
 template <int ALG>
@@ -47,7 +47,7 @@ KernelFn resident_fn(int v, bool wide) {
       return nullptr;
   }
   // per-iteration pick
-  return wide ? relax_resident<ALG, -1, false, I2_EB_MIN_BLOCKS> : relax_resident<ALG, -1>;
+  return wide ? relax_resident<ALG, -1, false, I2_FIXED_MIN_BLOCKS> : relax_resident<ALG, -1>;
 }
 
 }  // namespace i2

@@ -36,12 +36,7 @@ namespace i2 {
 namespace cg = cooperative_groups;
 
 constexpr int kScanItems = kQueue / kBlock;                 // staged entries per thread in a flush
-// Edges per lane of the edge-balanced tile, and the resident blocks per SM its
-// kernels are compiled for (which bounds their registers: 6 -> 40 per thread).
-// Measured on RMAT-22 and a 2048^2 grid (ms, SSSP / BFS / CC on RMAT):
-// 2 edges at 6 blocks 2.65 / 1.12 / 2.21 (default), 4 at 5 blocks 2.80 / 1.14
-// / 2.23, 3 at 5 2.78 / 1.14 / 2.30, 1 at 8 3.11 / 1.24 / 2.39; 2 at 7 or 8
-// blocks and 4 at 6 spill and run 1.2-2x slower.
+// Edges per lane of the edge-balanced tile (measured beside I2_EB_MIN_BLOCKS).
 #ifndef I2_EB_EDGES
 #define I2_EB_EDGES 2
 #endif
@@ -138,12 +133,10 @@ __device__ __forceinline__ int heavy_tiles(int deg) { return (deg + kHeavyTile -
 // S is any shared struct with `Acc red[kBlock / kWarp]` and `int last`.
 template <typename S>
 __device__ __forceinline__ void acc_reduce(Acc a, S& s) {
-  for (int o = 16; o > 0; o >>= 1) {
-    a.maxdeg = max(a.maxdeg, __shfl_down_sync(0xffffffffu, a.maxdeg, o));
-    a.mindist = min(a.mindist, __shfl_down_sync(0xffffffffu, a.mindist, o));
-    a.visited += __shfl_down_sync(0xffffffffu, a.visited, o);
-    a.fmin = min(a.fmin, __shfl_down_sync(0xffffffffu, a.fmin, o));
-  }
+  a.maxdeg = __reduce_max_sync(0xffffffffu, a.maxdeg);
+  a.mindist = __reduce_min_sync(0xffffffffu, a.mindist);
+  a.visited = __reduce_add_sync(0xffffffffu, a.visited);
+  a.fmin = __reduce_min_sync(0xffffffffu, a.fmin);
   __syncthreads();
   if ((threadIdx.x & 31) == 0) s.red[threadIdx.x >> 5] = a;
   __syncthreads();
@@ -221,10 +214,10 @@ __device__ __forceinline__ void hist_far(const Hists& hs, int val, int deg) {
 // the pile is full: the caller then pushes v into the next frontier, which is
 // always valid. With the edge budget (hs) new entries are histogrammed.
 struct WarpStage;
-__device__ __forceinline__ bool stage_far(const Ctx& c, WarpStage* ws, int v, int deg);
+__device__ __forceinline__ bool stage_far(const Ctx& c, int pile, WarpStage* ws, int v, int deg);
 
-__device__ __forceinline__ bool defer_vertex(const Ctx& c, Acc& a, int v, int val, WarpStage* ws = nullptr,
-                                             const Hists* hs = nullptr) {
+__device__ __forceinline__ bool defer_vertex(const Ctx& c, Acc& a, int pile, int v, int val, WarpStage* ws,
+                                             const Hists* hs) {
   const unsigned bit = 1u << (v & 31);
   unsigned* w = &c.fbm[v >> 5];
   if (*(volatile unsigned*)w & bit) {
@@ -240,7 +233,7 @@ __device__ __forceinline__ bool defer_vertex(const Ctx& c, Acc& a, int v, int va
     atomicAnd(w, ~bit);
     return true;
   }
-  if (ws ? !stage_far(c, ws, v, deg) : !pile_append(c, c.ctl->pcur, v, deg)) {
+  if (!stage_far(c, pile, ws, v, deg)) {
     atomicAnd(w, ~bit);
     return false;
   }
@@ -505,8 +498,8 @@ __device__ __forceinline__ void block_share(unsigned total, int nb, unsigned* lo
 // entries. Each block takes a contiguous share of the tile sequence, finds the
 // vertex of its first tile once, and walks forward.
 template <int ALG>
-__device__ void heavy_path(const Ctx& c, Stage& s, Acc& a, int cur, int nxt, int active) {
-  const unsigned long long hp = c.ctl->slot[cur].hpacked;
+__device__ void heavy_path(const Ctx& c, const CtlHead& S, Stage& s, Acc& a, int cur, int nxt, int active) {
+  const unsigned long long hp = S.slot[cur].hpacked;
   const int nh = slot_size(hp);
   const unsigned ntiles = slot_edges(hp);
   if (ntiles == 0) return;
@@ -535,8 +528,8 @@ __device__ void heavy_path(const Ctx& c, Stage& s, Acc& a, int cur, int nxt, int
 
 // Clear the bitmap of F_{i-1} (slot old): by entries when it is small, by
 // words otherwise. Spread over the launch's `active` blocks.
-__device__ __forceinline__ void clear_old(const Ctx& c, int old, int active) {
-  const int n = slot_size(c.ctl->slot[old].packed);
+__device__ __forceinline__ void clear_old(const Ctx& c, const CtlHead& S, int old, int active) {
+  const int n = slot_size(S.slot[old].packed);
   unsigned* bm = c.bm[old];
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)active * blockDim.x;
@@ -548,13 +541,34 @@ __device__ __forceinline__ void clear_old(const Ctx& c, int old, int active) {
   }
 }
 
-static __device__ void finish_iteration(const Ctx& c, int i, int cur, int nxt, int old);
+static __device__ __forceinline__ void finish_iteration(const Ctx& c, CtlHead& S, int i, int cur, int nxt, int old);
+
+// Copy the head of the control block to (or from) shared memory: one coalesced
+// access, from L2 (other blocks wrote it). Block-uniform; the caller synchronises.
+__device__ __forceinline__ void load_head(const Ctx& c, CtlHead& S) {
+  if (threadIdx.x < kHeadWords)
+    reinterpret_cast<unsigned*>(&S)[threadIdx.x] =
+        __ldcg(reinterpret_cast<const unsigned*>(static_cast<const CtlHead*>(c.ctl)) + threadIdx.x);
+}
+__device__ __forceinline__ void store_head(const Ctx& c, const CtlHead& S) {
+  if (threadIdx.x < kHeadWords)
+    __stcg(reinterpret_cast<unsigned*>(static_cast<CtlHead*>(c.ctl)) + threadIdx.x,
+           reinterpret_cast<const unsigned*>(&S)[threadIdx.x]);
+}
+
+// Count this block into `done` (thread 0, after the block's writes and a block
+// barrier): they are visible to the block that finishes the iteration.
+__device__ __forceinline__ unsigned arrive(const Ctx& c) {
+  unsigned t;
+  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(t) : "l"(&c.ctl->done) : "memory");
+  return t;
+}
 
 // Blocks of a launch that take part in it. Blocks at or above this index
 // return at once, so a small frontier does not pay for the whole grid; the
 // clearing of F_{i-1} is work too. Full sweeps pass `need` = gridDim.x.
-__device__ __forceinline__ int active_blocks(const Ctx& c, int old, long long need) {
-  const int n_old = slot_size(c.ctl->slot[old].packed);
+__device__ __forceinline__ int active_blocks(const Ctx& c, const CtlHead& S, int old, long long need) {
+  const int n_old = slot_size(S.slot[old].packed);
   const long long clear = ((long long)n_old * 4 > c.bm_words) ? ((long long)c.bm_words + 8191) / 8192
                                                                 : ((long long)n_old + 2047) / 2048;
   long long a = need > clear ? need : clear;
@@ -566,9 +580,9 @@ __device__ __forceinline__ int active_blocks(const Ctx& c, int old, long long ne
 // Common epilogue: publish block statistics and let the last block finish the
 // iteration. Every block of the launch, active or not, counts into `done`, so
 // the iteration advances only after every block has read its state.
-template <typename S>
-__device__ __forceinline__ bool block_epilogue(const Ctx& c, S& s, const Acc& a, int i, int cur, int nxt, int old,
-                                               int /*active*/) {
+template <typename Sh>
+__device__ __forceinline__ bool block_epilogue(const Ctx& c, CtlHead& S, Sh& s, const Acc& a, int i, int cur, int nxt,
+                                               int old) {
   acc_reduce(a, s);
   if (threadIdx.x == 0) {
     const Acc& r = s.red[0];
@@ -577,39 +591,27 @@ __device__ __forceinline__ bool block_epilogue(const Ctx& c, S& s, const Acc& a,
     if (r.mindist != kInf) atomicMin(&sl.mindist, r.mindist);
     if (r.visited) atomicAdd((unsigned long long*)&c.ctl->visited, (unsigned long long)r.visited);
     // far pushes of a relax or trim launch go onto pile pcur, a move's onto the other
-    if (r.fmin != kInf) atomicMin(&c.ctl->pmin[c.ctl->split == 1 ? 1 - c.ctl->pcur : c.ctl->pcur], r.fmin);
-    __threadfence();
-    const unsigned t = atomicAdd(&c.ctl->done, 1u);
-    s.last = (t == gridDim.x - 1);
+    if (r.fmin != kInf) atomicMin(&c.ctl->pmin[S.split == 1 ? 1 - S.pcur : S.pcur], r.fmin);
+    s.last = (arrive(c) == gridDim.x - 1);
   }
   __syncthreads();
   const bool last = s.last;
-  if (last) {
-    __threadfence();
-    finish_iteration(c, i, cur, nxt, old);
-  }
+  if (last) finish_iteration(c, S, i, cur, nxt, old);
+  return last;  // this block finished the iteration
+}
+
+// Epilogue of a block with no work in this launch.
+template <typename Sh>
+__device__ __forceinline__ bool idle_epilogue(const Ctx& c, CtlHead& S, Sh& s, int i, int cur, int nxt, int old) {
+  if (threadIdx.x == 0) s.last = (arrive(c) == gridDim.x - 1);
+  __syncthreads();
+  const bool last = s.last;
+  if (last) finish_iteration(c, S, i, cur, nxt, old);
   return last;  // this block finished the iteration
 }
 
 // The launch's start time is taken by block 0, which the scheduler dispatches
 // first; the last block reads it after every block has finished.
-// Epilogue of a block with no work in this launch.
-template <typename S>
-__device__ __forceinline__ bool idle_epilogue(const Ctx& c, S& s, int i, int cur, int nxt, int old) {
-  if (threadIdx.x == 0) {
-    __threadfence();
-    const unsigned t = atomicAdd(&c.ctl->done, 1u);
-    s.last = (t == gridDim.x - 1);
-  }
-  __syncthreads();
-  const bool last = s.last;
-  if (last) {
-    __threadfence();
-    finish_iteration(c, i, cur, nxt, old);
-  }
-  return last;  // this block finished the iteration
-}
-
 __device__ __forceinline__ void block_prologue(const Ctx& c) {
   if (blockIdx.x == 0 && threadIdx.x == 0) c.ctl->tstart = globaltimer();
 }
@@ -619,20 +621,20 @@ __device__ __forceinline__ void block_prologue(const Ctx& c) {
 // vertex. Heavy vertices are skipped here and taken by the heavy path.
 
 template <int ALG, int VAR>
-__device__ __forceinline__ bool body_push(const Ctx& c, Stage& s) {
+__device__ __forceinline__ bool body_push(const Ctx& c, CtlHead& S, Stage& s) {
   block_prologue(c);
-  const int i = c.ctl->iter;
+  const int i = S.iter;
   const int cur = i % 3, nxt = (i + 1) % 3, old = (i + 2) % 3;
-  const int n = slot_size(c.ctl->slot[cur].packed);
+  const int n = slot_size(S.slot[cur].packed);
   const int per = VAR == kVPThread ? kBlock : (VAR == kVPWarp ? kBlock / kWarp : 1);
-  const int active = active_blocks(c, old, ((long long)n + per - 1) / per + slot_edges(c.ctl->slot[cur].hpacked));
+  const int active = active_blocks(c, S, old, ((long long)n + per - 1) / per + slot_edges(S.slot[cur].hpacked));
   if (blockIdx.x >= active) {
-    return idle_epilogue(c, s, i, cur, nxt, old);
+    return idle_epilogue(c, S, s, i, cur, nxt, old);
   }
   stage_init(s);
   Acc a;
   acc_init(a);
-  clear_old(c, old, active);
+  clear_old(c, S, old, active);
   __syncthreads();
   const int* wl = c.wl[cur];
 
@@ -667,9 +669,9 @@ __device__ __forceinline__ bool body_push(const Ctx& c, Stage& s) {
     }
     stage_flush_if_half(c, s, nxt);
   }
-  heavy_path<ALG>(c, s, a, cur, nxt, active);
+  heavy_path<ALG>(c, S, s, a, cur, nxt, active);
   stage_flush(c, s, nxt);
-  return block_epilogue(c, s, a, i, cur, nxt, old, active);
+  return block_epilogue(c, S, s, a, i, cur, nxt, old);
 }
 
 // ---------------------------------------------------------------------------
@@ -719,14 +721,14 @@ __device__ __forceinline__ void warp_stage_entry(const Ctx& c, WarpStage& ws, Ac
 // Stage a far-pile entry of the near/far ordering: kept in the warp's queue
 // as ~v (negative) beside its degree, and published by warp_publish<true>.
 // Without room in the queue it is appended at once.
-__device__ __forceinline__ bool stage_far(const Ctx& c, WarpStage* ws, int v, int deg) {
+__device__ __forceinline__ bool stage_far(const Ctx& c, int pile, WarpStage* ws, int v, int deg) {
   const int p = atomicAdd(&ws->n, 1);
   if (p < kWarpQueue) {
     ws->q[p] = ~v;
     ws->qd[p] = deg;
     return true;
   }
-  return pile_append(c, c.ctl->pcur, v, deg);
+  return pile_append(c, pile, v, deg);
 }
 
 // Publish the warp's resolved queue entries [0, n) (warp-uniform call): q[j] a
@@ -736,7 +738,7 @@ __device__ __forceinline__ bool stage_far(const Ctx& c, WarpStage* ws, int v, in
 // pile with one more atomic. Far entries that find the pile full join the next
 // frontier. Lane l owns the entries l, l + 32, ...
 template <bool DEFER = false>
-__device__ __forceinline__ void warp_publish(const Ctx& c, WarpStage& ws, int nxt, int n) {
+__device__ __forceinline__ void warp_publish(const Ctx& c, WarpStage& ws, int nxt, int n, int pile) {
   constexpr int kPer = kWarpQueue / kWarp;
   const int lane = threadIdx.x & 31;
   if constexpr (DEFER) {
@@ -753,7 +755,7 @@ __device__ __forceinline__ void warp_publish(const Ctx& c, WarpStage& ws, int nx
     }
     const int ftot = __shfl_sync(0xffffffffu, fincl, 31);
     if (ftot) {
-      const int p = c.ctl->pcur;
+      const int p = pile;
       unsigned pb = 0;
       if (lane == 0) pb = atomicAdd(&c.ctl->psize[p], (unsigned)ftot);
       pb = __shfl_sync(0xffffffffu, pb, 0);
@@ -822,7 +824,7 @@ __device__ __forceinline__ void warp_publish(const Ctx& c, WarpStage& ws, int nx
 // to relax in any style, and the bit keeps its visit counted once.
 template <int ALG, bool DEFER>
 __device__ __forceinline__ void warp_resolve(const Ctx& c, WarpStage& ws, Acc& a, int nxt, int n, int thr,
-                                             const Hists& hs) {
+                                             const Hists& hs, int pile) {
   constexpr int kPer = kWarpQueue / kWarp;
   constexpr int kPart = 3;
   static_assert(kPer % kPart == 0, "whole parts");
@@ -883,7 +885,7 @@ __device__ __forceinline__ void warp_resolve(const Ctx& c, WarpStage& ws, Acc& a
       if (j < n) ws.qd[j] = won ? deg[r] : 0;
     }
   }
-  warp_publish<DEFER>(c, ws, nxt, n);
+  warp_publish<DEFER>(c, ws, nxt, n, pile);
 }
 
 // Relax this lane's candidate edges and queue the vertices whose values fell:
@@ -931,18 +933,28 @@ struct EpiStage {
   int last;
 };
 
+// Resident blocks per SM that the edge-balanced kernels are compiled for: 5
+// leaves them 48 registers, no spills but 48 bytes in the near/far form (6: 40
+// registers, 192 bytes there). ER 2M SSSP 1,318 us (6 blocks 1,367; 4 blocks
+// 1,323), RMAT-22 near/far 2,007 (2,238; 2,057), RMAT-25 ordered 16,213
+// (17,455; 17,664); 3 edges per lane at 5 and 4 blocks 1,396 and 1,342, 2,025
+// and 1,967, 16,288 and 16,608.
 #ifndef I2_EB_MIN_BLOCKS
-#define I2_EB_MIN_BLOCKS 6
+#define I2_EB_MIN_BLOCKS 5
+#endif
+// ... and the other fixed styles' kernels, and the selectors' on the largest graphs.
+#ifndef I2_FIXED_MIN_BLOCKS
+#define I2_FIXED_MIN_BLOCKS 6
 #endif
 // Resident blocks per SM that the selectors' kernels (every style in one
-// kernel) are compiled for: 4 leaves them 64 registers, where 6 (the fixed
-// styles' 40) spilled 160-224 bytes per thread. Held-out RMAT/ER/grid graphs
+// kernel) are compiled for: 4 leaves them 64 registers, where 6 (40 registers)
+// spilled 160-224 bytes per thread. Held-out RMAT/ER/grid graphs
 // of 2^18 and 2^20 vertices, geomean time against 6: BFS 0.90, SSSP 0.97-0.98,
 // CC 0.97-0.98 for both selectors (5 blocks: 0.93-0.98); grid 4096² BFS 0.92.
 // On RMAT-26 the heuristic BFS took 1.21x as long at 4 blocks (its pull
 // iterations over 2^26 vertices need the warps), so graphs of
-// kWideSelectorNodes vertices or more get the selector kernel compiled for the
-// fixed styles' I2_EB_MIN_BLOCKS.
+// kWideSelectorNodes vertices or more get the selector kernel compiled for
+// I2_FIXED_MIN_BLOCKS.
 #ifndef I2_SEL_MIN_BLOCKS
 #define I2_SEL_MIN_BLOCKS 4
 #endif
@@ -978,12 +990,12 @@ __device__ __forceinline__ void block_hist_end(const unsigned* h, unsigned long 
 
 // Publish a split launch's staged entries once there are `least` of them
 // (warp-uniform call).
-__device__ __forceinline__ void split_flush(const Ctx& c, WarpStage& ws, int nxt, int least) {
+__device__ __forceinline__ void split_flush(const Ctx& c, WarpStage& ws, int nxt, int least, int pile) {
   __syncwarp();
   const int n = min(ws.n, kWarpQueue);
   __syncwarp();
   if (n < least) return;
-  warp_publish<true>(c, ws, nxt, n);
+  warp_publish<true>(c, ws, nxt, n, pile);
   if ((threadIdx.x & 31) == 0) ws.n = 0;
   __syncwarp();
 }
@@ -1004,30 +1016,29 @@ __device__ __forceinline__ void split_flush(const Ctx& c, WarpStage& ws, int nxt
 //    others onto the pile (nothing is relaxed).
 // The loop is block-uniform: a block appends the entries it keeps with one
 // atomic per pass (a single pile counter takes every block's appends).
-__device__ __forceinline__ bool body_split(const Ctx& c, EBSharedFar& sh, int i, int cur, int nxt, int old) {
+__device__ __forceinline__ bool body_split(const Ctx& c, CtlHead& S, EBSharedFar& sh, int i, int cur, int nxt, int old) {
   __shared__ int s_keep[kWarpsPerBlock];
   __shared__ unsigned s_kbase;
   EpiStage& s = sh.s;
-  Ctl* ctl = c.ctl;
-  const int mode = ctl->split;
-  const bool budget = ctl->delta < 0;
-  const int p = ctl->pcur;
-  const unsigned long long P = ctl->slot[cur].packed;
+  const int mode = S.split;
+  const bool budget = S.delta < 0;
+  const int p = S.pcur;
+  const unsigned long long P = S.slot[cur].packed;
   // F_i's entries first (a trim's input, or what an early move carries), then
   // the pile's (a move)
   const unsigned nf = (unsigned)slot_size(P);
-  const unsigned n = nf + (mode == 1 ? min(ctl->psize[p], c.pile_cap) : 0u);
-  const int T = ctl->threshold, T0 = ctl->prev_threshold;
-  const Hists hs = budget ? Hists{sh.hist, ctl->hbase, ctl->pbase, ctl->hshift} : Hists{};
-  const int active = active_blocks(c, old, ((long long)n + kBlock - 1) / kBlock);
+  const unsigned n = nf + (mode == 1 ? min(S.psize[p], c.pile_cap) : 0u);
+  const int T = S.threshold, T0 = S.prev_threshold;
+  const Hists hs = budget ? Hists{sh.hist, S.hbase, S.pbase, S.hshift} : Hists{};
+  const int active = active_blocks(c, S, old, ((long long)n + kBlock - 1) / kBlock);
   if (blockIdx.x >= active) {
-    return idle_epilogue(c, s, i, cur, nxt, old);
+    return idle_epilogue(c, S, s, i, cur, nxt, old);
   }
   if (threadIdx.x == 0) s.last = 0;
   Acc a;
   acc_init(a);
   if (budget) block_hist_begin(sh.hist);
-  clear_old(c, old, active);
+  clear_old(c, S, old, active);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   WarpStage& ws = sh.wss[wid];
   if (lane == 0) ws.n = 0;
@@ -1072,7 +1083,7 @@ __device__ __forceinline__ bool body_split(const Ctx& c, EBSharedFar& sh, int i,
       if (!in[r]) continue;
       const unsigned bit = 1u << (v[r] & 31);
       if (front[r]) {  // a frontier entry: below T it stays near, else it goes onto the pile
-        if (d[r] >= T && defer_vertex(c, a, v[r], d[r], &ws, budget ? &hs : nullptr)) {
+        if (d[r] >= T && defer_vertex(c, a, p, v[r], d[r], &ws, budget ? &hs : nullptr)) {
           // on the pile
         } else if (!(atomicOr(&c.bm[nxt][v[r] >> 5], bit) & bit)) {
           a.mindist = min(a.mindist, d[r]);
@@ -1121,7 +1132,7 @@ __device__ __forceinline__ bool body_split(const Ctx& c, EBSharedFar& sh, int i,
           s_keep[w] = t;
           t += x;
         }
-        s_kbase = t ? atomicAdd(&ctl->psize[1 - p], (unsigned)t) : 0u;
+        s_kbase = t ? atomicAdd(&c.ctl->psize[1 - p], (unsigned)t) : 0u;
       }
       __syncthreads();
       unsigned pos = s_kbase + (unsigned)s_keep[wid] + (unsigned)(incl - nkeep);
@@ -1137,44 +1148,44 @@ __device__ __forceinline__ bool body_split(const Ctx& c, EBSharedFar& sh, int i,
       }
       __syncthreads();  // s_keep and s_kbase are rewritten by the next pass
     }
-    split_flush(c, ws, nxt, kWarpQueue - kR * kWarp);
+    split_flush(c, ws, nxt, kWarpQueue - kR * kWarp, p);
   }
-  split_flush(c, ws, nxt, 1);
+  split_flush(c, ws, nxt, 1, p);
   if (budget) block_hist_end(sh.hist, c.hist);
   __syncthreads();
-  return block_epilogue(c, s, a, i, cur, nxt, old, active);
+  return block_epilogue(c, S, s, a, i, cur, nxt, old);
 }
 
 // DEFER: SSSP near/far ordering (pushes at or above the threshold go onto the
 // far pile, and split launches refill the frontier from it).
 template <int ALG, bool DEFER = false>
-__device__ __forceinline__ bool body_edge_balanced(const Ctx& c, EBSharedT<DEFER>& sh) {
+__device__ __forceinline__ bool body_edge_balanced(const Ctx& c, CtlHead& S, EBSharedT<DEFER>& sh) {
   static_assert(!DEFER || ALG == kSSSP, "near/far ordering is for SSSP");
   EpiStage& s = sh.s;
   block_prologue(c);
-  const int i = c.ctl->iter;
+  const int i = S.iter;
   const int cur = i % 3, nxt = (i + 1) % 3, old = (i + 2) % 3;
   if constexpr (DEFER) {
-    if (c.ctl->split) return body_split(c, sh, i, cur, nxt, old);
+    if (S.split) return body_split(c, S, sh, i, cur, nxt, old);
   }
-  const int thr = DEFER ? c.ctl->threshold : kInf;
+  const int thr = DEFER ? S.threshold : kInf;
   Hists hs{};
   if constexpr (DEFER) {
-    if (c.ctl->delta < 0) hs = Hists{sh.hist, c.ctl->hbase, c.ctl->pbase, c.ctl->hshift};
+    if (S.delta < 0) hs = Hists{sh.hist, S.hbase, S.pbase, S.hshift};
   }
-  const unsigned long long P = c.ctl->slot[cur].packed;
+  const unsigned long long P = S.slot[cur].packed;
   const int n = slot_size(P);
   const unsigned total = slot_edges(P);
-  const int active = active_blocks(c, old, ((long long)total + kWarpTile * kWarpsPerBlock - 1) /
+  const int active = active_blocks(c, S, old, ((long long)total + kWarpTile * kWarpsPerBlock - 1) /
                                               (kWarpTile * kWarpsPerBlock));
   if (blockIdx.x >= active) {
-    return idle_epilogue(c, s, i, cur, nxt, old);
+    return idle_epilogue(c, S, s, i, cur, nxt, old);
   }
   if (threadIdx.x == 0) s.last = 0;
   Acc a;
   acc_init(a);
   if (DEFER && hs.h) block_hist_begin(hs.h);
-  clear_old(c, old, active);
+  clear_old(c, S, old, active);
   const int lane = threadIdx.x & 31;
   WarpStage& ws = sh.wss[threadIdx.x >> 5];
   int qn = 0;  // queued vertices of this warp
@@ -1239,30 +1250,30 @@ __device__ __forceinline__ bool body_edge_balanced(const Ctx& c, EBSharedT<DEFER
       j += (ws.off[m] == e1) ? m : m - 1;
       __syncwarp();
       if (qn > kWarpQueue - kWarpTile) {  // the next tile's might not fit
-        warp_resolve<ALG, DEFER>(c, ws, a, nxt, qn, thr, hs);
+        warp_resolve<ALG, DEFER>(c, ws, a, nxt, qn, thr, hs, DEFER ? S.pcur : 0);
         qn = 0;
       }
     }
   }
-  if (qn) warp_resolve<ALG, DEFER>(c, ws, a, nxt, qn, thr, hs);
+  if (qn) warp_resolve<ALG, DEFER>(c, ws, a, nxt, qn, thr, hs, DEFER ? S.pcur : 0);
   if (DEFER && hs.h) block_hist_end(hs.h, c.hist);
   __syncthreads();
-  return block_epilogue(c, s, a, i, cur, nxt, old, active);
+  return block_epilogue(c, S, s, a, i, cur, nxt, old);
 }
 
 // ---------------------------------------------------------------------------
 // Bitmap-gated topology sweep: thread per vertex, light vertices only; heavy
 // frontier vertices take the shared heavy path.
 template <int ALG>
-__device__ __forceinline__ bool body_push_topo(const Ctx& c, Stage& s) {
+__device__ __forceinline__ bool body_push_topo(const Ctx& c, CtlHead& S, Stage& s) {
   block_prologue(c);
   stage_init(s);
   Acc a;
   acc_init(a);
-  const int i = c.ctl->iter;
+  const int i = S.iter;
   const int cur = i % 3, nxt = (i + 1) % 3, old = (i + 2) % 3;
   const int active = gridDim.x;  // topology sweeps use the whole grid
-  clear_old(c, old, active);
+  clear_old(c, S, old, active);
   __syncthreads();
   const unsigned* bmc = c.bm[cur];
   const int V = c.g.nodes;
@@ -1276,23 +1287,23 @@ __device__ __forceinline__ bool body_push_topo(const Ctx& c, Stage& s) {
     }
     stage_flush_if_half(c, s, nxt);
   }
-  heavy_path<ALG>(c, s, a, cur, nxt, active);
+  heavy_path<ALG>(c, S, s, a, cur, nxt, active);
   stage_flush(c, s, nxt);
-  return block_epilogue(c, s, a, i, cur, nxt, old, active);
+  return block_epilogue(c, S, s, a, i, cur, nxt, old);
 }
 
 // ---------------------------------------------------------------------------
 // Edge-centric sweep over all CSR entries, gated by the source's frontier bit.
 template <int ALG>
-__device__ __forceinline__ bool body_edge_topo(const Ctx& c, Stage& s) {
+__device__ __forceinline__ bool body_edge_topo(const Ctx& c, CtlHead& S, Stage& s) {
   block_prologue(c);
   stage_init(s);
   Acc a;
   acc_init(a);
-  const int i = c.ctl->iter;
+  const int i = S.iter;
   const int cur = i % 3, nxt = (i + 1) % 3, old = (i + 2) % 3;
   const int active = gridDim.x;  // topology sweeps use the whole grid
-  clear_old(c, old, active);
+  clear_old(c, S, old, active);
   __syncthreads();
   const unsigned* bmc = c.bm[cur];
   const int E = c.g.edges;
@@ -1337,7 +1348,7 @@ __device__ __forceinline__ bool body_edge_topo(const Ctx& c, Stage& s) {
     stage_flush_if_half(c, s, nxt);
   }
   stage_flush(c, s, nxt);
-  return block_epilogue(c, s, a, i, cur, nxt, old, active);
+  return block_epilogue(c, S, s, a, i, cur, nxt, old);
 }
 
 // ---------------------------------------------------------------------------
@@ -1346,21 +1357,21 @@ __device__ __forceinline__ bool body_edge_topo(const Ctx& c, Stage& s) {
 // frontier's bitmap is written with one plain store per warp. dist[v] is only
 // written by v's own thread, so no atomics are needed on it.
 template <int ALG, bool FRONTIER>
-__device__ __forceinline__ bool body_pull(const Ctx& c, Stage& s) {
+__device__ __forceinline__ bool body_pull(const Ctx& c, CtlHead& S, Stage& s) {
   block_prologue(c);
   stage_init(s);
   Acc a;
   acc_init(a);
-  const int i = c.ctl->iter;
+  const int i = S.iter;
   const int cur = i % 3, nxt = (i + 1) % 3, old = (i + 2) % 3;
   const int active = gridDim.x;  // every vertex is visited
-  clear_old(c, old, active);
+  clear_old(c, S, old, active);
   __syncthreads();
   const unsigned* bmc = c.bm[cur];
   const int V = c.g.nodes;
   const int* __restrict__ nl = c.g.nlist;
   const int* __restrict__ ew = c.g.eweight;
-  const int fmin = c.ctl->slot[cur].mindist;
+  const int fmin = S.slot[cur].mindist;
   // Smallest candidate any frontier vertex can produce.
   const int bound = FRONTIER ? (fmin == kInf ? kInf : Op<ALG>::cand(fmin, c.gs.wmin)) : INT_MIN;
   for (long long base = (long long)blockIdx.x * kBlock; base < V; base += (long long)gridDim.x * kBlock) {
@@ -1404,7 +1415,7 @@ __device__ __forceinline__ bool body_pull(const Ctx& c, Stage& s) {
     stage_flush_if_half(c, s, nxt);
   }
   stage_flush(c, s, nxt);
-  return block_epilogue(c, s, a, i, cur, nxt, old, active);
+  return block_epilogue(c, S, s, a, i, cur, nxt, old);
 }
 
 // ---------------------------------------------------------------------------
@@ -1489,7 +1500,7 @@ __device__ __forceinline__ void vote_merge(int& cand, int& cnt, int c2, int n2) 
 // correct; the vote only decides how many vertices the second hook launch can
 // skip. Registers and 64 bytes of shared memory: this runs in the epilogue of
 // every relax kernel, whose shared-memory size sets the L1 left to it.
-__device__ __forceinline__ void uf_sample_giant(const Ctx& c) {
+__device__ __forceinline__ void uf_sample_giant(const Ctx& c, CtlHead& S) {
   __shared__ int wc[kBlock / kWarp], wn[kBlock / kWarp];
   const int V = c.g.nodes;
   int cand = -1, cnt = 0;
@@ -1507,7 +1518,7 @@ __device__ __forceinline__ void uf_sample_giant(const Ctx& c) {
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int w = 1; w < (int)(blockDim.x >> 5); ++w) vote_merge(cand, cnt, wc[w], wn[w]);
-    c.ctl->uf_giant = cand;
+    S.uf_giant = cand;
   }
   __syncthreads();
 }
@@ -1524,21 +1535,21 @@ __device__ __forceinline__ void uf_sample_giant(const Ctx& c) {
 // IPDPS 2018). On graphs with a giant component the second launch skips most
 // edges.
 template <int ALG>
-__device__ __forceinline__ bool body_union(const Ctx& c, Stage& s) {
+__device__ __forceinline__ bool body_union(const Ctx& c, CtlHead& S, Stage& s) {
   block_prologue(c);
   stage_init(s);
   Acc a;
   acc_init(a);
-  const int i = c.ctl->iter;
+  const int i = S.iter;
   const int cur = i % 3, nxt = (i + 1) % 3, old = (i + 2) % 3;
   const int active = gridDim.x;
-  clear_old(c, old, active);
+  clear_old(c, S, old, active);
   int* p = c.dist;
   const int V = c.g.nodes;
   const int* __restrict__ nl = c.g.nlist;
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
-  const int phase = c.ctl->uf_phase;
+  const int phase = S.uf_phase;
   if (phase == 0) {
     for (long long v = tid; v < V; v += stride) {
       const int b = c.g.nindex[v];
@@ -1549,7 +1560,7 @@ __device__ __forceinline__ bool body_union(const Ctx& c, Stage& s) {
       }
     }
   } else if (phase == 1) {
-    const int giant = c.ctl->uf_giant;
+    const int giant = S.uf_giant;
     for (long long v = tid; v < V; v += stride) {
       const int b = c.g.nindex[v] + kAfforestLinks;
       const int e = c.g.nindex[v + 1];
@@ -1567,7 +1578,7 @@ __device__ __forceinline__ bool body_union(const Ctx& c, Stage& s) {
       if (r != (int)v) p[v] = r;
     }
   }
-  return block_epilogue(c, s, a, i, cur, nxt, old, active);
+  return block_epilogue(c, S, s, a, i, cur, nxt, old);
 }
 
 // ---------------------------------------------------------------------------
@@ -1638,13 +1649,13 @@ __device__ __forceinline__ void mis_flush(const Ctx& c, Stage& s, int nxt) {
   __syncthreads();
 }
 
-__device__ __forceinline__ bool body_mis(const Ctx& c, Stage& s) {
+__device__ __forceinline__ bool body_mis(const Ctx& c, CtlHead& S, Stage& s) {
   block_prologue(c);
-  const int i = c.ctl->iter;
+  const int i = S.iter;
   const int cur = i % 3, nxt = (i + 1) % 3, old = (i + 2) % 3;
-  const int n = slot_size(c.ctl->slot[cur].packed);
+  const int n = slot_size(S.slot[cur].packed);
   const int active = (int)min((long long)gridDim.x, ((long long)n + kBlock - 1) / kBlock);
-  if (blockIdx.x >= active) return idle_epilogue(c, s, i, cur, nxt, old);
+  if (blockIdx.x >= active) return idle_epilogue(c, S, s, i, cur, nxt, old);
   stage_init(s);
   if (threadIdx.x == 0) s.m = 0;
   Acc a;
@@ -1829,56 +1840,80 @@ __device__ __forceinline__ bool body_mis(const Ctx& c, Stage& s) {
   }
   mis_flush(c, s, nxt);
   __syncthreads();
-  return block_epilogue(c, s, a, i, cur, nxt, old, active);
+  return block_epilogue(c, S, s, a, i, cur, nxt, old);
 }
 
 // ---------------------------------------------------------------------------
 // Kernel wrappers.
 template <int ALG, int VAR>
-__global__ void __launch_bounds__(kBlock) relax_push(Ctx c) {
+__global__ void __launch_bounds__(kBlock) relax_push(const __grid_constant__ Ctx c) {
   __shared__ Stage s;
-  body_push<ALG, VAR>(c, s);
+  __shared__ CtlHead S;
+  load_head(c, S);
+  __syncthreads();
+  body_push<ALG, VAR>(c, S, s);
 }
 
 template <int ALG>
-__global__ void __launch_bounds__(kBlock, I2_EB_MIN_BLOCKS) relax_edge_balanced(Ctx c) {
+__global__ void __launch_bounds__(kBlock, I2_EB_MIN_BLOCKS) relax_edge_balanced(const __grid_constant__ Ctx c) {
   __shared__ EBShared sh;
-  body_edge_balanced<ALG>(c, sh);
+  __shared__ CtlHead S;
+  load_head(c, S);
+  __syncthreads();
+  body_edge_balanced<ALG>(c, S, sh);
 }
 
-static __global__ void __launch_bounds__(kBlock, I2_EB_MIN_BLOCKS) relax_mis(Ctx c) {
+static __global__ void __launch_bounds__(kBlock, I2_FIXED_MIN_BLOCKS) relax_mis(const __grid_constant__ Ctx c) {
   __shared__ Stage s;
-  body_mis(c, s);
+  __shared__ CtlHead S;
+  load_head(c, S);
+  __syncthreads();
+  body_mis(c, S, s);
 }
 
 // Edge-balanced SSSP push with near/far ordering (Ctl::delta != 0).
-static __global__ void __launch_bounds__(kBlock, I2_EB_MIN_BLOCKS) relax_near_far(Ctx c) {
+static __global__ void __launch_bounds__(kBlock, I2_EB_MIN_BLOCKS) relax_near_far(const __grid_constant__ Ctx c) {
   __shared__ EBSharedFar sh;
-  body_edge_balanced<kSSSP, true>(c, sh);
+  __shared__ CtlHead S;
+  load_head(c, S);
+  __syncthreads();
+  body_edge_balanced<kSSSP, true>(c, S, sh);
 }
 
 template <int ALG>
-__global__ void __launch_bounds__(kBlock) relax_push_topo(Ctx c) {
+__global__ void __launch_bounds__(kBlock) relax_push_topo(const __grid_constant__ Ctx c) {
   __shared__ Stage s;
-  body_push_topo<ALG>(c, s);
+  __shared__ CtlHead S;
+  load_head(c, S);
+  __syncthreads();
+  body_push_topo<ALG>(c, S, s);
 }
 
 template <int ALG>
-__global__ void __launch_bounds__(kBlock) relax_edge_topo(Ctx c) {
+__global__ void __launch_bounds__(kBlock) relax_edge_topo(const __grid_constant__ Ctx c) {
   __shared__ Stage s;
-  body_edge_topo<ALG>(c, s);
+  __shared__ CtlHead S;
+  load_head(c, S);
+  __syncthreads();
+  body_edge_topo<ALG>(c, S, s);
 }
 
 template <int ALG>
-__global__ void __launch_bounds__(kBlock) relax_union(Ctx c) {
+__global__ void __launch_bounds__(kBlock) relax_union(const __grid_constant__ Ctx c) {
   __shared__ Stage s;
-  body_union<ALG>(c, s);
+  __shared__ CtlHead S;
+  load_head(c, S);
+  __syncthreads();
+  body_union<ALG>(c, S, s);
 }
 
 template <int ALG, bool FRONTIER>
-__global__ void __launch_bounds__(kBlock) relax_pull(Ctx c) {
+__global__ void __launch_bounds__(kBlock) relax_pull(const __grid_constant__ Ctx c) {
   __shared__ Stage s;
-  body_pull<ALG, FRONTIER>(c, s);
+  __shared__ CtlHead S;
+  load_head(c, S);
+  __syncthreads();
+  body_pull<ALG, FRONTIER>(c, S, s);
 }
 
 template <bool DEFER = false>
@@ -1900,97 +1935,117 @@ union AnyShared {
 // bodies read the frontier lists, bitmaps and values with coherent loads only
 // (the read-only path is used for the graph arrays alone).
 
-// Thread 0 of a block: return once bar_gen has moved past `gen`, or once the
-// wait has run out (status kStatusStall) or another block has given up.
-__device__ __forceinline__ void grid_wait(Ctl* ctl, unsigned gen) {
+// Thread 0 of a block: wait until bar_gen has moved past `gen`. False once the
+// wait has run out (status kStatusStall) or another block has given up. The
+// polls are plain reads of one line; the fence after them orders what follows
+// (an acquire in every poll would drop the L1 of the SM's working blocks).
+__device__ __forceinline__ bool grid_wait(const Ctx& c, unsigned gen, unsigned long long limit) {
   const unsigned long long t0 = globaltimer();
-  const unsigned long long limit = *(volatile unsigned long long*)&ctl->stall_ns;
+  Ctl* ctl = c.ctl;
+  bool ok = true;
   for (unsigned k = 1;; ++k) {
-    if (*(volatile unsigned*)&ctl->bar_gen != gen) break;
-    if (*(volatile int*)&ctl->status & kStatusStall) break;
-    __nanosleep(k < 256 ? 20 : 200);
+    unsigned g, st;
+    asm volatile("ld.relaxed.gpu.global.v2.u32 {%0, %1}, [%2];" : "=r"(g), "=r"(st) : "l"(&ctl->bar_gen) : "memory");
+    if (st & kStatusStall) ok = false;
+    if (g != gen || !ok) break;
+    if (k >= 256) __nanosleep(100);
     if ((k & 63) == 0 && globaltimer() - t0 > limit) {
       atomicOr(&ctl->status, kStatusStall);
+      ok = false;
       break;
     }
   }
+  asm volatile("fence.acq_rel.gpu;" ::: "memory");
+  return ok;
 }
 
 template <int ALG, int VAR, bool DEFER>
-__device__ __forceinline__ bool run_body(const Ctx& c, AnyShared<DEFER>& sh) {
+__device__ __forceinline__ bool run_body(const Ctx& c, CtlHead& S, AnyShared<DEFER>& sh) {
   if constexpr (ALG == kMIS) {
-    return body_mis(c, sh.st);  // one style
+    return body_mis(c, S, sh.st);  // one style
   } else {
-    const int v = VAR >= 0 ? VAR : *(volatile int*)&c.ctl->variant;  // uniform: written before the release
+    const int v = VAR >= 0 ? VAR : S.variant;
     switch (v) {
-      case kVPThread: return body_push<ALG, kVPThread>(c, sh.st);
-      case kVPWarp: return body_push<ALG, kVPWarp>(c, sh.st);
-      case kVPCta: return body_edge_balanced<ALG, DEFER>(c, sh.eb);
-      case kVPBlock: return body_push<ALG, kVPBlock>(c, sh.st);
-      case kPullFrontier: return body_pull<ALG, true>(c, sh.st);
-      case kPullTopo: return body_pull<ALG, false>(c, sh.st);
-      case kEdgeTopo: return body_edge_topo<ALG>(c, sh.st);
+      case kVPThread: return body_push<ALG, kVPThread>(c, S, sh.st);
+      case kVPWarp: return body_push<ALG, kVPWarp>(c, S, sh.st);
+      case kVPCta: return body_edge_balanced<ALG, DEFER>(c, S, sh.eb);
+      case kVPBlock: return body_push<ALG, kVPBlock>(c, S, sh.st);
+      case kPullFrontier: return body_pull<ALG, true>(c, S, sh.st);
+      case kPullTopo: return body_pull<ALG, false>(c, S, sh.st);
+      case kEdgeTopo: return body_edge_topo<ALG>(c, S, sh.st);
       case kUnionFind:
-        if constexpr (ALG == kCC) return body_union<ALG>(c, sh.st);
+        if constexpr (ALG == kCC) return body_union<ALG>(c, S, sh.st);
         [[fallthrough]];  // not allowed for BFS/SSSP
-      default: return body_push_topo<ALG>(c, sh.st);
+      default: return body_push_topo<ALG>(c, S, sh.st);
     }
   }
 }
 
 // VAR >= 0: that style every iteration; VAR < 0: the style picked for each
 // iteration by the previous one (heuristic or learned selector).
-template <int ALG, int VAR, bool DEFER = false, int MINB = (VAR < 0 ? I2_SEL_MIN_BLOCKS : I2_EB_MIN_BLOCKS)>
-__global__ void __launch_bounds__(kBlock, MINB) relax_resident(Ctx c) {
+template <int ALG, int VAR, bool DEFER = false,
+          int MINB = (VAR < 0 ? I2_SEL_MIN_BLOCKS : VAR == kVPCta ? I2_EB_MIN_BLOCKS : I2_FIXED_MIN_BLOCKS)>
+__global__ void __launch_bounds__(kBlock, MINB) relax_resident(const __grid_constant__ Ctx c) {
   __shared__ AnyShared<DEFER> sh;
-  __shared__ int s_go;
-  Ctl* ctl = c.ctl;
-  if (threadIdx.x == 0) s_go = !(*(volatile int*)&ctl->status & kStatusStall);
+  __shared__ CtlHead S;
+  // thread 0's: barrier generation, whether to go on, the test hook (kept in
+  // shared memory: the bodies have no register to spare)
+  __shared__ unsigned s_gen;
+  __shared__ int s_ok, s_hold;
+  load_head(c, S);
+  if (threadIdx.x == 0) {
+    s_ok = !(*(volatile int*)&c.ctl->status & kStatusStall);
+    s_gen = *(volatile unsigned*)&c.ctl->bar_gen;  // no iteration ends before every block arrives
+    s_hold = c.ctl->hold;
+  }
   __syncthreads();
-  if (!s_go) {  // an earlier launch of this traversal gave up: end the graph's loop
+  if (!s_ok) {  // an earlier launch of this traversal gave up: end the graph's loop
     if (blockIdx.x == 0 && threadIdx.x == 0 && c.use_loop)
       cudaGraphSetConditional((cudaGraphConditionalHandle)c.loop_h, 0u);
     return;
   }
-  unsigned gen = *(volatile unsigned*)&ctl->bar_gen;  // no iteration ends before every block arrives
-  bool first = true;
   for (;;) {
-    const bool last = run_body<ALG, VAR, DEFER>(c, sh);
-    if (threadIdx.x == 0) {
-      if (last && !(first && *(volatile int*)&ctl->hold)) {
-        __threadfence();
-        atomicAdd(&ctl->bar_gen, 1u);
-      } else {
-        grid_wait(ctl, gen);
-      }
-      __threadfence();
-      s_go = *(volatile int*)&ctl->go && !(*(volatile int*)&ctl->status & kStatusStall);
+    if (run_body<ALG, VAR, DEFER>(c, S, sh) && !s_hold) {
+      // this block advanced S and wrote it back (every thread a word)
+      __syncthreads();
+      if (threadIdx.x == 0)
+        asm volatile("red.add.release.gpu.global.u32 [%0], 1;" ::"l"(&c.ctl->bar_gen) : "memory");
+    } else {
+      if (threadIdx.x == 0) s_ok = grid_wait(c, s_gen, S.stall_ns);
+      __syncthreads();
+      if (!s_ok) break;
+      load_head(c, S);
     }
-    first = false;
-    ++gen;
+    if (threadIdx.x == 0) {
+      ++s_gen;
+      s_hold = 0;  // the hook withholds the first release only
+    }
     __syncthreads();
-    if (!s_go) break;
+    if (!S.go) break;
   }
 }
 
 template <int ALG, int MINB = I2_SEL_MIN_BLOCKS>
-__global__ void __launch_bounds__(kBlock, MINB) relax_dispatch(Ctx c) {
+__global__ void __launch_bounds__(kBlock, MINB) relax_dispatch(const __grid_constant__ Ctx c) {
   __shared__ AnyShared<> sh;
-  switch (c.ctl->variant) {  // same value for every thread of the launch
-    case kVPThread: body_push<ALG, kVPThread>(c, sh.st); break;
-    case kVPWarp: body_push<ALG, kVPWarp>(c, sh.st); break;
-    case kVPCta: body_edge_balanced<ALG>(c, sh.eb); break;
-    case kVPBlock: body_push<ALG, kVPBlock>(c, sh.st); break;
-    case kPullFrontier: body_pull<ALG, true>(c, sh.st); break;
-    case kPullTopo: body_pull<ALG, false>(c, sh.st); break;
-    case kEdgeTopo: body_edge_topo<ALG>(c, sh.st); break;
+  __shared__ CtlHead S;
+  load_head(c, S);
+  __syncthreads();
+  switch (S.variant) {
+    case kVPThread: body_push<ALG, kVPThread>(c, S, sh.st); break;
+    case kVPWarp: body_push<ALG, kVPWarp>(c, S, sh.st); break;
+    case kVPCta: body_edge_balanced<ALG>(c, S, sh.eb); break;
+    case kVPBlock: body_push<ALG, kVPBlock>(c, S, sh.st); break;
+    case kPullFrontier: body_pull<ALG, true>(c, S, sh.st); break;
+    case kPullTopo: body_pull<ALG, false>(c, S, sh.st); break;
+    case kEdgeTopo: body_edge_topo<ALG>(c, S, sh.st); break;
     case kUnionFind:
       if constexpr (ALG == kCC) {
-        body_union<ALG>(c, sh.st);
+        body_union<ALG>(c, S, sh.st);
         break;
       }
       [[fallthrough]];  // not allowed for BFS/SSSP
-    default: body_push_topo<ALG>(c, sh.st); break;
+    default: body_push_topo<ALG>(c, S, sh.st); break;
   }
 }
 
