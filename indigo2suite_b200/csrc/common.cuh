@@ -170,6 +170,8 @@ struct CtlHead {
   int pcur;                 // current far pile
   int uf_phase;             // union-find CC: 1 after the hook launch (the compress launch follows)
   int uf_giant;             // union-find CC: root of the sampled largest tree
+  int uf_start;             // union-find CC from the first iteration: no frontier is built
+  unsigned uf_step;         // union-find CC: order of the vertices (body_union)
   int then_at;              // mode 3: iteration from which then_variant runs
   int then_variant;
   int go;                   // 1 while another iteration follows

@@ -21,6 +21,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <numeric>
 #include <vector>
 #include "../../include/i2b200.h"
 #include "common.cuh"
@@ -38,7 +39,9 @@ static_assert((int)kNumVariants == (int)I2_NUM_VARIANTS, "variant count");
 // ---------------------------------------------------------------------------
 // Init kernels.
 
-// dist[v] = INF (BFS/SSSP) or v (CC). For CC every vertex enters F_0.
+// dist[v] = INF (BFS/SSSP) or v (CC). For CC every vertex enters F_0, unless
+// union-find runs from the first iteration (uf_start): it reads no frontier, so
+// none is built.
 template <int ALG>
 __global__ void __launch_bounds__(kBlock) k_fill(Ctx c) {
   __shared__ Stage s;
@@ -47,6 +50,16 @@ __global__ void __launch_bounds__(kBlock) k_fill(Ctx c) {
   acc_init(a);
   __syncthreads();
   const int V = c.g.nodes;
+  if (ALG == kCC && c.ctl->uf_start) {
+    const unsigned stride = gridDim.x * kBlock;
+    for (unsigned v = blockIdx.x * kBlock + threadIdx.x; v < (unsigned)V; v += stride) c.dist[v] = (int)v;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {  // the record's frontier: every vertex
+      c.ctl->slot[0].packed = ((unsigned long long)V << 32) | (unsigned)c.g.edges;
+      c.ctl->slot[0].maxdeg = c.gs.maxdeg;
+      c.ctl->slot[0].mindist = 0;
+    }
+    return;
+  }
   for (long long base = (long long)blockIdx.x * kBlock; base < V; base += (long long)gridDim.x * kBlock) {
     const int v = (int)base + threadIdx.x;
     const bool in = v < V;
@@ -130,7 +143,8 @@ __global__ void __launch_bounds__(kBlock) k_seed(Ctx c) {
 // Per-run parameters, passed by value to k_reset so that queued runs never
 // share a host buffer.
 struct RunParams {
-  int algo, mode, fixed_variant, allowed, src, nsrc, iter_cap, delta, hold, stall_ms, then_at, then_variant, hshift;
+  int algo, mode, fixed_variant, allowed, src, nsrc, iter_cap, delta, hold, stall_ms, then_at, then_variant, hshift, uf_start;
+  unsigned uf_step;
   bool operator!=(const RunParams& o) const { return std::memcmp(this, &o, sizeof(RunParams)) != 0; }
 };
 
@@ -154,6 +168,8 @@ __global__ void k_reset(Ctl* ctl, RunParams p) {
   ctl->then_at = p.then_at;
   ctl->then_variant = p.then_variant;
   ctl->hold = p.hold;
+  ctl->uf_start = p.uf_start;
+  ctl->uf_step = p.uf_step;
   ctl->stall_ns = (unsigned long long)p.stall_ms * 1000000ull;
   ctl->threshold = p.delta > 0 ? p.delta : kInf;  // sources start at 0
   ctl->pmin[0] = kInf;
@@ -886,6 +902,17 @@ static int budget_shift(const i2_graph* g) {
   return s;
 }
 
+// Union-find links in ascending order below this average degree (body_union).
+constexpr float kUfLocalDegree = 6.f;
+
+// A step near the golden section of n that is coprime to n: multiples of it
+// mod n visit every index once, neighbours in time far apart (union-find).
+static unsigned spread_step(unsigned n) {
+  unsigned s = (unsigned)(n * 0.6180339887498949) | 1u;
+  while (s < 3 || std::gcd(s, n) != 1) s += 2;  // 1 means ascending order
+  return s;
+}
+
 static RunParams make_params(const i2_graph* g, int algo, int mode, int variant, int src, int nsrc, int cap,
                              int delta = 0) {
   RunParams p{};
@@ -897,6 +924,7 @@ static RunParams make_params(const i2_graph* g, int algo, int mode, int variant,
   p.nsrc = nsrc;
   p.delta = delta;
   p.hshift = budget_shift(g);
+  p.uf_step = algo != I2_CC ? 0 : g->gs.avgdeg < kUfLocalDegree ? 1u : spread_step((unsigned)((g->g.nodes + 31LL) / 32));
   // Test hook: withhold the first barrier release of a resident traversal,
   // so that every block's bounded wait runs out (I2_STALL_MS bounds it).
   const char* hold = std::getenv("I2_TEST_HOLD_BARRIER");
@@ -1243,6 +1271,10 @@ int run_traversal(i2_graph* g, int algo, int src, const int* srcs_host, int nsrc
     rp.then_at = o.then_at;
     rp.then_variant = o.then_variant;
   }
+  // union-find from the first iteration: fixed, or by the selectors' rule
+  rp.uf_start = algo == I2_CC && ((mode == 0 && variant == kUnionFind) ||
+                                  ((mode == 1 || mode == 2) && ((rp.allowed >> kUnionFind) & 1) &&
+                                   union_find_pays(g->g.nodes, g->gs.avgdeg)));
   ExecEntry* ex = nullptr;
   const bool graph_loop = o.loop_mode == I2_LOOP_GRAPH || o.loop_mode == I2_LOOP_RELAUNCH;
   if (graph_loop) {

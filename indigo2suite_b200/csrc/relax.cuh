@@ -946,6 +946,10 @@ struct EpiStage {
 #ifndef I2_FIXED_MIN_BLOCKS
 #define I2_FIXED_MIN_BLOCKS 6
 #endif
+// ... and union-find's (4, 6 and 8 within the noise of its links).
+#ifndef I2_UF_MIN_BLOCKS
+#define I2_UF_MIN_BLOCKS 6
+#endif
 // Resident blocks per SM that the selectors' kernels (every style in one
 // kernel) are compiled for: 4 leaves them 64 registers, where 6 (40 registers)
 // spilled 160-224 bytes per thread. Held-out RMAT/ER/grid graphs
@@ -1437,39 +1441,69 @@ __device__ __forceinline__ bool body_pull(const Ctx& c, CtlHead& S, Stage& s) {
 // result is the minimum-ID labelling that label propagation converges to,
 // reached from any propagation state in two launches.
 
-// Root of x. With HALVE, each step also points the visited vertex at its
-// grandparent (path halving): any ancestor is a valid label, and a vertex that
-// is not a root never becomes one again, so these plain writes cannot undo a
-// link. The loads may be served from this SM's L1 and so be stale: a stale
+// Reads of parents may be served from this SM's L1 and so be stale: a stale
 // parent is still an ancestor (links are never undone), and a vertex wrongly
 // seen as a root only makes the linking compare-and-swap fail and return its
-// true parent, from which the search continues (parents only decrease, so it
-// ends). Cached loads matter: almost every find ends at a component's root,
-// and reading that one entry from L2 every time serialises on it.
-template <bool HALVE>
+// true parent, from which the climb continues (ancestors only decrease, so it
+// ends). Cached loads matter: the ancestors near a component's root are read by
+// most vertices, and L2 would serialise on them.
+
+// Root of x; each step points the visited vertex at its grandparent (path
+// halving: any ancestor is a valid label, and a vertex that is not a root never
+// becomes one again, so these plain writes cannot undo a link).
 __device__ __forceinline__ int uf_find(int* p, int x) {
   for (;;) {
     const int px = p[x];
     if (px == x) return x;
     const int ppx = p[px];
-    if (HALVE && ppx != px) p[x] = ppx;
+    if (ppx != px) p[x] = ppx;
     x = ppx;
   }
 }
 
+// Link the roots of a and b, the larger below the smaller.
 __device__ __forceinline__ void uf_union(int* p, int a, int b) {
-  int ra = uf_find<true>(p, a), rb = uf_find<true>(p, b);
+  int ra = uf_find(p, a), rb = uf_find(p, b);
   while (ra != rb) {
     if (ra < rb) {
       const int t = ra;
       ra = rb;
       rb = t;
     }
-    const int seen = atomicCAS(&p[ra], ra, rb);  // link the larger root below the smaller
+    const int seen = atomicCAS(&p[ra], ra, rb);
     if (seen == ra) return;
-    ra = uf_find<true>(p, seen);  // ra was linked meanwhile: continue from its root
-    rb = uf_find<true>(p, rb);
+    ra = uf_find(p, seen);  // ra was linked meanwhile: continue from its root
+    rb = uf_find(p, rb);
   }
+}
+
+// The same without finding the roots first: pa and pb are ancestors of a and b;
+// climb from the larger of the two until the ancestors meet or the larger is a
+// root, which is then linked below the smaller. Two vertices whose parents are
+// the same are done after those two reads. Returns an ancestor of both.
+__device__ __forceinline__ int uf_climb(int* p, int pa, int pb) {
+  while (pa != pb) {
+    const int high = max(pa, pb), low = min(pa, pb);
+    int ph = p[high];
+    if (ph == low) return low;
+    if (ph == high) {
+      ph = atomicCAS(&p[high], high, low);
+      if (ph == high) return low;
+    }
+    pa = p[ph];
+    pb = p[low];
+    if (pa != ph) p[high] = pa;  // halve the path (high is no root)
+  }
+  return pa;
+}
+
+// Link vertex v with u, pv being v's parent as last seen, by climbing, and put
+// both (where they are no roots) below the ancestor found. Returns it or pv.
+__device__ __forceinline__ int uf_link(int* p, int v, int pv, int u, int pu) {
+  const int low = uf_climb(p, pv, pu);
+  if (pu != u && low < pu) p[u] = low;
+  if (pv != v && low < pv) p[v] = low;
+  return min(pv, low);
 }
 
 // Neighbours each vertex is linked with before the largest tree is sampled.
@@ -1523,7 +1557,7 @@ __device__ __forceinline__ void uf_sample_giant(const Ctx& c, CtlHead& S) {
   __syncthreads();
 }
 
-// Three launches (Ctl::uf_phase): (0) link every vertex with its first
+// Three launches (CtlHead::uf_phase): (0) link every vertex with its first
 // kAfforestLinks neighbours, after which the last block samples the largest
 // tree; (1) link the remaining neighbours of every vertex whose root is not
 // that tree's (an edge from a skipped vertex to a vertex outside the tree is
@@ -1534,6 +1568,19 @@ __device__ __forceinline__ void uf_sample_giant(const Ctx& c, CtlHead& S) {
 // "Optimizing parallel graph connectivity computation via subgraph sampling",
 // IPDPS 2018). On graphs with a giant component the second launch skips most
 // edges.
+// Order and links (CtlHead::uf_step). On graphs of average degree 6 or more
+// (RMAT, ER: neighbours all over the ID range) warps take chunks of 32
+// consecutive vertices spread over the whole graph (chunk k * uf_step mod
+// chunks, a step near the golden section) and link by climbing. On sparser
+// ones (grids, road networks: neighbours close by, trees as deep as the graph
+// is long) they take them in ascending order and link roots, whose finds
+// flatten the paths that the next vertices walk. Launch 0, us, links spread /
+// ascending: RMAT-22 104-121 / 222-333, ER 4M 163-170 / 296-345, grid 4096^2
+// 900-1,120 / 455, grid 1000^2 96-139 / 85-92. The whole traversal against one
+// order (grid-stride, finds) with a frontier built by the fill: RMAT-22 442 ->
+// 231, ER 4M 487 -> 270, RMAT-20 272 -> 221, ER 600,000 248 -> 169, grid 4096^2
+// 1,380 -> 666, grid 1000^2 191 -> 158. Bound by the latency of dependent
+// parent reads.
 template <int ALG>
 __device__ __forceinline__ bool body_union(const Ctx& c, CtlHead& S, Stage& s) {
   block_prologue(c);
@@ -1542,40 +1589,62 @@ __device__ __forceinline__ bool body_union(const Ctx& c, CtlHead& S, Stage& s) {
   acc_init(a);
   const int i = S.iter;
   const int cur = i % 3, nxt = (i + 1) % 3, old = (i + 2) % 3;
-  const int active = gridDim.x;
-  clear_old(c, S, old, active);
   int* p = c.dist;
   const int V = c.g.nodes;
   const int* __restrict__ nl = c.g.nlist;
-  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long stride = (long long)gridDim.x * blockDim.x;
+  const int* __restrict__ ni = c.g.nindex;
   const int phase = S.uf_phase;
-  if (phase == 0) {
-    for (long long v = tid; v < V; v += stride) {
-      const int b = c.g.nindex[v];
-      const int e = min(c.g.nindex[v + 1], b + kAfforestLinks);
+  const int giant = S.uf_giant;
+  const bool climb = S.uf_step != 1;
+  const int lane = threadIdx.x & 31;
+  const unsigned chunks = ((unsigned)V + kWarp - 1) / kWarp;
+  const unsigned nw = gridDim.x * kWarpsPerBlock;
+  const unsigned w0 = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  unsigned at = (unsigned)(((unsigned long long)w0 * S.uf_step) % chunks);
+  const unsigned step = (unsigned)(((unsigned long long)nw * S.uf_step) % chunks);
+  int top = giant;  // the largest tree's root once every link is made
+  if (phase == 2)
+    for (int px; (px = p[top]) != top;) top = px;
+  for (unsigned k = w0; k < chunks; k += nw) {
+    const unsigned v = at * kWarp + lane;
+    at += step;
+    if (at >= chunks) at -= chunks;
+    if (v >= (unsigned)V) continue;
+    if (phase == 0) {
+      const int b = ni[v], e = ni[v + 1];
+      int u[kAfforestLinks], pu[kAfforestLinks];
+#pragma unroll
+      for (int r = 0; r < kAfforestLinks; ++r) u[r] = b + r < e ? ld_adj(nl + b + r) : (int)v;
+      int pv = p[v];
+#pragma unroll
+      for (int r = 0; r < kAfforestLinks; ++r) pu[r] = climb ? p[u[r]] : 0;
+#pragma unroll
+      for (int r = 0; r < kAfforestLinks; ++r) {
+        if (climb) pv = uf_link(p, (int)v, pv, u[r], pu[r]);
+        else if (u[r] != (int)v) uf_union(p, (int)v, u[r]);
+      }
+    } else if (phase == 1) {
+      const int b = ni[v] + kAfforestLinks, e = ni[v + 1];
+      if (b >= e) continue;
+      int x = (int)v;
+      for (int px; x != giant && (px = p[x]) != x;) x = px;
+      if (x == giant) {
+        if (p[v] != giant && (int)v != giant) p[v] = giant;
+        continue;
+      }
       for (int j = b; j < e; ++j) {
         const int u = ld_adj(nl + j);
-        if (u != (int)v) uf_union(p, (int)v, u);
+        if (climb) uf_climb(p, p[v], p[u]);
+        else uf_union(p, (int)v, u);
       }
-    }
-  } else if (phase == 1) {
-    const int giant = S.uf_giant;
-    for (long long v = tid; v < V; v += stride) {
-      const int b = c.g.nindex[v] + kAfforestLinks;
-      const int e = c.g.nindex[v + 1];
-      if (b >= e || uf_find<true>(p, (int)v) == giant) continue;
-      for (int j = b; j < e; ++j) {
-        const int u = ld_adj(nl + j);
-        if (u != (int)v) uf_union(p, (int)v, u);
-      }
-    }
-  } else {
-    // compress: read-only finds (a halving write could replace a finished
-    // label with an intermediate ancestor), each thread writing its own labels
-    for (long long v = tid; v < V; v += stride) {
-      const int r = uf_find<false>(p, (int)v);
-      if (r != (int)v) p[v] = r;
+    } else {
+      // compress: read-only finds (a shortening write could replace a finished
+      // label with an intermediate ancestor), each thread writing its own label
+      const int pv = p[v];
+      int x = pv;
+      for (int px; x != giant && x != top && (px = p[x]) != x;) x = px;
+      if (x == giant) x = top;
+      if (x != pv) p[v] = x;
     }
   }
   return block_epilogue(c, S, s, a, i, cur, nxt, old);
@@ -1984,7 +2053,10 @@ __device__ __forceinline__ bool run_body(const Ctx& c, CtlHead& S, AnyShared<DEF
 // VAR >= 0: that style every iteration; VAR < 0: the style picked for each
 // iteration by the previous one (heuristic or learned selector).
 template <int ALG, int VAR, bool DEFER = false,
-          int MINB = (VAR < 0 ? I2_SEL_MIN_BLOCKS : VAR == kVPCta ? I2_EB_MIN_BLOCKS : I2_FIXED_MIN_BLOCKS)>
+          int MINB = (VAR < 0                 ? I2_SEL_MIN_BLOCKS
+                      : VAR == kVPCta     ? I2_EB_MIN_BLOCKS
+                      : VAR == kUnionFind ? I2_UF_MIN_BLOCKS
+                                          : I2_FIXED_MIN_BLOCKS)>
 __global__ void __launch_bounds__(kBlock, MINB) relax_resident(const __grid_constant__ Ctx c) {
   __shared__ AnyShared<DEFER> sh;
   __shared__ CtlHead S;

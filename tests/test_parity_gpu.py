@@ -433,3 +433,25 @@ def test_queued_vertices_around_tile_and_queue_sizes(gpu, mid, leaves):
             np.testing.assert_array_equal(dg.sssp(0, loop=loop, budget=budget)[0], oracle.sssp(g, 0))
         np.testing.assert_array_equal(dg.sssp(0, loop=loop, delta=60)[0], oracle.sssp(g, 0))
     dg.free()
+
+
+@pytest.mark.parametrize("n", [2, 31, 32, 33, 63, 65, 95, 257, 1025, 4097, 70001])
+def test_union_find_order_and_links_on_sparse_and_dense_graphs(gpu, n):
+    # below and above the average degree where the links and the order change,
+    # with several components and isolated vertices; from the initial labels and
+    # from a propagation state
+    rng = np.random.default_rng(n)
+    for pairs in (max(1, n // 3), 2 * n, 5 * n):
+        u, v = rng.integers(0, n, pairs), rng.integers(0, n, pairs)
+        u, v = np.concatenate([u, v]), np.concatenate([v, u])
+        key = np.unique(u[u != v] * np.int64(n) + v[u != v])
+        ni = np.zeros(n + 1, np.int32)
+        np.cumsum(np.bincount(key // n, minlength=n), out=ni[1:])
+        g = i2.ECLGraph(n, len(key), ni, (key % n).astype(np.int32), np.ones(len(key), np.int32))
+        dg = i2.DeviceGraph.upload(g)
+        ref = oracle.cc(g)
+        for loop in (i2.I2_LOOP_GRAPH, i2.I2_LOOP_HOST):
+            np.testing.assert_array_equal(dg.cc(variant="union_find", loop=loop)[0], ref)
+            np.testing.assert_array_equal(dg.cc(variant="heuristic", loop=loop)[0], ref)
+        np.testing.assert_array_equal(dg.cc(variant="vp_cta", then_variant="union_find", then_at=1)[0], ref)
+        dg.free()
