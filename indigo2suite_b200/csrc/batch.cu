@@ -100,7 +100,7 @@ int i2_batch_upload(const i2_eclgraph* graphs, int n, i2_batch** out) {
     delete b;
     return bad_input ? I2_ERR_FORMAT : cuda_status(e);
   }
-  int st = graph_adopt((int)V, (int)E, nindex, nlist, w, &b->g);
+  int st = graph_adopt((int)V, (int)E, nindex, nlist, w, -1, &b->g);
   if (st) {
     delete b;
     return st;
@@ -153,7 +153,7 @@ int i2_batch_from_device(i2_graph* const* graphs, int n, i2_batch** out) {
     delete b;
     return cuda_status(e);
   }
-  int st = graph_adopt((int)V, (int)E, nindex, nlist, w, &b->g);
+  int st = graph_adopt((int)V, (int)E, nindex, nlist, w, -1, &b->g);
   if (st) {
     delete b;
     return st;

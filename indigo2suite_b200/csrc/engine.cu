@@ -226,7 +226,7 @@ struct DevStats {
 __global__ void k_degree_stats(DGraph g, int heavy, DevStats* st) {
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
-  int mx = 0, nh = 0, uns = 0;
+  int mx = 0, nh = 0;
   double s2 = 0.0;
   for (long long v = tid; v < g.nodes; v += stride) {
     const int b = g.nindex[v], e = g.nindex[v + 1];
@@ -243,12 +243,38 @@ __global__ void k_degree_stats(DGraph g, int heavy, DevStats* st) {
       wmin = min(wmin, w);
       ws += (double)w;
     }
+  // one set of atomics per block: from every thread they were 0.4 ms on one line
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  nh = __reduce_add_sync(0xffffffffu, nh);
+  wmin = __reduce_min_sync(0xffffffffu, wmin);
+  for (int o = 16; o > 0; o >>= 1) {
+    s2 += __shfl_down_sync(0xffffffffu, s2, o);
+    ws += __shfl_down_sync(0xffffffffu, ws, o);
+  }
+  __shared__ int smx[kWarp], snh[kWarp], swm[kWarp];
+  __shared__ double ss2[kWarp], sws[kWarp];
+  const int wid = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  if ((threadIdx.x & 31) == 0) {
+    smx[wid] = mx;
+    snh[wid] = nh;
+    swm[wid] = wmin;
+    ss2[wid] = s2;
+    sws[wid] = ws;
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int k = 1; k < nwarp; ++k) {
+    mx = max(mx, smx[k]);
+    nh += snh[k];
+    wmin = min(wmin, swm[k]);
+    s2 += ss2[k];
+    ws += sws[k];
+  }
   atomicMax(&st->maxdeg, mx);
-  atomicAdd(&st->wsum, ws);
   atomicAdd(&st->nheavy, nh);
   atomicMin(&st->wmin, wmin);
-  if (uns) atomicOr(&st->unsorted, 1);
   atomicAdd(&st->sumsq, s2);
+  if (g.eweight) atomicAdd(&st->wsum, ws);
 }
 
 // Adjacency lists strictly increasing (sorted, no duplicates)? One thread per
@@ -1235,7 +1261,8 @@ int run_traversal(i2_graph* g, int algo, int src, const int* srcs_host, int nsrc
     variant = kVPCta;
     if (o.sssp_budget <= 0) o.sssp_budget = I2_SSSP_BUDGET_AUTO;
   }
-  if (mode != 0 || variant == kEdgeTopo) {
+  // sp[] is for the edge sweeps, which the frequency rule never picks
+  if (mode >= 2 || variant == kEdgeTopo) {
     st = ensure_sp(g);
     if (st) return st;
   }
@@ -1307,7 +1334,9 @@ int run_traversal(i2_graph* g, int algo, int src, const int* srcs_host, int nsrc
   return fill_report(g, s, algo, rep, host_relax_ms);
 }
 
-int graph_adopt(int nodes, int edges, int* d_nindex, int* d_nlist, int* d_eweight, i2_graph** out) {
+bool graph_known_symmetric(const i2_graph* g) { return g && g->gs.symmetric == 1; }
+
+int graph_adopt(int nodes, int edges, int* d_nindex, int* d_nlist, int* d_eweight, int symmetric, i2_graph** out) {
   i2_graph* g = new i2_graph();
   g->owns = true;
   g->d_nindex = d_nindex;
@@ -1324,6 +1353,7 @@ int graph_adopt(int nodes, int edges, int* d_nindex, int* d_nlist, int* d_eweigh
     delete g;
     return st;
   }
+  g->gs.symmetric = symmetric;
   *out = g;
   return I2_OK;
 }

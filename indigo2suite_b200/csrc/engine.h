@@ -38,7 +38,12 @@ int run_traversal(i2_graph* g, int algo, int src, const int* srcs_host, int nsrc
 bool device_range_ok(const void* p, size_t bytes);
 
 // Take ownership of CSR arrays already on the device and build a graph handle.
-int graph_adopt(int nodes, int edges, int* d_nindex, int* d_nlist, int* d_eweight, i2_graph** out);
+// `symmetric`: 1 when the lists are known to be sorted and to hold every
+// (u, v, w) with its (v, u, w), -1 to have that checked on first need.
+int graph_adopt(int nodes, int edges, int* d_nindex, int* d_nlist, int* d_eweight, int symmetric, i2_graph** out);
+
+// Whether g is known to be symmetric (by construction, or checked before).
+bool graph_known_symmetric(const i2_graph* g);
 
 // The device CSR arrays of a graph (weights null when it has none).
 int graph_device_csr(const i2_graph* g, int* nodes, int* edges, const int** nindex, const int** nlist,

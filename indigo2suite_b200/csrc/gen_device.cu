@@ -1,9 +1,11 @@
 // Device-side construction of CSR graphs.
 //
-// One builder turns 64-bit (u << 32 | v) keys (~0: dropped) into a CSR: a CUB
-// radix sort of the keys (of key/weight pairs when the weights come with the
-// edges), duplicates merged (keeping the smallest weight), then the CSR cut by
-// a binary search per vertex. On top of it:
+// One builder turns 64-bit keys u << b | v, b the bits of a vertex ID (u = n:
+// dropped), into a CSR: a CUB radix sort of the keys over the bits they have (of
+// key/weight pairs when the weights come with the edges), duplicates merged
+// (keeping the smallest weight), then the CSR cut by a binary search per vertex.
+// Packed next to one another, the two IDs of a graph of 10^6 vertices take 5
+// passes of 8 bits instead of 8. On top of it:
 //  * i2_graph_from_coo_device: a graph from COO pairs already in device memory;
 //  * the seeded RMAT, ER and grid generators, which sample their edges with the
 //    same counter-based hashes as the host generators (graph_host.cpp), so that
@@ -21,10 +23,35 @@
 
 namespace i2 {
 
-constexpr unsigned long long kDropKey = ~0ull;
+// Keys of the vertex pairs of a graph of n vertices: `shift` bits hold an ID
+// (those of n, which marks dropped pairs), and keys sort over `bits` bits.
+struct KeyBits {
+  int shift;
+  int bits;
+  unsigned long long drop;
+  __host__ __device__ unsigned long long key(unsigned long long u, unsigned long long v) const {
+    return (u << shift) | v;
+  }
+  __host__ __device__ unsigned long long hi(unsigned long long k) const { return k >> shift; }
+  __host__ __device__ unsigned long long lo(unsigned long long k) const { return k & ((1ull << shift) - 1); }
+};
+
+static int bit_length(unsigned long long x) {
+  int b = 0;
+  for (; x; x >>= 1) ++b;
+  return b;
+}
+
+static KeyBits key_bits(int n) {
+  KeyBits k;
+  k.shift = std::max(1, bit_length((unsigned long long)n - 1));
+  k.bits = k.shift + bit_length((unsigned long long)n);
+  k.drop = (unsigned long long)n << k.shift;
+  return k;
+}
 
 __global__ void k_rmat_keys(uint64_t seed, int scale, RmatThresholds t, RmatPerm p, long long samples, int n,
-                            unsigned long long* keys) {
+                            KeyBits kb, unsigned long long* keys) {
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = tid; i < samples; i += stride) {
@@ -32,10 +59,10 @@ __global__ void k_rmat_keys(uint64_t seed, int scale, RmatThresholds t, RmatPerm
     rmat_sample(seed, scale, t, (uint64_t)i, &u, &v);
     u = perm_apply(p, u);
     v = perm_apply(p, v);
-    unsigned long long a = kDropKey, b = kDropKey;
+    unsigned long long a = kb.drop, b = kb.drop;
     if (u != v && u < (uint64_t)n && v < (uint64_t)n) {
-      a = (u << 32) | v;
-      b = (v << 32) | u;
+      a = kb.key(u, v);
+      b = kb.key(v, u);
     }
     keys[2 * i] = a;
     keys[2 * i + 1] = b;
@@ -50,19 +77,19 @@ struct CutWeights {
   const int* given;  // mode 2: weight of keys[k]
 };
 
-__global__ void k_cut_csr(const unsigned long long* __restrict__ keys, long long E, int nodes, CutWeights cw,
-                          int* __restrict__ nindex, int* __restrict__ nlist, int* __restrict__ w) {
+__global__ void k_cut_csr(const unsigned long long* __restrict__ keys, long long E, int nodes, KeyBits kb,
+                          CutWeights cw, int* __restrict__ nindex, int* __restrict__ nlist, int* __restrict__ w) {
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long k = tid; k < E; k += stride) {
     const unsigned long long key = keys[k];
-    const int u = (int)(key >> 32), v = (int)(key & 0xffffffffu);
+    const int u = (int)kb.hi(key), v = (int)kb.lo(key);
     nlist[k] = v;
     if (cw.mode == 1) w[k] = edge_weight(cw.seed, u, v);
     else if (cw.mode == 2) w[k] = cw.given[k];
   }
   for (long long v = tid; v <= nodes; v += stride) {
-    const unsigned long long target = (unsigned long long)v << 32;
+    const unsigned long long target = kb.key(v, 0);
     long long lo = 0, hi = E;  // first k with keys[k] >= target
     while (lo < hi) {
       const long long mid = lo + ((hi - lo) >> 1);
@@ -76,32 +103,48 @@ struct MinOp {
   __device__ __forceinline__ int operator()(int a, int b) const { return a < b ? a : b; }
 };
 
-// Scratch of a build, freed on every path (plain allocations: transient, so
-// the engine's pool never keeps them).
+// Scratch of a build, freed on every path. Up to kPooled bytes come from the
+// engine's pool, so that builds of ordinary graphs pay no cudaMalloc and
+// cudaFree (16 M keys: 3.4 of 4.6 ms); what is beyond them (tens of GB at RMAT
+// scale 26) is a plain allocation, which the pool never keeps.
 struct Scratch {
   static constexpr int kMax = 16;
+  static constexpr size_t kPooled = (size_t)2 << 30;
   void* p[kMax] = {nullptr};
+  bool pooled[kMax] = {false};
   int n = 0;
+  size_t total = 0;
   template <class T>
   cudaError_t get(T** out, size_t bytes) {
     *out = nullptr;
     if (n == kMax) return cudaErrorMemoryAllocation;  // more buffers than one build takes
+    bytes = bytes > 0 ? bytes : 1;
     void* q = nullptr;
-    const cudaError_t e = cudaMalloc(&q, bytes > 0 ? bytes : 1);
-    if (e == cudaSuccess) p[n++] = q;
+    const bool pool = total + bytes <= kPooled;
+    const cudaError_t e = pool ? dev_alloc(&q, bytes) : cudaMalloc(&q, bytes);
+    if (e == cudaSuccess) {
+      pooled[n] = pool;
+      p[n++] = q;
+      if (pool) total += bytes;
+    }
     *out = static_cast<T*>(q);
     return e;
   }
   ~Scratch() {
-    for (int k = 0; k < n; ++k) cudaFree(p[k]);
+    for (int k = 0; k < n; ++k) {
+      if (pooled[k]) dev_free(p[k]);
+      else cudaFree(p[k]);
+    }
   }
 };
 
 // CSR of `nodes` vertices from nkeys keys in k0 (k1: a buffer of the same
-// size; both are overwritten). Weights: cw.mode 1 seeded; cw.mode 2 given per
+// size; both are overwritten). `symmetric`: every pair comes in both directions
+// with the same weights. Weights: cw.mode 1 seeded; cw.mode 2 given per
 // key in w0 (w1: a buffer of the same size), duplicates keeping the smallest.
 static int csr_from_keys(unsigned long long* k0, unsigned long long* k1, int* w0, int* w1, long long nkeys,
-                         int nodes, CutWeights cw, i2_graph** out) {
+                         int nodes, CutWeights cw, bool symmetric, i2_graph** out) {
+  const KeyBits kb = key_bits(nodes);
   Scratch sc;
   long long* d_num = nullptr;
   void* tmp = nullptr;
@@ -113,16 +156,16 @@ static int csr_from_keys(unsigned long long* k0, unsigned long long* k1, int* w0
   cub::DoubleBuffer<unsigned long long> dk(k0, k1);
   cub::DoubleBuffer<int> dw(w0, w1);
   if (given) {
-    e = cub::DeviceRadixSort::SortPairs(nullptr, tb, dk, dw, nkeys);
+    e = cub::DeviceRadixSort::SortPairs(nullptr, tb, dk, dw, nkeys, 0, kb.bits);
     if (e == cudaSuccess) e = cub::DeviceReduce::ReduceByKey(nullptr, tb2, k0, k1, w0, w1, d_num, MinOp(), nkeys);
   } else {
-    e = cub::DeviceRadixSort::SortKeys(nullptr, tb, dk, nkeys);
+    e = cub::DeviceRadixSort::SortKeys(nullptr, tb, dk, nkeys, 0, kb.bits);
     if (e == cudaSuccess) e = cub::DeviceSelect::Unique(nullptr, tb2, k0, k1, d_num, nkeys);
   }
   if (e == cudaSuccess) e = sc.get(&tmp, std::max(tb, tb2));
   if (e != cudaSuccess) return cuda_status(e);
-  if (given) e = cub::DeviceRadixSort::SortPairs(tmp, tb, dk, dw, nkeys);
-  else e = cub::DeviceRadixSort::SortKeys(tmp, tb, dk, nkeys);
+  if (given) e = cub::DeviceRadixSort::SortPairs(tmp, tb, dk, dw, nkeys, 0, kb.bits);
+  else e = cub::DeviceRadixSort::SortKeys(tmp, tb, dk, nkeys, 0, kb.bits);
   if (e != cudaSuccess) return cuda_status(e);
   unsigned long long* sorted = dk.Current();
   unsigned long long* uniq = dk.Alternate();
@@ -135,7 +178,7 @@ static int csr_from_keys(unsigned long long* k0, unsigned long long* k1, int* w0
   if (e == cudaSuccess) e = cudaMemcpy(&num, d_num, sizeof(long long), cudaMemcpyDeviceToHost);
   if (e == cudaSuccess && num > 0) e = cudaMemcpy(&last, uniq + num - 1, sizeof(last), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return cuda_status(e);
-  const long long E = num - ((num > 0 && last == kDropKey) ? 1 : 0);
+  const long long E = num - ((num > 0 && last == kb.drop) ? 1 : 0);
   if (E > 0x7fffffffLL) return I2_ERR_OVERFLOW;
   int *nindex = nullptr, *nlist = nullptr, *w = nullptr;
   e = dev_alloc(&nindex, sizeof(int) * ((size_t)nodes + 1));
@@ -144,7 +187,7 @@ static int csr_from_keys(unsigned long long* k0, unsigned long long* k1, int* w0
   if (e == cudaSuccess) {
     CutWeights c2 = cw;
     c2.given = wuniq;
-    k_cut_csr<<<4096, 256>>>(uniq, E, nodes, c2, nindex, nlist, w);
+    k_cut_csr<<<4096, 256>>>(uniq, E, nodes, kb, c2, nindex, nlist, w);
     e = cudaDeviceSynchronize();
   }
   if (e != cudaSuccess) {
@@ -154,14 +197,15 @@ static int csr_from_keys(unsigned long long* k0, unsigned long long* k1, int* w0
     dev_free(w);
     return cuda_status(e);
   }
-  return graph_adopt(nodes, (int)E, nindex, nlist, w, out);
+  return graph_adopt(nodes, (int)E, nindex, nlist, w, symmetric ? 1 : -1, out);
 }
 
 // ---------------------------------------------------------------------------
 // COO pairs -> keys.
 
 __global__ void k_coo_keys(const int* __restrict__ src, const int* __restrict__ dst, const int* __restrict__ w,
-                           long long m, int nodes, int sym, unsigned long long* keys, int* wk, int* bad) {
+                           long long m, int nodes, int sym, KeyBits kb, unsigned long long* keys, int* wk,
+                           int* bad) {
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
   const int per = sym ? 2 : 1;
@@ -169,13 +213,13 @@ __global__ void k_coo_keys(const int* __restrict__ src, const int* __restrict__ 
     const int u = src[k], v = dst[k];
     if ((unsigned)u >= (unsigned)nodes || (unsigned)v >= (unsigned)nodes) {
       atomicOr(bad, 1);
-      keys[per * k] = kDropKey;
-      if (sym) keys[per * k + 1] = kDropKey;
+      keys[per * k] = kb.drop;
+      if (sym) keys[per * k + 1] = kb.drop;
       continue;
     }
     const bool loop = u == v;
-    keys[per * k] = loop ? kDropKey : ((unsigned long long)u << 32) | (unsigned)v;
-    if (sym) keys[per * k + 1] = loop ? kDropKey : ((unsigned long long)v << 32) | (unsigned)u;
+    keys[per * k] = loop ? kb.drop : kb.key(u, v);
+    if (sym) keys[per * k + 1] = loop ? kb.drop : kb.key(v, u);
     if (w) {
       wk[per * k] = w[k];
       if (sym) wk[per * k + 1] = w[k];
@@ -184,10 +228,11 @@ __global__ void k_coo_keys(const int* __restrict__ src, const int* __restrict__ 
 }
 
 // ---------------------------------------------------------------------------
-// Candidate pairs of ER and of the grid's long-range edges: key (lo << 32 | hi)
-// or kDropKey, with the candidate's index as the value.
+// Candidate pairs of ER and of the grid's long-range edges: the key of (lo, hi)
+// or a dropped one, with the candidate's index as the value.
 
-__global__ void k_er_candidates(uint64_t seed, int n, long long first, long long count, unsigned long long* keys,
+__global__ void k_er_candidates(uint64_t seed, int n, long long first, long long count, KeyBits kb,
+                                unsigned long long* keys,
                                 unsigned long long* idx) {
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -196,7 +241,7 @@ __global__ void k_er_candidates(uint64_t seed, int n, long long first, long long
     const uint64_t u = h3(seed, kStreamErU, j) % (uint64_t)n;
     const uint64_t v = h3(seed, kStreamErV, j) % (uint64_t)n;
     const uint64_t lo = u < v ? u : v, hi = u < v ? v : u;
-    keys[k] = u == v ? kDropKey : ((lo << 32) | hi);
+    keys[k] = u == v ? kb.drop : kb.key(lo, hi);
     idx[k] = j;
   }
 }
@@ -205,7 +250,7 @@ __device__ __forceinline__ bool grid_kept(uint64_t seed, uint64_t drop, long lon
   return h3(seed, kStreamGridDrop, (uint64_t)idx) >= drop;
 }
 
-__global__ void k_grid_extra_candidates(uint64_t seed, int side, uint64_t drop, long long count,
+__global__ void k_grid_extra_candidates(uint64_t seed, int side, uint64_t drop, long long count, KeyBits kb,
                                         unsigned long long* keys, unsigned long long* idx) {
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -223,7 +268,7 @@ __global__ void k_grid_extra_candidates(uint64_t seed, int side, uint64_t drop, 
       else if (hi == lo + side) gi = H + lo;
       if (gi >= 0 && grid_kept(seed, drop, gi)) ok = false;
     }
-    keys[k] = ok ? (((unsigned long long)lo << 32) | (unsigned long long)hi) : kDropKey;
+    keys[k] = ok ? kb.key(lo, hi) : kb.drop;
     idx[k] = j;
   }
 }
@@ -237,12 +282,13 @@ __global__ void k_grid_count(uint64_t seed, uint64_t drop, long long G, unsigned
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(kept, c);
 }
 
-__global__ void k_grid_keys(uint64_t seed, int side, uint64_t drop, long long G, unsigned long long* keys) {
+__global__ void k_grid_keys(uint64_t seed, int side, uint64_t drop, long long G, KeyBits kb,
+                            unsigned long long* keys) {
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
   const long long H = (long long)side * (side - 1);
   for (long long i = tid; i < G; i += stride) {
-    unsigned long long a = kDropKey, b = kDropKey;
+    unsigned long long a = kb.drop, b = kb.drop;
     if (grid_kept(seed, drop, i)) {
       long long u, v;
       if (i < H) {
@@ -252,23 +298,23 @@ __global__ void k_grid_keys(uint64_t seed, int side, uint64_t drop, long long G,
         u = i - H;
         v = u + side;
       }
-      a = ((unsigned long long)u << 32) | (unsigned long long)v;
-      b = ((unsigned long long)v << 32) | (unsigned long long)u;
+      a = kb.key(u, v);
+      b = kb.key(v, u);
     }
     keys[2 * i] = a;
     keys[2 * i + 1] = b;
   }
 }
 
-// Both directions of `count` pair keys (lo << 32 | hi).
-__global__ void k_both_directions(const unsigned long long* __restrict__ pairs, long long count,
+// Both directions of `count` pair keys (lo, hi).
+__global__ void k_both_directions(const unsigned long long* __restrict__ pairs, long long count, KeyBits kb,
                                   unsigned long long* out) {
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long k = tid; k < count; k += stride) {
     const unsigned long long p = pairs[k];
     out[2 * k] = p;
-    out[2 * k + 1] = (p << 32) | (p >> 32);
+    out[2 * k + 1] = kb.key(kb.lo(p), kb.hi(p));
   }
 }
 
@@ -278,7 +324,8 @@ __global__ void k_both_directions(const unsigned long long* __restrict__ pairs, 
 // distinct pairs are found. Returns I2_OK, I2_ERR_ARG when the count has
 // passed `limit` without enough of them, or a CUDA status.
 template <class Make>
-static int first_distinct(long long want, long long start, long long limit, Make make, unsigned long long* out) {
+static int first_distinct(long long want, long long start, long long limit, KeyBits kb, Make make,
+                          unsigned long long* out) {
   long long C = start;
   for (;;) {
     Scratch sc;
@@ -293,12 +340,12 @@ static int first_distinct(long long want, long long start, long long limit, Make
     make(C, k0, i0);
     size_t tb = 0, tb2 = 0;
     cub::DoubleBuffer<unsigned long long> dk(k0, k1), di(i0, i1);
-    e = cub::DeviceRadixSort::SortPairs(nullptr, tb, dk, di, C);
+    e = cub::DeviceRadixSort::SortPairs(nullptr, tb, dk, di, C, 0, kb.bits);
     if (e == cudaSuccess) e = cub::DeviceSelect::UniqueByKey(nullptr, tb2, k0, i0, k1, i1, d_num, C);
     void* tmp = nullptr;
     if (e == cudaSuccess) e = sc.get(&tmp, std::max(tb, tb2));
     // stable: equal pairs keep their index order, so the first of each run has the smallest index
-    if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(tmp, tb, dk, di, C);
+    if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(tmp, tb, dk, di, C, 0, kb.bits);
     if (e != cudaSuccess) return cuda_status(e);
     unsigned long long *uk = dk.Alternate(), *ui = di.Alternate();
     e = cub::DeviceSelect::UniqueByKey(tmp, tb2, dk.Current(), di.Current(), uk, ui, d_num, C);
@@ -307,16 +354,17 @@ static int first_distinct(long long want, long long start, long long limit, Make
     if (e == cudaSuccess) e = cudaMemcpy(&U, d_num, sizeof(long long), cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && U > 0) e = cudaMemcpy(&last, uk + U - 1, sizeof(last), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_status(e);
-    if (U > 0 && last == kDropKey) --U;
+    if (U > 0 && last == kb.drop) --U;
     if (U >= want || C > limit) {
       if (U < want) return I2_ERR_ARG;
       // survivors by index: sort (index, pair) and keep the first `want`
       cub::DoubleBuffer<unsigned long long> bi(ui, dk.Current()), bk(uk, di.Current());
       size_t tb3 = 0;
-      e = cub::DeviceRadixSort::SortPairs(nullptr, tb3, bi, bk, U);
+      const int ibits = bit_length((unsigned long long)C);
+      e = cub::DeviceRadixSort::SortPairs(nullptr, tb3, bi, bk, U, 0, ibits);
       void* tmp2 = nullptr;
       if (e == cudaSuccess) e = sc.get(&tmp2, tb3);
-      if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(tmp2, tb3, bi, bk, U);
+      if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(tmp2, tb3, bi, bk, U, 0, ibits);
       if (e == cudaSuccess && want > 0)
         e = cudaMemcpy(out, bk.Current(), sizeof(unsigned long long) * want, cudaMemcpyDeviceToDevice);
       if (e == cudaSuccess) e = cudaDeviceSynchronize();
@@ -340,8 +388,9 @@ static int generate_rmat(long long n, int scale, long long samples, double a, do
   cudaError_t e = sc.get(&k0, sizeof(unsigned long long) * nkeys);
   if (e == cudaSuccess) e = sc.get(&k1, sizeof(unsigned long long) * nkeys);
   if (e != cudaSuccess) return cuda_status(e);
-  k_rmat_keys<<<4096, 256>>>(seed, scale, make_thresholds(a, b, c), make_perm(seed, scale), samples, (int)n, k0);
-  return csr_from_keys(k0, k1, nullptr, nullptr, nkeys, (int)n, CutWeights{weighted ? 1 : 0, seed, nullptr}, out);
+  k_rmat_keys<<<4096, 256>>>(seed, scale, make_thresholds(a, b, c), make_perm(seed, scale), samples, (int)n,
+                             key_bits((int)n), k0);
+  return csr_from_keys(k0, k1, nullptr, nullptr, nkeys, (int)n, CutWeights{weighted ? 1 : 0, seed, nullptr}, true, out);
 }
 
 extern "C" int i2_graph_generate_rmat(int scale, int edge_factor, double a, double b, double c, uint64_t seed,
@@ -377,17 +426,18 @@ extern "C" int i2_graph_generate_er(int n, long long m, uint64_t seed, int weigh
   cudaError_t e = sc.get(&pairs, sizeof(unsigned long long) * std::max(1LL, m));
   if (e != cudaSuccess) return cuda_status(e);
   // the host generator's candidate counts: m + m/16 + 64, growing by a quarter, until past 8 (m + 64)
-  int st = first_distinct(m, m + m / 16 + 64, 8 * (m + 64),
+  const KeyBits kb = key_bits(n);
+  int st = first_distinct(m, m + m / 16 + 64, 8 * (m + 64), kb,
                           [&](long long C, unsigned long long* keys, unsigned long long* idx) {
-                            k_er_candidates<<<4096, 256>>>(seed, n, 0, C, keys, idx);
+                            k_er_candidates<<<4096, 256>>>(seed, n, 0, C, kb, keys, idx);
                           },
                           pairs);
   if (st) return st;
   e = sc.get(&k0, sizeof(unsigned long long) * std::max(1LL, 2 * m));
   if (e == cudaSuccess) e = sc.get(&k1, sizeof(unsigned long long) * std::max(1LL, 2 * m));
   if (e != cudaSuccess) return cuda_status(e);
-  k_both_directions<<<4096, 256>>>(pairs, m, k0);
-  return csr_from_keys(k0, k1, nullptr, nullptr, 2 * m, n, CutWeights{weighted ? 1 : 0, seed, nullptr}, out);
+  k_both_directions<<<4096, 256>>>(pairs, m, kb, k0);
+  return csr_from_keys(k0, k1, nullptr, nullptr, 2 * m, n, CutWeights{weighted ? 1 : 0, seed, nullptr}, true, out);
 }
 
 extern "C" int i2_graph_generate_grid(int side, double remove_frac, double add_frac, uint64_t seed, int weighted,
@@ -415,22 +465,23 @@ extern "C" int i2_graph_generate_grid(int side, double remove_frac, double add_f
   e = sc.get(&k0, sizeof(unsigned long long) * nkeys);
   if (e == cudaSuccess) e = sc.get(&k1, sizeof(unsigned long long) * nkeys);
   if (e != cudaSuccess) return cuda_status(e);
-  k_grid_keys<<<4096, 256>>>(seed, side, drop, G, k0);
+  const KeyBits kb = key_bits((int)V);
+  k_grid_keys<<<4096, 256>>>(seed, side, drop, G, kb, k0);
   if (K > 0) {
     unsigned long long* extra = nullptr;
     e = sc.get(&extra, sizeof(unsigned long long) * K);
     if (e != cudaSuccess) return cuda_status(e);
     // the host draws candidates until K new pairs are found; a stream that
     // dries up within 64 (K + 64) candidates is refused
-    int st = first_distinct(K, K + K / 8 + 64, 64 * (K + 64),
+    int st = first_distinct(K, K + K / 8 + 64, 64 * (K + 64), kb,
                             [&](long long C, unsigned long long* keys, unsigned long long* idx) {
-                              k_grid_extra_candidates<<<4096, 256>>>(seed, side, drop, C, keys, idx);
+                              k_grid_extra_candidates<<<4096, 256>>>(seed, side, drop, C, kb, keys, idx);
                             },
                             extra);
     if (st) return st;
-    k_both_directions<<<4096, 256>>>(extra, K, k0 + 2 * G);
+    k_both_directions<<<4096, 256>>>(extra, K, kb, k0 + 2 * G);
   }
-  return csr_from_keys(k0, k1, nullptr, nullptr, nkeys, (int)V, CutWeights{weighted ? 1 : 0, seed, nullptr}, out);
+  return csr_from_keys(k0, k1, nullptr, nullptr, nkeys, (int)V, CutWeights{weighted ? 1 : 0, seed, nullptr}, true, out);
 }
 
 extern "C" int i2_graph_from_coo_device(int nodes, long long m, const int* src, const int* dst, const int* w,
@@ -454,12 +505,12 @@ extern "C" int i2_graph_from_coo_device(int nodes, long long m, const int* src, 
   if (e == cudaSuccess) e = sc.get(&bad, sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(bad, 0, sizeof(int));
   if (e != cudaSuccess) return cuda_status(e);
-  if (m > 0) k_coo_keys<<<4096, 256>>>(src, dst, w, m, nodes, symmetrize ? 1 : 0, k0, w0, bad);
+  if (m > 0) k_coo_keys<<<4096, 256>>>(src, dst, w, m, nodes, symmetrize ? 1 : 0, key_bits(nodes), k0, w0, bad);
   int hbad = 0;
   e = cudaMemcpy(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return cuda_status(e);
   if (hbad) return I2_ERR_FORMAT;
-  return csr_from_keys(k0, k1, w0, w1, nkeys, nodes, CutWeights{w ? 2 : 0, 0, nullptr}, out);
+  return csr_from_keys(k0, k1, w0, w1, nkeys, nodes, CutWeights{w ? 2 : 0, 0, nullptr}, symmetrize != 0, out);
 }
 
 // ---------------------------------------------------------------------------
@@ -487,19 +538,19 @@ __global__ void k_invert(const int* __restrict__ perm, int n, int* __restrict__ 
 }
 
 // One warp per vertex (grid-stride): every CSR entry e of old vertex u becomes
-// the key (inv[u] << 32 | inv[nlist[e]]) at position e, its weight beside it.
+// the key of (inv[u], inv[nlist[e]]) at position e, its weight beside it.
 __global__ void k_relabel_keys(const int* __restrict__ nindex, const int* __restrict__ nlist,
-                               const int* __restrict__ w, const int* __restrict__ inv, int n,
+                               const int* __restrict__ w, const int* __restrict__ inv, int n, KeyBits kb,
                                unsigned long long* __restrict__ keys, int* __restrict__ wk) {
   const int lane = threadIdx.x & 31;
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
   for (long long u = warp; u < n; u += nwarps) {
-    const unsigned long long hi = (unsigned long long)(unsigned)inv[u] << 32;
+    const int iu = inv[u];
     const int beg = nindex[u], end = nindex[u + 1];
     for (int e = beg + lane; e < end; e += 32) {
       const int v = nlist[e];  // in range in every graph handle; dropped if not
-      keys[e] = (unsigned)v < (unsigned)n ? (hi | (unsigned)inv[v]) : kDropKey;
+      keys[e] = (unsigned)v < (unsigned)n ? kb.key(iu, inv[v]) : kb.drop;
       if (w) wk[e] = w[e];
     }
   }
@@ -540,14 +591,14 @@ int degree_ordered_copy(const i2_graph* g, i2_graph** twin, int** inv_out) {
   if (e == cudaSuccess && w) e = sc.get(&w0, sizeof(int) * nk);
   if (e == cudaSuccess && w) e = sc.get(&w1, sizeof(int) * nk);
   if (e == cudaSuccess) {
-    k_relabel_keys<<<4096, 256>>>(nindex, nlist, w, inv, n, k0, w0);
+    k_relabel_keys<<<4096, 256>>>(nindex, nlist, w, inv, n, key_bits(n), k0, w0);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) {
     dev_free(inv);
     return cuda_status(e);
   }
-  st = csr_from_keys(k0, k1, w0, w1, E, n, CutWeights{w ? 2 : 0, 0, nullptr}, twin);
+  st = csr_from_keys(k0, k1, w0, w1, E, n, CutWeights{w ? 2 : 0, 0, nullptr}, graph_known_symmetric(g), twin);
   if (st) {
     dev_free(inv);
     return st;
