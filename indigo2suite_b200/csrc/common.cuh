@@ -188,6 +188,15 @@ struct CtlHead {
   int chunk;                // dynamic work counter of the current launch
   alignas(128) unsigned done;  // blocks finished in the current launch
 };
+// A block's copy of the head, by what the end of an iteration may have to do:
+// pick the next style (every kernel but the resident ones of one fixed style,
+// which leave the network's code and its registers out).
+struct SelectHead : CtlHead {
+  static constexpr bool kSelect = true;
+};
+struct FixedHead : CtlHead {
+  static constexpr bool kSelect = false;
+};
 constexpr int kHeadWords = sizeof(CtlHead) / 4;
 static_assert(kHeadWords <= kBlock, "one word of the head per thread");
 

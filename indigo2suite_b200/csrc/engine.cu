@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kBlock) k_seed(Ctx c) {
   __threadfence();
   __syncthreads();
   // the head with the seeded frontier: its features, and the first style
-  __shared__ CtlHead S;
+  __shared__ SelectHead S;
   load_head(c, S);
   __syncthreads();
   if (threadIdx.x < kFeatures) {
@@ -179,20 +179,6 @@ __global__ void k_reset(Ctl* ctl, RunParams p) {
 // ---------------------------------------------------------------------------
 // Graph maintenance kernels.
 
-// *best = the smallest vertex of degree maxdeg.
-__global__ void k_hub(DGraph g, int maxdeg, int* best) {
-  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  int b = INT_MAX;
-  for (long long v = tid; v < g.nodes; v += stride)
-    if (g.nindex[v + 1] - g.nindex[v] == maxdeg) {
-      b = (int)v;
-      break;  // later vertices of this thread are larger
-    }
-  for (int o = 16; o > 0; o >>= 1) b = min(b, __shfl_down_sync(0xffffffffu, b, o));
-  if ((threadIdx.x & 31) == 0 && b != INT_MAX) atomicMin(best, b);
-}
-
 // Sets bit 8 of *bad when a weight is negative (SSSP needs weights >= 0).
 __global__ void k_negative_weights(const int* w, long long n, int* bad) {
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -213,7 +199,7 @@ __global__ void k_validate(DGraph g, int* bad) {
 }
 
 struct DevStats {
-  int maxdeg;
+  unsigned long long hub;  // largest degree << 32 | ~vertex: the lowest ID on ties
   int nheavy;
   int wmin;
   int unsorted;
@@ -226,12 +212,13 @@ struct DevStats {
 __global__ void k_degree_stats(DGraph g, int heavy, DevStats* st) {
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
-  int mx = 0, nh = 0;
+  unsigned long long hub = 0;
+  int nh = 0;
   double s2 = 0.0;
   for (long long v = tid; v < g.nodes; v += stride) {
     const int b = g.nindex[v], e = g.nindex[v + 1];
     const int d = e - b;
-    mx = max(mx, d);
+    hub = max(hub, ((unsigned long long)d << 32) | (unsigned)~v);
     nh += d >= heavy;
     s2 += (double)d * d;
   }
@@ -244,18 +231,19 @@ __global__ void k_degree_stats(DGraph g, int heavy, DevStats* st) {
       ws += (double)w;
     }
   // one set of atomics per block: from every thread they were 0.4 ms on one line
-  mx = __reduce_max_sync(0xffffffffu, mx);
   nh = __reduce_add_sync(0xffffffffu, nh);
   wmin = __reduce_min_sync(0xffffffffu, wmin);
   for (int o = 16; o > 0; o >>= 1) {
+    hub = max(hub, __shfl_down_sync(0xffffffffu, hub, o));
     s2 += __shfl_down_sync(0xffffffffu, s2, o);
     ws += __shfl_down_sync(0xffffffffu, ws, o);
   }
-  __shared__ int smx[kWarp], snh[kWarp], swm[kWarp];
+  __shared__ int snh[kWarp], swm[kWarp];
+  __shared__ unsigned long long shub[kWarp];
   __shared__ double ss2[kWarp], sws[kWarp];
   const int wid = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   if ((threadIdx.x & 31) == 0) {
-    smx[wid] = mx;
+    shub[wid] = hub;
     snh[wid] = nh;
     swm[wid] = wmin;
     ss2[wid] = s2;
@@ -264,13 +252,13 @@ __global__ void k_degree_stats(DGraph g, int heavy, DevStats* st) {
   __syncthreads();
   if (threadIdx.x != 0) return;
   for (int k = 1; k < nwarp; ++k) {
-    mx = max(mx, smx[k]);
+    hub = max(hub, shub[k]);
     nh += snh[k];
     wmin = min(wmin, swm[k]);
     s2 += ss2[k];
     ws += sws[k];
   }
-  atomicMax(&st->maxdeg, mx);
+  atomicMax(&st->hub, hub);
   atomicAdd(&st->nheavy, nh);
   atomicMin(&st->wmin, wmin);
   atomicAdd(&st->sumsq, s2);
@@ -525,6 +513,7 @@ struct ExecEntry {
 struct i2_graph {
   DGraph g{};
   GStats gs{};
+  int hub = 0;  // highest-degree vertex, the lowest ID on ties
   int device = 0;
   bool owns = false;
   int* d_nindex = nullptr;
@@ -733,7 +722,8 @@ static int compute_stats(i2_graph* g) {
   GStats& s = g->gs;
   s.nodes = g->g.nodes;
   s.edges = g->g.edges;
-  s.maxdeg = h.maxdeg;
+  s.maxdeg = (int)(h.hub >> 32);
+  g->hub = (int)~(unsigned)h.hub;
   s.nheavy = h.nheavy;
   s.wmin = g->g.eweight ? (h.wmin == INT_MAX ? 1 : h.wmin) : 1;
   s.symmetric = -1;  // decided on first need (ensure_symmetry)
@@ -845,6 +835,18 @@ constexpr long long kUnionFindKernelNodes = 1LL << 22;
 // Whether the selectors run in the form compiled for more resident blocks.
 static bool wide_selector(const i2_graph* g) { return (long long)g->g.nodes >= kWideSelectorNodes; }
 
+// Whether a resident traversal takes its kernel's form for more resident blocks
+// per SM. The selectors': graphs of kWideSelectorNodes vertices or more. The
+// edge-balanced style: graphs of skewed degrees, where the tiles of the hubs
+// keep more warps busy than 5 blocks have, at the price of spills that cost the
+// short iterations of other graphs. us, 6 / 5 blocks: SSSP RMAT 10^6 678 / 711,
+// 4 x 10^6 2,102 / 2,204, 25 x 10^6 degree-ordered 10,122 / 10,978; CC RMAT
+// 4 x 10^6 1,854 / 2,104, 25 x 10^6 ordered 11,630 / 12,792; but ER 2 x 10^6
+// SSSP 1,388 / 1,367, CC 1,104 / 966, grid 10^6 SSSP 2,358 / 2,078.
+static bool wide_form(const i2_graph* g, int variant) {
+  return variant == kVPCta ? g->gs.degcv > 1.f : wide_selector(g);
+}
+
 static int allowed_mask(const i2_graph* g, int algo) {
   int m = 0;
   for (int v = 0; v < kNumVariants; ++v) m |= 1 << v;
@@ -928,8 +930,15 @@ static int budget_shift(const i2_graph* g) {
   return s;
 }
 
-// Union-find links in ascending order below this average degree (body_union).
-constexpr float kUfLocalDegree = 6.f;
+// Whether union-find links in ascending order (body_union): on graphs of low
+// average degree, and on graphs numbered with the hubs in front (the
+// degree-ordered copies among them), where the first vertices' links already
+// tie most of the graph to the smallest IDs. First launch, us, ascending /
+// spread, on degree-ordered copies: RMAT 10^6 33 / 294, 9 x 10^6 123 / 362,
+// 25 x 10^6 253 / 511.
+static bool union_in_order(const i2_graph* g) {
+  return g->gs.avgdeg < 6.f || g->hub < g->g.nodes / 256;
+}
 
 // A step near the golden section of n that is coprime to n: multiples of it
 // mod n visit every index once, neighbours in time far apart (union-find).
@@ -950,7 +959,7 @@ static RunParams make_params(const i2_graph* g, int algo, int mode, int variant,
   p.nsrc = nsrc;
   p.delta = delta;
   p.hshift = budget_shift(g);
-  p.uf_step = algo != I2_CC ? 0 : g->gs.avgdeg < kUfLocalDegree ? 1u : spread_step((unsigned)((g->g.nodes + 31LL) / 32));
+  p.uf_step = algo != I2_CC ? 0 : union_in_order(g) ? 1u : spread_step((unsigned)((g->g.nodes + 31LL) / 32));
   // Test hook: withhold the first barrier release of a resident traversal,
   // so that every block's bounded wait runs out (I2_STALL_MS bounds it).
   const char* hold = std::getenv("I2_TEST_HOLD_BARRIER");
@@ -1033,7 +1042,7 @@ static int build_exec(i2_graph* g, int algo, int mode, int variant, bool multi, 
   // branch on the style the previous iteration selected.
   {
     cudaGraphNode_t n;
-    KernelFn fn = resident ? resident_kernel(algo, mode == 0 ? variant : -1, rp.delta != 0, wide_selector(g))
+    KernelFn fn = resident ? resident_kernel(algo, mode == 0 ? variant : -1, rp.delta != 0, wide_form(g, mode == 0 ? variant : -1))
                   : mode == 0 ? relax_kernel(algo, variant, rp.delta != 0)
                               : dispatch_kernel(algo, wide_selector(g));
     st = add_kernel_node(body, &n, nullptr, 0, fn, grid_for(fn, g->blocks_per_sm), &c);
@@ -1269,6 +1278,18 @@ int run_traversal(i2_graph* g, int algo, int src, const int* srcs_host, int nsrc
   if (mode != 0 || variant == kPullFrontier || variant == kPullTopo || variant == kUnionFind) {
     st = ensure_symmetry(g);
     if (st) return st;
+  }
+  // The frequency rule picks the edge-balanced push for every iteration of SSSP,
+  // and of CC where union-find does not pay: that style's own kernel runs them.
+  // SSSP, us, own kernel / the selectors': RMAT 10^6 655 / 785, degree-ordered
+  // 2.5 x 10^6 1,086 / 1,205, 5.5 x 10^5 374 / 399.
+  if (mode == 1 && (algo == I2_SSSP ||
+                    (algo == I2_CC && !(((allowed_mask(g, algo) >> kUnionFind) & 1) &&
+                                        union_find_pays(g->g.nodes, g->gs.avgdeg))))) {
+    mode = 0;
+    variant = kVPCta;
+    o.sssp_delta = 0;  // options of the fixed style: not the rule's
+    o.sssp_budget = 0;
   }
   if ((mode == 0 || mode == 3) && !((allowed_mask(g, algo) >> variant) & 1)) return I2_ERR_UNSUPPORTED;
   if (mode == 3 && !((allowed_mask(g, algo) >> o.then_variant) & 1)) return I2_ERR_UNSUPPORTED;
@@ -1621,18 +1642,7 @@ int i2_graph_upload(const i2_eclgraph* h, i2_graph** out) {
 int i2_graph_hub(i2_graph* g, int* v) {
   if (!g || !v) return I2_ERR_ARG;
   I2_CK(cudaSetDevice(g->device));
-  int* d = nullptr;
-  I2_CK(dev_alloc(&d, sizeof(int)));
-  int h = INT_MAX;
-  cudaError_t e = cudaMemcpyAsync(d, &h, sizeof(int), cudaMemcpyHostToDevice, g->stream);
-  if (e == cudaSuccess) {
-    k_hub<<<4 * sm_count(), 256, 0, g->stream>>>(g->g, g->gs.maxdeg, d);
-    e = cudaMemcpyAsync(&h, d, sizeof(int), cudaMemcpyDeviceToHost, g->stream);
-  }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-  dev_free(d);
-  if (e != cudaSuccess) return cuda_status(e);
-  *v = h == INT_MAX ? 0 : h;
+  *v = g->hub;  // found with the degree statistics
   return I2_OK;
 }
 

@@ -55,43 +55,48 @@ static __device__ int heuristic_pick(const GStats& gs, int algo, int allowed, in
 // than any it was trained on it defers to the frequency rule (no inference):
 // measured on RMAT-24 and RMAT-26 BFS, its picks there cost 1.08-1.38x the
 // rule's time even with the size features clamped to the training range.
-static __device__ void select_next(const Ctx& c, CtlHead& S, int next_iter, int nxt, bool cond, int force) {
-  __shared__ float h1[kHidden], h2[kHidden], y[kOut];
+template <class H>
+static __device__ void select_next(const Ctx& c, H& S, int next_iter, int nxt, bool cond, int force) {
   const unsigned long long p = S.slot[nxt].packed;
   const int n = slot_size(p);
   const unsigned e = slot_edges(p);
-  const int mode = S.mode;
-  const bool learned = c.mlp && c.gs.nodes <= kMaxTrainedNodes;
-  const long long sn = S.sel_n, se = S.sel_e;
-  const bool moved = next_iter == 0 || 2LL * n > 3LL * sn || 3LL * n < 2LL * sn || 2LL * e > 3LL * se ||
-                     3LL * e < 2LL * se || next_iter - S.sel_iter >= 16;
-  const bool infer = mode == 2 && learned && cond && moved && force < 0;
-  if (infer) mlp_forward_block(c.mlp, S.feat, h1, h2, y);
-  if (threadIdx.x == 0) {
-    int v = S.fixed_variant;
-    if (mode == 3) {
-      v = next_iter >= S.then_at ? S.then_variant : S.fixed_variant;
-    } else if ((mode == 1 || mode == 2) && union_find_first(c.gs, S.algo, S.allowed, next_iter)) {
-      v = kUnionFind;
-    } else if (mode == 1 || (mode == 2 && !learned)) {
-      v = heuristic_pick(c.gs, S.algo, S.allowed, n, e);
-    } else if (mode == 2) {
-      v = S.variant;
-      if (infer) {
-        const int h = heuristic_pick(c.gs, S.algo, S.allowed, n, e);
-        float best = 3.0e38f;
-        int bv = -1;
-        for (int k = 0; k < kOut; ++k)  // per-iteration styles only (see union_find_first)
-          if (k != kUnionFind && ((S.allowed >> k) & 1) && y[k] < best) {
-            best = y[k];
-            bv = k;
-          }
-        v = (bv >= 0 && best + kLearnedMargin < y[h]) ? bv : h;
-        S.sel_n = n;
-        S.sel_e = e;
-        S.sel_iter = next_iter;
+  int v = S.fixed_variant;
+  if constexpr (H::kSelect) {
+    __shared__ float h1[kHidden], h2[kHidden], y[kOut];
+    const int mode = S.mode;
+    const bool learned = c.mlp && c.gs.nodes <= kMaxTrainedNodes;
+    const long long sn = S.sel_n, se = S.sel_e;
+    const bool moved = next_iter == 0 || 2LL * n > 3LL * sn || 3LL * n < 2LL * sn || 2LL * e > 3LL * se ||
+                       3LL * e < 2LL * se || next_iter - S.sel_iter >= 16;
+    const bool infer = mode == 2 && learned && cond && moved && force < 0;
+    if (infer) mlp_forward_block(c.mlp, S.feat, h1, h2, y);
+    if (threadIdx.x == 0) {
+      if (mode == 3) {
+        v = next_iter >= S.then_at ? S.then_variant : S.fixed_variant;
+      } else if ((mode == 1 || mode == 2) && union_find_first(c.gs, S.algo, S.allowed, next_iter)) {
+        v = kUnionFind;
+      } else if (mode == 1 || (mode == 2 && !learned)) {
+        v = heuristic_pick(c.gs, S.algo, S.allowed, n, e);
+      } else if (mode == 2) {
+        v = S.variant;
+        if (infer) {
+          const int h = heuristic_pick(c.gs, S.algo, S.allowed, n, e);
+          float best = 3.0e38f;
+          int bv = -1;
+          for (int k = 0; k < kOut; ++k)  // per-iteration styles only (see union_find_first)
+            if (k != kUnionFind && ((S.allowed >> k) & 1) && y[k] < best) {
+              best = y[k];
+              bv = k;
+            }
+          v = (bv >= 0 && best + kLearnedMargin < y[h]) ? bv : h;
+          S.sel_n = n;
+          S.sel_e = e;
+          S.sel_iter = next_iter;
+        }
       }
     }
+  }
+  if (threadIdx.x == 0) {
     if (force >= 0) v = force;
     S.variant = v;
     if (cond) atomicAdd(&c.ctl->hist[v], 1);
@@ -196,7 +201,8 @@ static __device__ int budget_next(CtlHead& S, const int* q, long long n, unsigne
 // that every block has added), advanced in shared memory by thread 0 while the
 // second warp writes the record and computes the next frontier's features, and
 // written back with one store per thread.
-static __device__ __forceinline__ void finish_iteration(const Ctx& c, CtlHead& S, int i, int cur, int nxt, int old) {
+template <class H>
+static __device__ __forceinline__ void finish_iteration(const Ctx& c, H& S, int i, int cur, int nxt, int old) {
   __shared__ int s_cond, s_force, s_clear;
   __shared__ int s_q[2];
   const unsigned long long t1 = globaltimer();

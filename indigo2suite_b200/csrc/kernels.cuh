@@ -36,7 +36,7 @@ KernelFn resident_fn(int v, bool wide) {
   switch (v) {
     case kVPThread: return relax_resident<ALG, kVPThread>;
     case kVPWarp: return relax_resident<ALG, kVPWarp>;
-    case kVPCta: return relax_resident<ALG, kVPCta>;
+    case kVPCta: return wide ? relax_resident<ALG, kVPCta, false, I2_FIXED_MIN_BLOCKS> : relax_resident<ALG, kVPCta>;
     case kVPBlock: return relax_resident<ALG, kVPBlock>;
     case kPullFrontier: return relax_resident<ALG, kPullFrontier>;
     case kPullTopo: return relax_resident<ALG, kPullTopo>;

@@ -541,7 +541,8 @@ __device__ __forceinline__ void clear_old(const Ctx& c, const CtlHead& S, int ol
   }
 }
 
-static __device__ __forceinline__ void finish_iteration(const Ctx& c, CtlHead& S, int i, int cur, int nxt, int old);
+template <class H>
+static __device__ __forceinline__ void finish_iteration(const Ctx& c, H& S, int i, int cur, int nxt, int old);
 
 // Copy the head of the control block to (or from) shared memory: one coalesced
 // access, from L2 (other blocks wrote it). Block-uniform; the caller synchronises.
@@ -580,8 +581,8 @@ __device__ __forceinline__ int active_blocks(const Ctx& c, const CtlHead& S, int
 // Common epilogue: publish block statistics and let the last block finish the
 // iteration. Every block of the launch, active or not, counts into `done`, so
 // the iteration advances only after every block has read its state.
-template <typename Sh>
-__device__ __forceinline__ bool block_epilogue(const Ctx& c, CtlHead& S, Sh& s, const Acc& a, int i, int cur, int nxt,
+template <class H, typename Sh>
+__device__ __forceinline__ bool block_epilogue(const Ctx& c, H& S, Sh& s, const Acc& a, int i, int cur, int nxt,
                                                int old) {
   acc_reduce(a, s);
   if (threadIdx.x == 0) {
@@ -601,8 +602,8 @@ __device__ __forceinline__ bool block_epilogue(const Ctx& c, CtlHead& S, Sh& s, 
 }
 
 // Epilogue of a block with no work in this launch.
-template <typename Sh>
-__device__ __forceinline__ bool idle_epilogue(const Ctx& c, CtlHead& S, Sh& s, int i, int cur, int nxt, int old) {
+template <class H, typename Sh>
+__device__ __forceinline__ bool idle_epilogue(const Ctx& c, H& S, Sh& s, int i, int cur, int nxt, int old) {
   if (threadIdx.x == 0) s.last = (arrive(c) == gridDim.x - 1);
   __syncthreads();
   const bool last = s.last;
@@ -620,8 +621,8 @@ __device__ __forceinline__ void block_prologue(const Ctx& c) {
 // Data-driven push, vertex granularity: thread, warp or block per frontier
 // vertex. Heavy vertices are skipped here and taken by the heavy path.
 
-template <int ALG, int VAR>
-__device__ __forceinline__ bool body_push(const Ctx& c, CtlHead& S, Stage& s) {
+template <int ALG, int VAR, class H>
+__device__ __forceinline__ bool body_push(const Ctx& c, H& S, Stage& s) {
   block_prologue(c);
   const int i = S.iter;
   const int cur = i % 3, nxt = (i + 1) % 3, old = (i + 2) % 3;
@@ -892,10 +893,13 @@ __device__ __forceinline__ void warp_resolve(const Ctx& c, WarpStage& ws, Acc& a
 // all dist[] loads first, then all atomicMins, then the queue (its length qn
 // is warp-uniform and returned). BFS runs level by level in every style, so an
 // unreached neighbour takes the level with a plain store (every writer of the
-// iteration writes the same one).
+// iteration writes the same one). CC lowers a label many times in an iteration
+// (all vertices relax at once), so a vertex that the next frontier's bitmap
+// already holds is not queued again (ER 2M: 1,095 -> 931 us; for SSSP the read
+// costs more than it saves, 2%).
 template <int ALG, bool DEFER>
-__device__ __forceinline__ int warp_relax_batch(const Ctx& c, WarpStage& ws, Acc& a, const int* du, const int* nv,
-                                                const int* wv, const bool* ok, int thr, int qn) {
+__device__ __forceinline__ int warp_relax_batch(const Ctx& c, WarpStage& ws, Acc& a, int nxt, const int* du,
+                                                const int* nv, const int* wv, const bool* ok, int thr, int qn) {
   int cand[kEdgesPerThread], old[kEdgesPerThread];
   const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -911,11 +915,19 @@ __device__ __forceinline__ int warp_relax_batch(const Ctx& c, WarpStage& ws, Acc
       old[r] = atomicMin(&c.dist[nv[r]], cand[r]);
     }
   }
+  bool queue[kEdgesPerThread];
 #pragma unroll
   for (int r = 0; r < kEdgesPerThread; ++r) {
-    const bool fell = cand[r] < old[r];
-    const unsigned m = __ballot_sync(0xffffffffu, fell);
-    if (fell) {
+    queue[r] = cand[r] < old[r];
+    if (ALG == kCC && queue[r]) {
+      a.mindist = min(a.mindist, cand[r]);
+      queue[r] = !((*(volatile unsigned*)&c.bm[nxt][nv[r] >> 5] >> (nv[r] & 31)) & 1u);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kEdgesPerThread; ++r) {
+    const unsigned m = __ballot_sync(0xffffffffu, queue[r]);
+    if (queue[r]) {
       const int p = qn + __popc(m & ((1u << lane) - 1u));
       const bool far = DEFER && cand[r] >= thr;
       ws.q[p] = far ? ~nv[r] : nv[r];
@@ -1020,7 +1032,8 @@ __device__ __forceinline__ void split_flush(const Ctx& c, WarpStage& ws, int nxt
 //    others onto the pile (nothing is relaxed).
 // The loop is block-uniform: a block appends the entries it keeps with one
 // atomic per pass (a single pile counter takes every block's appends).
-__device__ __forceinline__ bool body_split(const Ctx& c, CtlHead& S, EBSharedFar& sh, int i, int cur, int nxt, int old) {
+template <class H>
+__device__ __forceinline__ bool body_split(const Ctx& c, H& S, EBSharedFar& sh, int i, int cur, int nxt, int old) {
   __shared__ int s_keep[kWarpsPerBlock];
   __shared__ unsigned s_kbase;
   EpiStage& s = sh.s;
@@ -1162,8 +1175,8 @@ __device__ __forceinline__ bool body_split(const Ctx& c, CtlHead& S, EBSharedFar
 
 // DEFER: SSSP near/far ordering (pushes at or above the threshold go onto the
 // far pile, and split launches refill the frontier from it).
-template <int ALG, bool DEFER = false>
-__device__ __forceinline__ bool body_edge_balanced(const Ctx& c, CtlHead& S, EBSharedT<DEFER>& sh) {
+template <int ALG, bool DEFER = false, class H>
+__device__ __forceinline__ bool body_edge_balanced(const Ctx& c, H& S, EBSharedT<DEFER>& sh) {
   static_assert(!DEFER || ALG == kSSSP, "near/far ordering is for SSSP");
   EpiStage& s = sh.s;
   block_prologue(c);
@@ -1249,7 +1262,7 @@ __device__ __forceinline__ bool body_edge_balanced(const Ctx& c, CtlHead& S, EBS
           ok[r] = Op<ALG>::valid(du[r]);
         }
       }
-      qn = warp_relax_batch<ALG, DEFER>(c, ws, a, du, nv, wv, ok, thr, qn);
+      qn = warp_relax_batch<ALG, DEFER>(c, ws, a, nxt, du, nv, wv, ok, thr, qn);
       // the next tile starts at e1: its first entry is the last one with offset <= e1
       j += (ws.off[m] == e1) ? m : m - 1;
       __syncwarp();
@@ -1268,8 +1281,8 @@ __device__ __forceinline__ bool body_edge_balanced(const Ctx& c, CtlHead& S, EBS
 // ---------------------------------------------------------------------------
 // Bitmap-gated topology sweep: thread per vertex, light vertices only; heavy
 // frontier vertices take the shared heavy path.
-template <int ALG>
-__device__ __forceinline__ bool body_push_topo(const Ctx& c, CtlHead& S, Stage& s) {
+template <int ALG, class H>
+__device__ __forceinline__ bool body_push_topo(const Ctx& c, H& S, Stage& s) {
   block_prologue(c);
   stage_init(s);
   Acc a;
@@ -1298,8 +1311,8 @@ __device__ __forceinline__ bool body_push_topo(const Ctx& c, CtlHead& S, Stage& 
 
 // ---------------------------------------------------------------------------
 // Edge-centric sweep over all CSR entries, gated by the source's frontier bit.
-template <int ALG>
-__device__ __forceinline__ bool body_edge_topo(const Ctx& c, CtlHead& S, Stage& s) {
+template <int ALG, class H>
+__device__ __forceinline__ bool body_edge_topo(const Ctx& c, H& S, Stage& s) {
   block_prologue(c);
   stage_init(s);
   Acc a;
@@ -1360,8 +1373,8 @@ __device__ __forceinline__ bool body_edge_topo(const Ctx& c, CtlHead& S, Stage& 
 // covers 32 consecutive vertices, i.e. exactly one bitmap word, so the next
 // frontier's bitmap is written with one plain store per warp. dist[v] is only
 // written by v's own thread, so no atomics are needed on it.
-template <int ALG, bool FRONTIER>
-__device__ __forceinline__ bool body_pull(const Ctx& c, CtlHead& S, Stage& s) {
+template <int ALG, bool FRONTIER, class H>
+__device__ __forceinline__ bool body_pull(const Ctx& c, H& S, Stage& s) {
   block_prologue(c);
   stage_init(s);
   Acc a;
@@ -1581,8 +1594,8 @@ __device__ __forceinline__ void uf_sample_giant(const Ctx& c, CtlHead& S) {
 // 231, ER 4M 487 -> 270, RMAT-20 272 -> 221, ER 600,000 248 -> 169, grid 4096^2
 // 1,380 -> 666, grid 1000^2 191 -> 158. Bound by the latency of dependent
 // parent reads.
-template <int ALG>
-__device__ __forceinline__ bool body_union(const Ctx& c, CtlHead& S, Stage& s) {
+template <int ALG, class H>
+__device__ __forceinline__ bool body_union(const Ctx& c, H& S, Stage& s) {
   block_prologue(c);
   stage_init(s);
   Acc a;
@@ -1718,7 +1731,8 @@ __device__ __forceinline__ void mis_flush(const Ctx& c, Stage& s, int nxt) {
   __syncthreads();
 }
 
-__device__ __forceinline__ bool body_mis(const Ctx& c, CtlHead& S, Stage& s) {
+template <class H>
+__device__ __forceinline__ bool body_mis(const Ctx& c, H& S, Stage& s) {
   block_prologue(c);
   const int i = S.iter;
   const int cur = i % 3, nxt = (i + 1) % 3, old = (i + 2) % 3;
@@ -1917,7 +1931,7 @@ __device__ __forceinline__ bool body_mis(const Ctx& c, CtlHead& S, Stage& s) {
 template <int ALG, int VAR>
 __global__ void __launch_bounds__(kBlock) relax_push(const __grid_constant__ Ctx c) {
   __shared__ Stage s;
-  __shared__ CtlHead S;
+  __shared__ SelectHead S;
   load_head(c, S);
   __syncthreads();
   body_push<ALG, VAR>(c, S, s);
@@ -1926,7 +1940,7 @@ __global__ void __launch_bounds__(kBlock) relax_push(const __grid_constant__ Ctx
 template <int ALG>
 __global__ void __launch_bounds__(kBlock, I2_EB_MIN_BLOCKS) relax_edge_balanced(const __grid_constant__ Ctx c) {
   __shared__ EBShared sh;
-  __shared__ CtlHead S;
+  __shared__ SelectHead S;
   load_head(c, S);
   __syncthreads();
   body_edge_balanced<ALG>(c, S, sh);
@@ -1934,7 +1948,7 @@ __global__ void __launch_bounds__(kBlock, I2_EB_MIN_BLOCKS) relax_edge_balanced(
 
 static __global__ void __launch_bounds__(kBlock, I2_FIXED_MIN_BLOCKS) relax_mis(const __grid_constant__ Ctx c) {
   __shared__ Stage s;
-  __shared__ CtlHead S;
+  __shared__ SelectHead S;
   load_head(c, S);
   __syncthreads();
   body_mis(c, S, s);
@@ -1943,7 +1957,7 @@ static __global__ void __launch_bounds__(kBlock, I2_FIXED_MIN_BLOCKS) relax_mis(
 // Edge-balanced SSSP push with near/far ordering (Ctl::delta != 0).
 static __global__ void __launch_bounds__(kBlock, I2_EB_MIN_BLOCKS) relax_near_far(const __grid_constant__ Ctx c) {
   __shared__ EBSharedFar sh;
-  __shared__ CtlHead S;
+  __shared__ SelectHead S;
   load_head(c, S);
   __syncthreads();
   body_edge_balanced<kSSSP, true>(c, S, sh);
@@ -1952,7 +1966,7 @@ static __global__ void __launch_bounds__(kBlock, I2_EB_MIN_BLOCKS) relax_near_fa
 template <int ALG>
 __global__ void __launch_bounds__(kBlock) relax_push_topo(const __grid_constant__ Ctx c) {
   __shared__ Stage s;
-  __shared__ CtlHead S;
+  __shared__ SelectHead S;
   load_head(c, S);
   __syncthreads();
   body_push_topo<ALG>(c, S, s);
@@ -1961,7 +1975,7 @@ __global__ void __launch_bounds__(kBlock) relax_push_topo(const __grid_constant_
 template <int ALG>
 __global__ void __launch_bounds__(kBlock) relax_edge_topo(const __grid_constant__ Ctx c) {
   __shared__ Stage s;
-  __shared__ CtlHead S;
+  __shared__ SelectHead S;
   load_head(c, S);
   __syncthreads();
   body_edge_topo<ALG>(c, S, s);
@@ -1970,7 +1984,7 @@ __global__ void __launch_bounds__(kBlock) relax_edge_topo(const __grid_constant_
 template <int ALG>
 __global__ void __launch_bounds__(kBlock) relax_union(const __grid_constant__ Ctx c) {
   __shared__ Stage s;
-  __shared__ CtlHead S;
+  __shared__ SelectHead S;
   load_head(c, S);
   __syncthreads();
   body_union<ALG>(c, S, s);
@@ -1979,7 +1993,7 @@ __global__ void __launch_bounds__(kBlock) relax_union(const __grid_constant__ Ct
 template <int ALG, bool FRONTIER>
 __global__ void __launch_bounds__(kBlock) relax_pull(const __grid_constant__ Ctx c) {
   __shared__ Stage s;
-  __shared__ CtlHead S;
+  __shared__ SelectHead S;
   load_head(c, S);
   __syncthreads();
   body_pull<ALG, FRONTIER>(c, S, s);
@@ -2028,8 +2042,8 @@ __device__ __forceinline__ bool grid_wait(const Ctx& c, unsigned gen, unsigned l
   return ok;
 }
 
-template <int ALG, int VAR, bool DEFER>
-__device__ __forceinline__ bool run_body(const Ctx& c, CtlHead& S, AnyShared<DEFER>& sh) {
+template <int ALG, int VAR, bool DEFER, class H>
+__device__ __forceinline__ bool run_body(const Ctx& c, H& S, AnyShared<DEFER>& sh) {
   if constexpr (ALG == kMIS) {
     return body_mis(c, S, sh.st);  // one style
   } else {
@@ -2059,7 +2073,7 @@ template <int ALG, int VAR, bool DEFER = false,
                                           : I2_FIXED_MIN_BLOCKS)>
 __global__ void __launch_bounds__(kBlock, MINB) relax_resident(const __grid_constant__ Ctx c) {
   __shared__ AnyShared<DEFER> sh;
-  __shared__ CtlHead S;
+  __shared__ typename std::conditional<(VAR < 0), SelectHead, FixedHead>::type S;
   // thread 0's: barrier generation, whether to go on, the test hook (kept in
   // shared memory: the bodies have no register to spare)
   __shared__ unsigned s_gen;
@@ -2100,7 +2114,7 @@ __global__ void __launch_bounds__(kBlock, MINB) relax_resident(const __grid_cons
 template <int ALG, int MINB = I2_SEL_MIN_BLOCKS>
 __global__ void __launch_bounds__(kBlock, MINB) relax_dispatch(const __grid_constant__ Ctx c) {
   __shared__ AnyShared<> sh;
-  __shared__ CtlHead S;
+  __shared__ SelectHead S;
   load_head(c, S);
   __syncthreads();
   switch (S.variant) {

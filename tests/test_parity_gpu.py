@@ -441,8 +441,10 @@ def test_union_find_order_and_links_on_sparse_and_dense_graphs(gpu, n):
     # with several components and isolated vertices; from the initial labels and
     # from a propagation state
     rng = np.random.default_rng(n)
-    for pairs in (max(1, n // 3), 2 * n, 5 * n):
-        u, v = rng.integers(0, n, pairs), rng.integers(0, n, pairs)
+    for pairs in (max(1, n // 3), 2 * n, 5 * n, -5 * n):
+        u, v = rng.integers(0, n, abs(pairs)), rng.integers(0, n, abs(pairs))
+        if pairs < 0:  # numbered with the hub in front
+            u[: n // 2] = 0
         u, v = np.concatenate([u, v]), np.concatenate([v, u])
         key = np.unique(u[u != v] * np.int64(n) + v[u != v])
         ni = np.zeros(n + 1, np.int32)
