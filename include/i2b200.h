@@ -81,9 +81,8 @@ enum {
 
 /* Loop modes. */
 enum {
-  I2_LOOP_GRAPH = 0,   /* whole traversal is one CUDA graph; its relax kernel is one
-                          cooperative launch that runs every iteration, the grid
-                          meeting at a barrier between iterations */
+  I2_LOOP_GRAPH = 0,   /* a start kernel and one cooperative launch that runs every
+                          iteration, the grid meeting at a barrier between them */
   I2_LOOP_HOST = 1,    /* host launches each iteration and reads the frontier size back */
   I2_LOOP_RELAUNCH = 2 /* one CUDA graph with a device-side while loop that launches
                           the relax kernel once per iteration */

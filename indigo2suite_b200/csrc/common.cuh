@@ -206,6 +206,7 @@ struct Ctl : CtlHead {
   alignas(128) unsigned bar_gen;  // barrier generation, bumped once per iteration
   int status;               // error bits, see kStatus*
   int hist[kMaxVariants];   // launches per variant
+  unsigned long long reached[2];  // reached vertices and the sum of their degrees (k_reached)
 };
 
 // Union-find CC pays on graphs of 2^19 vertices or more, or of average degree

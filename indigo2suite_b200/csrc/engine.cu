@@ -1,18 +1,17 @@
 // B200 relaxation engine: device graphs, traversal runs and the C ABI of
 // include/i2b200.h for BFS, SSSP and CC.
 //
-// A traversal is: reset the control block, fill dist/labels and seed F_0
-// (k_fill, k_seed), then one relax launch per iteration until the frontier is
-// empty (the do-while of the reference's host drivers, e.g.
+// A traversal is: reset the control block, fill dist/labels and seed F_0, then
+// one relaxation per iteration until the frontier is empty (the do-while of the
+// reference's host drivers, e.g.
 // BFS_CUDA_V_Data_Push_..._Warp_..._NonDup.cu:112-122). In the default loop
-// mode (I2_LOOP_GRAPH) the whole sequence is one CUDA graph whose WHILE
-// conditional node holds one cooperative relax launch that runs every
-// iteration itself, its blocks meeting at a bounded barrier between
-// iterations (relax_resident, relax.cuh). I2_LOOP_RELAUNCH keeps one launch
-// per iteration inside the graph: the fixed style's kernel, or the dispatch
-// kernel whose blocks branch on the style picked for this iteration. Either
-// way the last block of an iteration picks the next style and sets the loop
-// condition on the device, so there is no host round trip per iteration.
+// mode (I2_LOOP_GRAPH) that is two launches: k_start, and one cooperative
+// launch that runs every iteration itself, its blocks meeting at a bounded
+// barrier between iterations (relax_resident, relax.cuh). I2_LOOP_RELAUNCH is a
+// CUDA graph whose WHILE conditional node launches one kernel per iteration:
+// the fixed style's, or the dispatch kernel whose blocks branch on the style
+// picked for this iteration. Either way the last block of an iteration picks
+// the next style on the device, so there is no host round trip per iteration.
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cmath>
@@ -90,6 +89,18 @@ __global__ void __launch_bounds__(kBlock) k_fill(Ctx c) {
   }
 }
 
+// Whole block: the features of the seeded frontier F_0, and the first style.
+static __device__ void select_first(const Ctx& c, SelectHead& S) {
+  if (threadIdx.x < kFeatures) {
+    const Slot& f = S.slot[0];
+    S.feat[threadIdx.x] = frontier_feature(threadIdx.x, c.gs, S.algo, 0, slot_size(f.packed), slot_size(f.hpacked),
+                                           slot_edges(f.packed), f.maxdeg, S.visited);
+  }
+  __syncthreads();
+  select_next(c, S, 0, 0, true, -1);
+  __syncthreads();
+}
+
 // One block: seed the sources (BFS/SSSP) and select the first variant.
 template <int ALG>
 __global__ void __launch_bounds__(kBlock) k_seed(Ctx c) {
@@ -129,14 +140,7 @@ __global__ void __launch_bounds__(kBlock) k_seed(Ctx c) {
   __shared__ SelectHead S;
   load_head(c, S);
   __syncthreads();
-  if (threadIdx.x < kFeatures) {
-    const Slot& f = S.slot[0];
-    S.feat[threadIdx.x] = frontier_feature(threadIdx.x, c.gs, S.algo, 0, slot_size(f.packed), slot_size(f.hpacked),
-                                           slot_edges(f.packed), f.maxdeg, S.visited);
-  }
-  __syncthreads();
-  select_next(c, S, 0, 0, true, -1);
-  __syncthreads();
+  select_first(c, S);
   store_head(c, S);
 }
 
@@ -148,32 +152,104 @@ struct RunParams {
   bool operator!=(const RunParams& o) const { return std::memcmp(this, &o, sizeof(RunParams)) != 0; }
 };
 
+// The head of a run with these parameters (all its other words are zero).
+static __device__ __forceinline__ void reset_head(CtlHead& S, const RunParams& p) {
+  for (int k = 0; k < 3; ++k) S.slot[k].mindist = kInf;
+  S.tstart = ~0ull;
+  S.iter_cap = p.iter_cap;
+  S.mode = p.mode;
+  S.fixed_variant = p.fixed_variant;
+  S.variant = p.fixed_variant;
+  S.allowed = p.allowed;
+  S.src = p.src;
+  S.nsrc = p.nsrc;
+  S.algo = p.algo;
+  S.delta = p.delta;
+  S.hshift = p.hshift;
+  S.then_at = p.then_at;
+  S.then_variant = p.then_variant;
+  S.hold = p.hold;
+  S.uf_start = p.uf_start;
+  S.uf_step = p.uf_step;
+  S.stall_ns = (unsigned long long)p.stall_ms * 1000000ull;
+  S.threshold = p.delta > 0 ? p.delta : kInf;  // sources start at 0
+  S.pmin[0] = kInf;
+  S.pmin[1] = kInf;
+}
+
 __global__ void k_reset(Ctl* ctl, RunParams p) {
   unsigned* w = reinterpret_cast<unsigned*>(ctl);
   for (unsigned k = threadIdx.x; k < sizeof(Ctl) / sizeof(unsigned); k += blockDim.x) w[k] = 0u;
   __syncthreads();
-  if (threadIdx.x != 0) return;
-  for (int k = 0; k < 3; ++k) ctl->slot[k].mindist = kInf;
-  ctl->tstart = ~0ull;
-  ctl->iter_cap = p.iter_cap;
-  ctl->mode = p.mode;
-  ctl->fixed_variant = p.fixed_variant;
-  ctl->variant = p.fixed_variant;
-  ctl->allowed = p.allowed;
-  ctl->src = p.src;
-  ctl->nsrc = p.nsrc;
-  ctl->algo = p.algo;
-  ctl->delta = p.delta;
-  ctl->hshift = p.hshift;
-  ctl->then_at = p.then_at;
-  ctl->then_variant = p.then_variant;
-  ctl->hold = p.hold;
-  ctl->uf_start = p.uf_start;
-  ctl->uf_step = p.uf_step;
-  ctl->stall_ns = (unsigned long long)p.stall_ms * 1000000ull;
-  ctl->threshold = p.delta > 0 ? p.delta : kInf;  // sources start at 0
-  ctl->pmin[0] = kInf;
-  ctl->pmin[1] = kInf;
+  if (threadIdx.x == 0) reset_head(*ctl, p);
+}
+
+// Start of a resident traversal: control block, bitmaps and values in one
+// kernel. Where no frontier of many vertices is to be built (one source, or
+// union-find from the first iteration) it seeds the frontier and selects the
+// first variant too, so that the traversal is two launches; CC, MIS and runs
+// from many sources have k_fill and k_seed after it. Five nodes of a CUDA graph
+// (memset, reset, fill, seed, conditional loop) took 16-20 us more: SSSP on RMAT
+// with 3,001 vertices 151 -> 130 us, BFS RMAT-20 138 -> 118; and instantiating
+// the graph cost a new graph's first traversal 0.25 ms.
+template <int ALG>
+__global__ void __launch_bounds__(kBlock) k_start(const __grid_constant__ Ctx c, RunParams p, unsigned words) {
+  const bool single = (ALG == kBFS || ALG == kSSSP) && !c.srcs;
+  const bool whole = single || (ALG == kCC && p.uf_start);
+  const int V = c.g.nodes;
+  const int src = single ? p.src : -1;
+  const int deg = single ? c.g.nindex[src + 1] - c.g.nindex[src] : 0;
+  const unsigned stride = gridDim.x * kBlock;
+  const unsigned tid = blockIdx.x * kBlock + threadIdx.x;
+  // bitmaps, far-pile bitmap and histograms; a vertex without edges is never in a frontier
+  const unsigned sword = deg > 0 ? (unsigned)src >> 5 : ~0u;
+  for (unsigned w = tid; w < words; w += stride) c.bm[0][w] = w == sword ? 1u << (src & 31) : 0u;
+  if (whole || ALG == kBFS || ALG == kSSSP) {
+    // values, 16 bytes a store (the array starts on a 256-byte boundary)
+    const unsigned quads = (unsigned)V >> 2;
+    int4* d4 = reinterpret_cast<int4*>(c.dist);
+    for (unsigned q = tid; q < quads; q += stride) {
+      const int v = (int)(q << 2);
+      d4[q] = ALG == kCC ? make_int4(v, v + 1, v + 2, v + 3)
+                         : make_int4(v == src ? 0 : kInf, v + 1 == src ? 0 : kInf, v + 2 == src ? 0 : kInf,
+                                     v + 3 == src ? 0 : kInf);
+    }
+    for (unsigned v = (quads << 2) + tid; v < (unsigned)V; v += stride)
+      c.dist[v] = ALG == kCC ? (int)v : (int)v == src ? 0 : kInf;
+  }
+  if (blockIdx.x != 0) return;
+  __shared__ SelectHead S;
+  for (unsigned k = threadIdx.x; k < sizeof(Ctl) / sizeof(unsigned); k += kBlock)
+    reinterpret_cast<unsigned*>(c.ctl)[k] = 0u;
+  if (threadIdx.x < kHeadWords) reinterpret_cast<unsigned*>(&S)[threadIdx.x] = 0u;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    reset_head(S, p);
+    Slot& sl = S.slot[0];
+    if (single) {
+      S.visited = 1;
+      sl.mindist = 0;
+      if (deg > 0) {
+        sl.maxdeg = deg;
+        sl.packed = (1ull << 32) | (unsigned)deg;
+        c.wl[0][0] = src;
+        c.woff[0][0] = 0;
+        if (deg >= c.heavy) {
+          sl.hpacked = (1ull << 32) | (unsigned)heavy_tiles(deg);
+          c.hwl[0][0] = src;
+          c.htoff[0][0] = 0;
+        }
+      }
+    } else if (whole) {  // the record's frontier: every vertex
+      S.visited = V;
+      sl.packed = ((unsigned long long)V << 32) | (unsigned)c.g.edges;
+      sl.maxdeg = c.gs.maxdeg;
+      sl.mindist = 0;
+    }
+  }
+  __syncthreads();
+  if (whole) select_first(c, S);
+  store_head(c, S);
 }
 
 // ---------------------------------------------------------------------------
@@ -201,7 +277,7 @@ __global__ void k_validate(DGraph g, int* bad) {
 struct DevStats {
   unsigned long long hub;  // largest degree << 32 | ~vertex: the lowest ID on ties
   int nheavy;
-  int wmin;
+  unsigned winv;           // INT_MAX - smallest weight (0: no weights)
   int unsorted;
   int asym;
   int pad;
@@ -222,30 +298,31 @@ __global__ void k_degree_stats(DGraph g, int heavy, DevStats* st) {
     nh += d >= heavy;
     s2 += (double)d * d;
   }
-  int wmin = INT_MAX;
+  unsigned winv = 0;
   double ws = 0.0;
   if (g.eweight)
     for (long long e = tid; e < g.edges; e += stride) {
       const int w = g.eweight[e];
-      wmin = min(wmin, w);
+      winv = max(winv, (unsigned)INT_MAX - (unsigned)w);
       ws += (double)w;
     }
   // one set of atomics per block: from every thread they were 0.4 ms on one line
   nh = __reduce_add_sync(0xffffffffu, nh);
-  wmin = __reduce_min_sync(0xffffffffu, wmin);
+  winv = __reduce_max_sync(0xffffffffu, winv);
   for (int o = 16; o > 0; o >>= 1) {
     hub = max(hub, __shfl_down_sync(0xffffffffu, hub, o));
     s2 += __shfl_down_sync(0xffffffffu, s2, o);
     ws += __shfl_down_sync(0xffffffffu, ws, o);
   }
-  __shared__ int snh[kWarp], swm[kWarp];
+  __shared__ int snh[kWarp];
+  __shared__ unsigned swi[kWarp];
   __shared__ unsigned long long shub[kWarp];
   __shared__ double ss2[kWarp], sws[kWarp];
   const int wid = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   if ((threadIdx.x & 31) == 0) {
     shub[wid] = hub;
     snh[wid] = nh;
-    swm[wid] = wmin;
+    swi[wid] = winv;
     ss2[wid] = s2;
     sws[wid] = ws;
   }
@@ -254,13 +331,13 @@ __global__ void k_degree_stats(DGraph g, int heavy, DevStats* st) {
   for (int k = 1; k < nwarp; ++k) {
     hub = max(hub, shub[k]);
     nh += snh[k];
-    wmin = min(wmin, swm[k]);
+    winv = max(winv, swi[k]);
     s2 += ss2[k];
     ws += sws[k];
   }
   atomicMax(&st->hub, hub);
   atomicAdd(&st->nheavy, nh);
-  atomicMin(&st->wmin, wmin);
+  atomicMax(&st->winv, winv);
   atomicAdd(&st->sumsq, s2);
   if (g.eweight) atomicAdd(&st->wsum, ws);
 }
@@ -336,10 +413,19 @@ __global__ void k_reached(DGraph g, const int* dist, unsigned long long* out) {
     nv += __shfl_down_sync(0xffffffffu, nv, o);
     ne += __shfl_down_sync(0xffffffffu, ne, o);
   }
+  __shared__ unsigned long long sv[kWarp], se[kWarp];
   if ((threadIdx.x & 31) == 0) {
-    atomicAdd(&out[0], nv);
-    atomicAdd(&out[1], ne);
+    sv[threadIdx.x >> 5] = nv;
+    se[threadIdx.x >> 5] = ne;
   }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int k = 1; k < (int)(blockDim.x >> 5); ++k) {
+    nv += sv[k];
+    ne += se[k];
+  }
+  atomicAdd(&out[0], nv);
+  atomicAdd(&out[1], ne);
 }
 
 // Values of a traversal on the degree-ordered copy, back in original IDs:
@@ -492,14 +578,13 @@ using namespace i2;
 // Graph handle.
 
 struct ExecKey {
-  int algo, mode, variant, multi, near_far, resident;
+  int algo, mode, variant, multi, near_far;
   bool operator<(const ExecKey& o) const {
     if (algo != o.algo) return algo < o.algo;
     if (mode != o.mode) return mode < o.mode;
     if (variant != o.variant) return variant < o.variant;
     if (multi != o.multi) return multi < o.multi;
-    if (near_far != o.near_far) return near_far < o.near_far;
-    return resident < o.resident;
+    return near_far < o.near_far;
   }
 };
 
@@ -525,6 +610,8 @@ struct i2_graph {
   int blocks_per_sm = 8;  // cap; the occupancy of each kernel decides below it
   // workspace
   bool ws_ready = false;
+  char* ws_base = nullptr;     // one block: values, frontier lists, bitmaps, control block, records
+  char* heavy_base = nullptr;  // one block: the heavy lists (sized by the heavy threshold)
   int* dist = nullptr;
   int* wl[3] = {nullptr, nullptr, nullptr};
   unsigned* woff[3] = {nullptr, nullptr, nullptr};
@@ -535,17 +622,19 @@ struct i2_graph {
   unsigned long long* hist = nullptr;  // near/far distance histograms, after fbm
   int* pile[2] = {nullptr, nullptr};
   int bm_words = 0;
-  bool resident_ok = true;  // cleared if the device refuses the cooperative loop node
+  bool resident_ok = true;  // cleared if the device refuses the cooperative launch
   Ctl* ctl = nullptr;
   IterRec* recs = nullptr;
   int rec_cap = 0;
   int* srcs = nullptr;
   int srcs_cap = 0;
-  unsigned long long* reach = nullptr;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, ev3 = nullptr;
   Ctl* h_ctl = nullptr;  // pinned
+  int* h_stage = nullptr;  // pinned, kStageInts ints (results of small graphs on their way to the caller)
+  bool staged = false;     // the last run's result has reached the caller's array
   std::map<ExecKey, ExecEntry> execs;
+  std::map<KernelFn, int> grids;  // launch grids of the resident kernels
   std::vector<cudaGraph_t> graphs;
   int last_iters = 0;
   // sweep scratch
@@ -570,6 +659,7 @@ namespace {
 struct DevPool {
   cudaMemPool_t pool = nullptr;
   cudaStream_t s = nullptr;  // allocations and frees are ordered on it
+  cudaStream_t copy[2] = {nullptr, nullptr};  // uploads (several at once share them: each waits for both)
 };
 std::mutex g_pool_mu;
 DevPool g_pools[64];
@@ -603,6 +693,15 @@ static DevPool* dev_pool() {
       cudaMemPoolDestroy(pool);
       return nullptr;
     }
+    for (cudaStream_t& cs : p.copy)
+      if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess) {
+        cudaGetLastError();
+        if (p.copy[0]) cudaStreamDestroy(p.copy[0]);
+        p.copy[0] = p.copy[1] = nullptr;
+        cudaStreamDestroy(s);
+        cudaMemPoolDestroy(pool);
+        return nullptr;
+      }
     p.pool = pool;
     p.s = s;
   }
@@ -627,13 +726,19 @@ cudaError_t dev_alloc_bytes(void** ptr, size_t bytes) {
   return e;
 }
 
-void dev_free(void* ptr) {
-  if (!ptr) return;
+static void dev_free_all(void* const* ptrs, int n) {
   DevPool* p = dev_pool();
   if (!p) return;
-  cudaDeviceSynchronize();
-  cudaFreeAsync(ptr, p->s);
+  bool waited = false;
+  for (int k = 0; k < n; ++k) {
+    if (!ptrs[k]) continue;
+    if (!waited) cudaDeviceSynchronize();
+    waited = true;
+    cudaFreeAsync(ptrs[k], p->s);
+  }
 }
+
+void dev_free(void* ptr) { dev_free_all(&ptr, 1); }
 
 static int trim_pool() {
   DevPool* p = dev_pool();
@@ -661,71 +766,101 @@ static void ctl_host_put(Ctl* c) {
   g_ctl_free.push_back(c);
 }
 
+// Results of up to kStageInts values go to the caller through a pinned block,
+// copied with the report before its one wait for the device; a copy into
+// pageable memory waits by itself after that. Blocks of freed graphs are kept
+// for the next ones, at most kStageKept of them.
+constexpr int kStageInts = 1 << 16;
+constexpr size_t kStageKept = 16;
+static std::mutex g_stage_mu;
+static std::vector<int*> g_stage_free;
+
+static bool stage_get(i2_graph* g) {
+  if (g->g.nodes > kStageInts) return false;
+  if (g->h_stage) return true;
+  {
+    std::lock_guard<std::mutex> lk(g_stage_mu);
+    if (!g_stage_free.empty()) {
+      g->h_stage = g_stage_free.back();
+      g_stage_free.pop_back();
+      return true;
+    }
+  }
+  if (cudaMallocHost(&g->h_stage, sizeof(int) * kStageInts) == cudaSuccess) return true;
+  cudaGetLastError();
+  g->h_stage = nullptr;
+  return false;
+}
+
+static void stage_put(i2_graph* g) {
+  if (!g->h_stage) return;
+  {
+    std::lock_guard<std::mutex> lk(g_stage_mu);
+    if (g_stage_free.size() < kStageKept) {
+      g_stage_free.push_back(g->h_stage);
+      g->h_stage = nullptr;
+    }
+  }
+  if (g->h_stage) cudaFreeHost(g->h_stage);
+  g->h_stage = nullptr;
+}
+
 static void drop_execs(i2_graph* g) {
   for (auto& kv : g->execs) cudaGraphExecDestroy(kv.second.ex);
   g->execs.clear();
+  g->grids.clear();
 }
 
 static void free_graph_state(i2_graph* g) {
   drop_execs(g);
   for (auto gr : g->graphs) cudaGraphDestroy(gr);
   g->graphs.clear();
-  dev_free(g->dist);
-  for (int k = 0; k < 3; ++k) {
-    dev_free(g->wl[k]);
-    dev_free(g->woff[k]);
-    dev_free(g->hwl[k]);
-    dev_free(g->htoff[k]);
+  // one wait for the device, then every block back to the pool
+  void* blocks[] = {g->ws_base, g->heavy_base, g->pile[0],  g->pile[1], g->srcs,  g->snap_dist,
+                    g->snap_bm, g->snap_wl,    g->snap_hwl, g->d_sp,    g->d_inv, nullptr,
+                    nullptr,    nullptr};
+  int nb = 11;
+  if (g->owns) {
+    blocks[nb++] = g->d_nindex;
+    blocks[nb++] = g->d_nlist;
   }
-  dev_free(g->bm[0]);
-  dev_free(g->pile[0]);
-  dev_free(g->pile[1]);
-  dev_free(g->ctl);
-  dev_free(g->recs);
-  dev_free(g->srcs);
-  dev_free(g->reach);
-  dev_free(g->snap_dist);
-  dev_free(g->snap_bm);
-  dev_free(g->snap_wl);
-  dev_free(g->snap_hwl);
+  if (g->owns || g->owns_weights) blocks[nb++] = g->d_eweight;
+  dev_free_all(blocks, nb);
+  g->d_inv = nullptr;
   if (g->h_ctl) ctl_host_put(g->h_ctl);
+  stage_put(g);
   if (g->ev0) cudaEventDestroy(g->ev0);
   if (g->ev1) cudaEventDestroy(g->ev1);
   if (g->ev2) cudaEventDestroy(g->ev2);
   if (g->ev3) cudaEventDestroy(g->ev3);
   if (g->stream) cudaStreamDestroy(g->stream);
-  dev_free(g->d_sp);
   if (g->twin) i2_graph_free(g->twin);
   g->twin = nullptr;
-  dev_free(g->d_inv);
-  g->d_inv = nullptr;
-  if (g->owns) {
-    dev_free(g->d_nindex);
-    dev_free(g->d_nlist);
-  }
-  if (g->owns || g->owns_weights) dev_free(g->d_eweight);
 }
 
 static int compute_stats(i2_graph* g) {
   DevStats* st = nullptr;
   I2_CK(dev_alloc(&st, sizeof(DevStats)));
-  DevStats h{};
-  h.wmin = INT_MAX;
-  cudaMemcpy(st, &h, sizeof(h), cudaMemcpyHostToDevice);
-  const int grid = 4 * sm_count();
-  k_degree_stats<<<grid, 256, 0, g->stream>>>(g->g, g->heavy, st);
-  cudaStreamSynchronize(g->stream);
-  cudaMemcpy(&h, st, sizeof(h), cudaMemcpyDeviceToHost);
-  cudaError_t e = cudaGetLastError();
+  static_assert(sizeof(DevStats) <= sizeof(Ctl), "read back through the pinned control block");
+  DevStats& h = *reinterpret_cast<DevStats*>(g->h_ctl);
+  cudaError_t e = cudaMemsetAsync(st, 0, sizeof(DevStats), g->stream);
+  if (e == cudaSuccess) {
+    k_degree_stats<<<4 * sm_count(), 256, 0, g->stream>>>(g->g, g->heavy, st);
+    e = cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, g->stream);
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
   dev_free(st);
-  if (e != cudaSuccess) return cuda_status(e);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return cuda_status(e);
+  }
   GStats& s = g->gs;
   s.nodes = g->g.nodes;
   s.edges = g->g.edges;
   s.maxdeg = (int)(h.hub >> 32);
   g->hub = (int)~(unsigned)h.hub;
   s.nheavy = h.nheavy;
-  s.wmin = g->g.eweight ? (h.wmin == INT_MAX ? 1 : h.wmin) : 1;
+  s.wmin = g->g.eweight && h.winv ? (int)((unsigned)INT_MAX - h.winv) : 1;
   s.symmetric = -1;  // decided on first need (ensure_symmetry)
   const double mean = (double)g->g.edges / (double)g->g.nodes;
   const double var = std::max(0.0, h.sumsq / (double)g->g.nodes - mean * mean);
@@ -752,28 +887,56 @@ static int finish_setup(i2_graph* g) {
 static size_t hist_offset_words(const i2_graph* g) { return (4ull * g->bm_words + 1) & ~1ull; }
 static size_t bm_block_words(const i2_graph* g) { return hist_offset_words(g) + 2ull * 2 * kHistBins; }
 
+// The three frontiers' heavy lists, one block for the six arrays.
+static int alloc_heavy(i2_graph* g) {
+  if (g->heavy_base) return I2_OK;
+  const size_t n = ((size_t)std::max(1, g->gs.nheavy) + 63) & ~(size_t)63;  // 256-byte boundaries
+  I2_CK(dev_alloc(&g->heavy_base, sizeof(int) * 6 * n));
+  for (int k = 0; k < 3; ++k) {
+    g->hwl[k] = reinterpret_cast<int*>(g->heavy_base) + (size_t)(2 * k) * n;
+    g->htoff[k] = reinterpret_cast<unsigned*>(g->heavy_base) + (size_t)(2 * k + 1) * n;
+  }
+  return I2_OK;
+}
+
 static int ensure_workspace(i2_graph* g) {
   if (g->ws_ready) return I2_OK;
   const long long V = g->g.nodes;
   g->bm_words = (int)((V + 31) / 32);
-  I2_CK(dev_alloc(&g->dist, sizeof(int) * V));
+  g->rec_cap = (int)std::min<long long>(V + 2, 1 << 16);
+  int st = alloc_heavy(g);
+  if (st) return st;
+  // one block, every array on a 256-byte boundary
+  size_t at = 0;
+  const auto take = [&](size_t bytes) {
+    const size_t o = at;
+    at += (bytes + 255) & ~(size_t)255;
+    return o;
+  };
+  const size_t o_dist = take(sizeof(int) * V);
+  size_t o_wl[3], o_off[3];
   for (int k = 0; k < 3; ++k) {
-    I2_CK(dev_alloc(&g->wl[k], sizeof(int) * V));
-    I2_CK(dev_alloc(&g->woff[k], sizeof(unsigned) * V));
-    I2_CK(dev_alloc(&g->hwl[k], sizeof(int) * std::max(1, g->gs.nheavy)));
-    I2_CK(dev_alloc(&g->htoff[k], sizeof(unsigned) * std::max(1, g->gs.nheavy)));
+    o_wl[k] = take(sizeof(int) * V);
+    o_off[k] = take(sizeof(unsigned) * V);
   }
-  // one block: the three frontier bitmaps, the far-pile bitmap and the
-  // near/far distance histograms (cleared together before every run)
-  unsigned* bm = nullptr;
-  I2_CK(dev_alloc(&bm, sizeof(unsigned) * bm_block_words(g)));
+  // the three frontier bitmaps, the far-pile bitmap and the near/far distance
+  // histograms (cleared together before every run)
+  const size_t o_bm = take(sizeof(unsigned) * bm_block_words(g));
+  const size_t o_ctl = take(sizeof(Ctl));
+  const size_t o_recs = take(sizeof(IterRec) * g->rec_cap);
+  I2_CK(dev_alloc(&g->ws_base, at));
+  const auto ptr = [&](size_t o) { return static_cast<void*>(g->ws_base + o); };
+  g->dist = static_cast<int*>(ptr(o_dist));
+  for (int k = 0; k < 3; ++k) {
+    g->wl[k] = static_cast<int*>(ptr(o_wl[k]));
+    g->woff[k] = static_cast<unsigned*>(ptr(o_off[k]));
+  }
+  unsigned* bm = static_cast<unsigned*>(ptr(o_bm));
   for (int k = 0; k < 3; ++k) g->bm[k] = bm + (size_t)k * g->bm_words;
   g->fbm = bm + 3ull * g->bm_words;
   g->hist = reinterpret_cast<unsigned long long*>(bm + hist_offset_words(g));
-  I2_CK(dev_alloc(&g->ctl, sizeof(Ctl)));
-  g->rec_cap = (int)std::min<long long>(V + 2, 1 << 16);
-  I2_CK(dev_alloc(&g->recs, sizeof(IterRec) * g->rec_cap));
-  I2_CK(dev_alloc(&g->reach, sizeof(unsigned long long) * 2));
+  g->ctl = static_cast<Ctl*>(ptr(o_ctl));
+  g->recs = static_cast<IterRec*>(ptr(o_recs));
   g->ws_ready = true;
   return I2_OK;
 }
@@ -986,9 +1149,9 @@ static int add_kernel_node(cudaGraph_t gr, cudaGraphNode_t* node, const cudaGrap
   return I2_OK;
 }
 
-static int build_exec(i2_graph* g, int algo, int mode, int variant, bool multi, bool resident, const RunParams& rp,
+static int build_exec(i2_graph* g, int algo, int mode, int variant, bool multi, const RunParams& rp,
                       ExecEntry** out) {
-  ExecKey key{algo, mode, mode == 0 ? variant : -1, multi ? 1 : 0, rp.delta != 0 ? 1 : 0, resident ? 1 : 0};
+  ExecKey key{algo, mode, mode == 0 ? variant : -1, multi ? 1 : 0, rp.delta != 0 ? 1 : 0};
   auto it = g->execs.find(key);
   if (it != g->execs.end()) {
     *out = &it->second;
@@ -1036,22 +1199,14 @@ static int build_exec(i2_graph* g, int algo, int mode, int variant, bool multi, 
   cp.conditional.size = 1;
   I2_CK(cudaGraphAddNode(&n_loop, gr, &n_seed, 1, &cp));
   cudaGraph_t body = cp.conditional.phGraph_out[0];
-  // The loop body is one kernel. Resident: a cooperative launch that runs
-  // every iteration itself (the loop then runs once). Otherwise one launch per
-  // iteration: the fixed style's kernel, or the dispatch kernel whose blocks
-  // branch on the style the previous iteration selected.
+  // The loop body is one kernel, launched once per iteration: the fixed style's,
+  // or the dispatch kernel whose blocks branch on the style the previous
+  // iteration selected.
   {
     cudaGraphNode_t n;
-    KernelFn fn = resident ? resident_kernel(algo, mode == 0 ? variant : -1, rp.delta != 0, wide_form(g, mode == 0 ? variant : -1))
-                  : mode == 0 ? relax_kernel(algo, variant, rp.delta != 0)
-                              : dispatch_kernel(algo, wide_selector(g));
+    KernelFn fn = mode == 0 ? relax_kernel(algo, variant, rp.delta != 0) : dispatch_kernel(algo, wide_selector(g));
     st = add_kernel_node(body, &n, nullptr, 0, fn, grid_for(fn, g->blocks_per_sm), &c);
     if (st) return st;
-    if (resident) {
-      cudaKernelNodeAttrValue av{};
-      av.cooperative = 1;
-      I2_CK(cudaGraphKernelNodeSetAttribute(n, cudaKernelNodeAttributeCooperative, &av));
-    }
   }
   ExecEntry e;
   I2_CK(cudaGraphInstantiate(&e.ex, gr, 0));
@@ -1079,6 +1234,43 @@ static int launch_exec(i2_graph* g, ExecEntry* e, const RunParams& rp, cudaStrea
     e->last = rp;
   }
   I2_CK(cudaGraphLaunch(e->ex, s));
+  return I2_OK;
+}
+
+typedef void (*StartFn)(Ctx, RunParams, unsigned);
+static StartFn start_kernel(int algo) {
+  if (algo == kBFS) return k_start<kBFS>;
+  if (algo == kSSSP) return k_start<kSSSP>;
+  if (algo == kCC) return k_start<kCC>;
+  return k_start<kMIS>;
+}
+
+// A resident traversal: its start (one kernel; with the frontier's own kernels
+// where many vertices are in it), and one cooperative launch that runs every
+// iteration.
+static int launch_resident(i2_graph* g, int algo, int mode, int variant, bool multi, const RunParams& rp,
+                           cudaStream_t s) {
+  Ctx c = make_ctx(g);
+  c.srcs = multi ? g->srcs : nullptr;
+  const int v = mode == 0 ? variant : -1;
+  KernelFn fn = resident_kernel(algo, v, rp.delta != 0, wide_form(g, v));
+  auto it = g->grids.find(fn);
+  if (it == g->grids.end()) it = g->grids.emplace(fn, grid_for(fn, g->blocks_per_sm)).first;
+  const unsigned words = (unsigned)bm_block_words(g);
+  const long long units = (long long)g->g.nodes / 4 + words;
+  const int start_grid = (int)std::max(1LL, std::min(8LL * sm_count(), units / (4 * kBlock)));
+  start_kernel(algo)<<<start_grid, kBlock, 0, s>>>(c, rp, words);
+  const bool frontier = algo == I2_MIS || (algo == I2_CC && !rp.uf_start);
+  if (frontier) {
+    KernelFn ff = fill_kernel(algo);
+    auto fi = g->grids.find(ff);
+    if (fi == g->grids.end()) fi = g->grids.emplace(ff, grid_for(ff, 8)).first;
+    ff<<<fi->second, kBlock, 0, s>>>(c);
+  }
+  if (frontier || multi) seed_kernel(algo)<<<1, kBlock, 0, s>>>(c);
+  I2_CK(cudaGetLastError());
+  void* args[1] = {&c};
+  I2_CK(cudaLaunchCooperativeKernel((const void*)fn, dim3(it->second), dim3(kBlock), args, 0, s));
   return I2_OK;
 }
 
@@ -1121,13 +1313,18 @@ static int run_host_loop(i2_graph* g, cudaStream_t s, int algo, bool multi, doub
   return I2_OK;
 }
 
-static int fill_report(i2_graph* g, cudaStream_t s, int algo, i2_report* rep, double host_relax_ms) {
+static int fill_report(i2_graph* g, cudaStream_t s, int algo, i2_report* rep, double host_relax_ms, int* host_out) {
+  // the counts join the control block (zeroed when the run began): one copy back
+  k_reached<<<std::min(4 * sm_count(), g->g.nodes / 1024 + 1), 256, 0, s>>>(g->g, g->dist, g->ctl->reached);
+  I2_CK(cudaGetLastError());
   I2_CK(cudaMemcpyAsync(g->h_ctl, g->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
-  I2_CK(cudaMemsetAsync(g->reach, 0, sizeof(unsigned long long) * 2, s));
-  k_reached<<<4 * sm_count(), 256, 0, s>>>(g->g, g->dist, g->reach);
-  unsigned long long r[2] = {0, 0};
-  I2_CK(cudaMemcpyAsync(r, g->reach, sizeof(r), cudaMemcpyDeviceToHost, s));
+  if (host_out && stage_get(g))
+    I2_CK(cudaMemcpyAsync(g->h_stage, g->dist, sizeof(int) * (size_t)g->g.nodes, cudaMemcpyDeviceToHost, s));
   I2_CK(cudaStreamSynchronize(s));
+  if (host_out && g->h_stage && !(g->h_ctl->status & kStatusStall)) {
+    std::memcpy(host_out, g->h_stage, sizeof(int) * (size_t)g->g.nodes);
+    g->staged = true;
+  }
   const Ctl* h = g->h_ctl;
   g->last_iters = h->iter;
   if (rep) {
@@ -1137,8 +1334,8 @@ static int fill_report(i2_graph* g, cudaStream_t s, int algo, i2_report* rep, do
     rep->relax_seconds = host_relax_ms >= 0.0 ? host_relax_ms * 1e-3 : h->relax_ns * 1e-9;
     rep->iterations = h->iter;
     for (int k = 0; k < 16; ++k) rep->variant_hist[k] = h->hist[k];
-    rep->reached_vertices = (long long)r[0];
-    rep->reached_edges = (long long)r[1];
+    rep->reached_vertices = (long long)h->reached[0];
+    rep->reached_edges = (long long)h->reached[1];
   }
   if (h->status & kStatusStall) return I2_ERR_STALL;
   if (h->status & kStatusIterCap) return I2_ERR_ITER_CAP;
@@ -1200,9 +1397,10 @@ static int run_on_twin(i2_graph* g, int algo, int src, const int* srcs_host, int
 }
 
 int run_traversal(i2_graph* g, int algo, int src, const int* srcs_host, int nsrc, const i2_opts* opts,
-                  i2_report* rep) {
+                  i2_report* rep, int* host_out) {
   if (!g) return I2_ERR_ARG;
   if (algo < I2_BFS || algo > I2_MIS) return I2_ERR_ARG;
+  g->staged = false;
   I2_CK(cudaSetDevice(g->device));
   if (g->twin && (algo == I2_BFS || algo == I2_SSSP)) return run_on_twin(g, algo, src, srcs_host, nsrc, opts, rep);
   if (g->twin && algo == I2_CC) {
@@ -1325,24 +1523,28 @@ int run_traversal(i2_graph* g, int algo, int src, const int* srcs_host, int nsrc
                                    union_find_pays(g->g.nodes, g->gs.avgdeg)));
   ExecEntry* ex = nullptr;
   const bool graph_loop = o.loop_mode == I2_LOOP_GRAPH || o.loop_mode == I2_LOOP_RELAUNCH;
-  if (graph_loop) {
-    // Resident traversal where the device takes the cooperative node; graphs
-    // with one launch per iteration otherwise.
-    const bool resident = o.loop_mode == I2_LOOP_GRAPH && g->resident_ok;
-    st = build_exec(g, algo, mode, variant, multi, resident, rp, &ex);
-    if (st && resident) {
-      cudaGetLastError();
-      g->resident_ok = false;
-      st = build_exec(g, algo, mode, variant, multi, false, rp, &ex);
-    }
+  // Resident traversal where the device takes the cooperative launch; a graph
+  // with one launch per iteration otherwise.
+  bool resident = o.loop_mode == I2_LOOP_GRAPH && g->resident_ok;
+  if (graph_loop && !resident) {
+    st = build_exec(g, algo, mode, variant, multi, rp, &ex);
     if (st) return st;
   }
   double host_relax_ms = -1.0;
   if (rep) I2_CK(cudaEventRecord(g->ev0, s));
-  if (graph_loop) {
+  if (resident) {
+    st = launch_resident(g, algo, mode, variant, multi, rp, s);
+    if (st) {  // refused: this graph's traversals relaunch from here on
+      cudaGetLastError();
+      g->resident_ok = false;
+      st = build_exec(g, algo, mode, variant, multi, rp, &ex);
+      if (st) return st;
+    }
+  }
+  if (graph_loop && (!resident || !g->resident_ok)) {
     st = launch_exec(g, ex, rp, s);
     if (st) return st;
-  } else {
+  } else if (!graph_loop) {
     st = prepare_run(g, s, rp);
     if (st) return st;
     st = run_host_loop(g, s, algo, multi, &host_relax_ms);
@@ -1352,7 +1554,7 @@ int run_traversal(i2_graph* g, int algo, int src, const int* srcs_host, int nsrc
   I2_CK(cudaGetLastError());
   // Without a report the call stays asynchronous on the stream.
   if (!rep && graph_loop) return I2_OK;
-  return fill_report(g, s, algo, rep, host_relax_ms);
+  return fill_report(g, s, algo, rep, host_relax_ms, host_out);
 }
 
 bool graph_known_symmetric(const i2_graph* g) { return g && g->gs.symmetric == 1; }
@@ -1597,15 +1799,18 @@ int i2_graph_upload(const i2_eclgraph* h, i2_graph** out) {
   i2_graph* g = new i2_graph();
   g->owns = true;
   const size_t nn = (size_t)h->nodes + 1, ne = (size_t)h->edges + 4;
-  cudaStream_t s1 = nullptr, s2 = nullptr;
+  DevPool* pool = dev_pool();
+  if (!pool) {
+    delete g;
+    return I2_ERR_CUDA;
+  }
+  cudaStream_t s1 = pool->copy[0], s2 = pool->copy[1];
   int* bad = nullptr;
   int hbad = 0;
   cudaError_t e = dev_alloc(&g->d_nindex, sizeof(int) * nn);
   if (e == cudaSuccess) e = dev_alloc(&g->d_nlist, sizeof(int) * ne);
   if (e == cudaSuccess && h->eweight) e = dev_alloc(&g->d_eweight, sizeof(int) * ne);
   if (e == cudaSuccess) e = dev_alloc(&bad, sizeof(int));
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s1, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s2, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMemsetAsync(bad, 0, sizeof(int), s1);
   if (e == cudaSuccess) e = cudaMemcpyAsync(g->d_nindex, h->nindex, sizeof(int) * nn, cudaMemcpyHostToDevice, s1);
   if (e == cudaSuccess)
@@ -1624,8 +1829,6 @@ int i2_graph_upload(const i2_eclgraph* h, i2_graph** out) {
   if (e == cudaSuccess) e = cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, s1);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s1);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s2);
-  if (s1) cudaStreamDestroy(s1);
-  if (s2) cudaStreamDestroy(s2);
   dev_free(bad);
   if (e != cudaSuccess || hbad) {
     cudaGetLastError();
@@ -1761,19 +1964,18 @@ int i2_graph_tune(i2_graph* g, int heavy_threshold, int blocks_per_sm, int smem_
   if (heavy_threshold && heavy_threshold != g->heavy) {
     g->heavy = std::max(32, heavy_threshold);
     // the heavy lists are sized by the number of heavy vertices
+    dev_free(g->heavy_base);
+    g->heavy_base = nullptr;
     for (int k = 0; k < 3; ++k) {
-      dev_free(g->hwl[k]);
-      dev_free(g->htoff[k]);
       g->hwl[k] = nullptr;
       g->htoff[k] = nullptr;
     }
     int st = compute_stats(g);
     if (st) return st;
-    if (g->ws_ready)
-      for (int k = 0; k < 3; ++k) {
-        I2_CK(dev_alloc(&g->hwl[k], sizeof(int) * std::max(1, g->gs.nheavy)));
-        I2_CK(dev_alloc(&g->htoff[k], sizeof(unsigned) * std::max(1, g->gs.nheavy)));
-      }
+    if (g->ws_ready) {
+      st = alloc_heavy(g);
+      if (st) return st;
+    }
   }
   if (g->twin) return i2_graph_tune(g->twin, heavy_threshold, blocks_per_sm, smem_carveout);
   return I2_OK;
@@ -1854,8 +2056,9 @@ int i2_trim_device_memory(void) {
 
 static int run_host_out(i2_graph* g, int algo, int src, int* out, const i2_opts* opts, i2_report* rep) {
   if (!out) return I2_ERR_ARG;
-  int st = run_traversal(g, algo, src, nullptr, 0, opts, rep);
+  int st = run_traversal(g, algo, src, nullptr, 0, opts, rep, out);
   if (st && st != I2_ERR_ITER_CAP) return st;
+  if (g->staged) return st;  // the result came with the report
   cudaStream_t s = (opts && opts->stream) ? (cudaStream_t)opts->stream : g->stream;
   I2_CK(cudaMemcpyAsync(out, g->dist, sizeof(int) * (size_t)g->g.nodes, cudaMemcpyDeviceToHost, s));
   I2_CK(cudaStreamSynchronize(s));

@@ -29,9 +29,10 @@ int mlp_install(const float* params, int count);
 
 // One traversal of a device graph from one source (srcs_host == nullptr) or
 // from nsrc sources at once (batched graphs). The result stays in the graph's
-// workspace.
+// workspace; one of a small graph may be copied to host_out (nodes ints) with
+// the report (i2_graph::staged).
 int run_traversal(i2_graph* g, int algo, int src, const int* srcs_host, int nsrc, const i2_opts* opts,
-                  i2_report* rep);
+                  i2_report* rep, int* host_out = nullptr);
 
 // True when [p, p + bytes) lies inside one allocation of the current device
 // (or managed memory); host pointers and other GPUs' memory are refused.

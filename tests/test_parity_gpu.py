@@ -457,3 +457,29 @@ def test_union_find_order_and_links_on_sparse_and_dense_graphs(gpu, n):
             np.testing.assert_array_equal(dg.cc(variant="heuristic", loop=loop)[0], ref)
         np.testing.assert_array_equal(dg.cc(variant="vp_cta", then_variant="union_find", then_at=1)[0], ref)
         dg.free()
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 7, 8, 9, 31, 33, 65, 1023])
+def test_start_kernel_from_every_place_of_a_quad(gpu, n):
+    # the values are filled four at a time and the source written among them:
+    # sources at every place, vertices without edges, host results of every
+    # length, one run after another on the same graph
+    rng = np.random.default_rng(100 + n)
+    u, v = rng.integers(0, n, 2 * n), rng.integers(0, n, 2 * n)
+    key = np.unique(np.concatenate([u * np.int64(n) + v, v * np.int64(n) + u]))
+    key = key[key // n != key % n]
+    ni = np.zeros(n + 1, np.int32)
+    np.cumsum(np.bincount(key // n, minlength=n), out=ni[1:])
+    g = i2.ECLGraph(n, len(key), ni, (key % n).astype(np.int32), np.ones(len(key), np.int32))
+    dg = i2.DeviceGraph.upload(g)
+    for s in sorted({0, n // 2, n - 1} | set(range(min(n, 9)))):
+        for variant in ("vp_cta", "heuristic", "vp_warp"):
+            d, rep = dg.bfs(s, variant=variant)
+            np.testing.assert_array_equal(d, oracle.bfs(g, s))
+            assert rep.reached_vertices == int((d != i2.INF).sum())
+            assert rep.reached_edges == int(np.diff(ni)[d != i2.INF].sum())
+            np.testing.assert_array_equal(dg.sssp(s, variant=variant)[0], oracle.sssp(g, s))
+        np.testing.assert_array_equal(dg.sssp(s, budget=8)[0], oracle.sssp(g, s))
+    for variant in ("union_find", "heuristic", "vp_cta"):
+        np.testing.assert_array_equal(dg.cc(variant=variant)[0], oracle.cc(g))
+    dg.free()
