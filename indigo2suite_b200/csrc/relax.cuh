@@ -1175,7 +1175,13 @@ __device__ __forceinline__ bool body_split(const Ctx& c, H& S, EBSharedFar& sh, 
 
 // DEFER: SSSP near/far ordering (pushes at or above the threshold go onto the
 // far pile, and split launches refill the frontier from it).
-template <int ALG, bool DEFER = false, class H>
+// LONG: tiles that lie inside one entry skip the offsets, the search and the
+// entry reads (the kernels of skewed graphs, where most edges are a hub's;
+// elsewhere the test costs 1%). us: RMAT-22 near/far 1,957 -> 1,931, RMAT-25
+// ordered 13,525 -> 13,204, CC RMAT 4 x 10^6 1,843 -> 1,741. Reading the next
+// such tile's adjacency ahead made it 6-9% slower (spills). What is left is the
+// neighbours' random value reads, one L1 or L2 sector an edge.
+template <int ALG, bool DEFER = false, bool LONG = false, class H>
 __device__ __forceinline__ bool body_edge_balanced(const Ctx& c, H& S, EBSharedT<DEFER>& sh) {
   static_assert(!DEFER || ALG == kSSSP, "near/far ordering is for SSSP");
   EpiStage& s = sh.s;
@@ -1221,50 +1227,80 @@ __device__ __forceinline__ bool body_edge_balanced(const Ctx& c, H& S, EBSharedT
   const unsigned W1 = gw < nw ? (unsigned)((total * (gw + 1)) / nw) : 0u;
   if (W0 < W1) {
     int j = owner_search_warp(woff, n, W0);  // entry holding edge W0
+    // the entry that the last tile ended in, where it fills the next tile too:
+    // its end, its vertex, and its adjacency's place relative to the edge space
+    unsigned lend = 0;
+    int lv = 0, lbase = 0;
     for (unsigned e0 = W0; e0 < W1; e0 += kWarpTile) {
       const unsigned e1 = min(W1, e0 + kWarpTile);
-      // offsets of the entries from j on, 32 at a time, until one reaches e1;
-      // each batch's vertex ids are loaded with its offsets, and the adjacency
-      // start and value of the entries inside the tile right after
-      int m = 0;
-      for (;;) {
-        const int jj = j + m + lane;
-        const bool in = jj < n;
-        const unsigned w = in ? woff[jj] : total;
-        const int v = in ? wl[jj] : 0;
-        ws.off[m + lane] = w;
-        const int below = __popc(__ballot_sync(0xffffffffu, w < e1));
-        if (lane < below) {  // offsets ascend: the entries below e1 are a prefix
-          ws.beg[m + lane] = c.g.nindex[v];
-          if (ALG != kBFS) ws.du[m + lane] = c.dist[v];
-        }
-        m += below;
-        if (below < kWarp) break;
-      }
-      __syncwarp();
-      const unsigned x0 = e0 + (unsigned)lane * kEdgesPerThread;
       int du[kEdgesPerThread], nv[kEdgesPerThread], wv[kEdgesPerThread];
       bool ok[kEdgesPerThread];
-      int o = x0 < e1 ? owner_search(ws.off, m, x0) : 0;
+      if (LONG && e1 <= lend) {  // warp-uniform
+        const int d = ALG == kBFS ? i : __ldcg(&c.dist[lv]);  // may have fallen since the last tile
+        const int b = lbase + (int)e0 + lane;
 #pragma unroll
-      for (int r = 0; r < kEdgesPerThread; ++r) {
-        const unsigned x = x0 + r;
-        ok[r] = x < e1;
-        nv[r] = 0;
-        wv[r] = 0;
-        du[r] = kInf;
-        if (ok[r]) {
-          while (x >= ws.off[o + 1]) ++o;
-          const int e = ws.beg[o] + (int)(x - ws.off[o]);
-          nv[r] = ld_adj(nl + e);
-          if (Op<ALG>::kWeighted) wv[r] = ld_adj(ew + e);
-          du[r] = ALG == kBFS ? i : ws.du[o];  // BFS: F_i is level i
-          ok[r] = Op<ALG>::valid(du[r]);
+        for (int r = 0; r < kEdgesPerThread; ++r) {
+          ok[r] = e0 + lane + r * kWarp < e1;
+          nv[r] = ok[r] ? ld_adj(nl + b + r * kWarp) : 0;
+          wv[r] = Op<ALG>::kWeighted && ok[r] ? ld_adj(ew + b + r * kWarp) : 0;
+          du[r] = d;
+        }
+#pragma unroll
+        for (int r = 0; r < kEdgesPerThread; ++r) ok[r] = ok[r] && Op<ALG>::valid(d);
+        if (e1 == lend) ++j;
+      } else {
+        // offsets of the entries from j on, 32 at a time, until one reaches e1;
+        // each batch's vertex ids are loaded with its offsets, and the adjacency
+        // start and value of the entries inside the tile right after
+        int m = 0;
+        for (;;) {
+          const int jj = j + m + lane;
+          const bool in = jj < n;
+          const unsigned w = in ? woff[jj] : total;
+          const int v = in ? wl[jj] : 0;
+          ws.off[m + lane] = w;
+          const int below = __popc(__ballot_sync(0xffffffffu, w < e1));
+          if (lane < below) {  // offsets ascend: the entries below e1 are a prefix
+            ws.beg[m + lane] = c.g.nindex[v];
+            if (ALG != kBFS) ws.du[m + lane] = c.dist[v];
+          }
+          m += below;
+          if (below < kWarp) break;
+        }
+        __syncwarp();
+        const unsigned x0 = e0 + (unsigned)lane * kEdgesPerThread;
+        int o = x0 < e1 ? owner_search(ws.off, m, x0) : 0;
+#pragma unroll
+        for (int r = 0; r < kEdgesPerThread; ++r) {
+          const unsigned x = x0 + r;
+          ok[r] = x < e1;
+          nv[r] = 0;
+          wv[r] = 0;
+          du[r] = kInf;
+          if (ok[r]) {
+            while (x >= ws.off[o + 1]) ++o;
+            const int e = ws.beg[o] + (int)(x - ws.off[o]);
+            nv[r] = ld_adj(nl + e);
+            if (Op<ALG>::kWeighted) wv[r] = ld_adj(ew + e);
+            du[r] = ALG == kBFS ? i : ws.du[o];  // BFS: F_i is level i
+            ok[r] = Op<ALG>::valid(du[r]);
+          }
+        }
+        // the next tile starts at e1: its first entry is the last one with offset <= e1
+        lend = ws.off[m];
+        if (lend == e1) {
+          j += m;
+        } else {
+          j += m - 1;
+          if (LONG && lend >= e1 + kWarpTile) {
+            lv = wl[j];
+            lbase = ws.beg[m - 1] - (int)ws.off[m - 1];
+          } else {
+            lend = 0;
+          }
         }
       }
       qn = warp_relax_batch<ALG, DEFER>(c, ws, a, nxt, du, nv, wv, ok, thr, qn);
-      // the next tile starts at e1: its first entry is the last one with offset <= e1
-      j += (ws.off[m] == e1) ? m : m - 1;
       __syncwarp();
       if (qn > kWarpQueue - kWarpTile) {  // the next tile's might not fit
         warp_resolve<ALG, DEFER>(c, ws, a, nxt, qn, thr, hs, DEFER ? S.pcur : 0);
@@ -2042,7 +2078,7 @@ __device__ __forceinline__ bool grid_wait(const Ctx& c, unsigned gen, unsigned l
   return ok;
 }
 
-template <int ALG, int VAR, bool DEFER, class H>
+template <int ALG, int VAR, bool DEFER, bool LONG, class H>
 __device__ __forceinline__ bool run_body(const Ctx& c, H& S, AnyShared<DEFER>& sh) {
   if constexpr (ALG == kMIS) {
     return body_mis(c, S, sh.st);  // one style
@@ -2051,7 +2087,7 @@ __device__ __forceinline__ bool run_body(const Ctx& c, H& S, AnyShared<DEFER>& s
     switch (v) {
       case kVPThread: return body_push<ALG, kVPThread>(c, S, sh.st);
       case kVPWarp: return body_push<ALG, kVPWarp>(c, S, sh.st);
-      case kVPCta: return body_edge_balanced<ALG, DEFER>(c, S, sh.eb);
+      case kVPCta: return body_edge_balanced<ALG, DEFER, LONG>(c, S, sh.eb);
       case kVPBlock: return body_push<ALG, kVPBlock>(c, S, sh.st);
       case kPullFrontier: return body_pull<ALG, true>(c, S, sh.st);
       case kPullTopo: return body_pull<ALG, false>(c, S, sh.st);
@@ -2074,6 +2110,7 @@ template <int ALG, int VAR, bool DEFER = false,
 __global__ void __launch_bounds__(kBlock, MINB) relax_resident(const __grid_constant__ Ctx c) {
   __shared__ AnyShared<DEFER> sh;
   __shared__ typename std::conditional<(VAR < 0), SelectHead, FixedHead>::type S;
+  constexpr bool LONG = DEFER || (VAR == kVPCta && MINB == I2_FIXED_MIN_BLOCKS);  // skewed graphs' forms
   // thread 0's: barrier generation, whether to go on, the test hook (kept in
   // shared memory: the bodies have no register to spare)
   __shared__ unsigned s_gen;
@@ -2091,7 +2128,7 @@ __global__ void __launch_bounds__(kBlock, MINB) relax_resident(const __grid_cons
     return;
   }
   for (;;) {
-    if (run_body<ALG, VAR, DEFER>(c, S, sh) && !s_hold) {
+    if (run_body<ALG, VAR, DEFER, LONG>(c, S, sh) && !s_hold) {
       // this block advanced S and wrote it back (every thread a word)
       __syncthreads();
       if (threadIdx.x == 0)

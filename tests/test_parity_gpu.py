@@ -405,7 +405,8 @@ def test_pooled_memory_reuse_and_trim(gpu):
 
 
 @pytest.mark.parametrize("mid,leaves", [(1, 63), (1, 64), (1, 65), (2, 32), (3, 43), (64, 1), (65, 3), (129, 2),
-                                        (192, 1), (193, 5), (700, 64)])
+                                        (192, 1), (193, 5), (700, 64), (1, 127), (1, 128), (1, 129), (1, 191), (1, 192),
+                                        (1, 193), (2, 499), (5, 1000), (40, 321)])
 def test_queued_vertices_around_tile_and_queue_sizes(gpu, mid, leaves):
     # source -> mid vertices -> leaves each: every edge lowers a value. The first
     # half of each vertex's leaves are shared by all (repeats in one warp's
