@@ -484,3 +484,28 @@ def test_start_kernel_from_every_place_of_a_quad(gpu, n):
     for variant in ("union_find", "heuristic", "vp_cta"):
         np.testing.assert_array_equal(dg.cc(variant=variant)[0], oracle.cc(g))
     dg.free()
+
+
+@pytest.mark.parametrize("degree", [3, 34, 35, 66, 2050, 2051, 4100, 70000])
+def test_union_find_long_lists_outside_the_largest_tree(gpu, degree):
+    # a large component without hubs (a ring with chords) takes the sample; a
+    # star whose hub comes last, with rings among its leaves, is linked by
+    # threads, warps or blocks, in both link orders
+    for chords in (0, 5):
+        big = 4 * degree + 64
+        ring = np.arange(big)
+        pairs = [(ring, (ring + 1 + k) % big) for k in range(1 + chords)]
+        leaves = big + np.arange(degree)
+        hub = np.full(degree, big + degree)
+        pairs += [(hub, leaves), (leaves[:-1:2], leaves[1::2])]
+        u = np.concatenate([p[0] for p in pairs] + [p[1] for p in pairs])
+        v = np.concatenate([p[1] for p in pairs] + [p[0] for p in pairs])
+        n = big + degree + 1
+        key = np.unique(u * np.int64(n) + v)
+        ni = np.zeros(n + 1, np.int32)
+        np.cumsum(np.bincount(key // n, minlength=n), out=ni[1:])
+        g = i2.ECLGraph(n, len(key), ni, (key % n).astype(np.int32), np.ones(len(key), np.int32))
+        dg = i2.DeviceGraph.upload(g)
+        for loop in (i2.I2_LOOP_GRAPH, i2.I2_LOOP_HOST):
+            np.testing.assert_array_equal(dg.cc(variant="union_find", loop=loop)[0], oracle.cc(g))
+        dg.free()
