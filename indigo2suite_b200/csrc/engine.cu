@@ -185,17 +185,18 @@ __global__ void k_reset(Ctl* ctl, RunParams p) {
 }
 
 // Start of a resident traversal: control block, bitmaps and values in one
-// kernel. Where no frontier of many vertices is to be built (one source, or
-// union-find from the first iteration) it seeds the frontier and selects the
-// first variant too, so that the traversal is two launches; CC, MIS and runs
-// from many sources have k_fill and k_seed after it. Five nodes of a CUDA graph
+// kernel. Where no frontier of many vertices is to be built (one source,
+// union-find from the first iteration, MIS, whose first iteration takes every
+// vertex) it seeds the frontier and selects the first variant too, so that the
+// traversal is two launches; CC by propagation has k_fill and k_seed after it,
+// runs from many sources k_seed. Five nodes of a CUDA graph
 // (memset, reset, fill, seed, conditional loop) took 16-20 us more: SSSP on RMAT
 // with 3,001 vertices 151 -> 130 us, BFS RMAT-20 138 -> 118; and instantiating
 // the graph cost a new graph's first traversal 0.25 ms.
 template <int ALG>
 __global__ void __launch_bounds__(kBlock) k_start(const __grid_constant__ Ctx c, RunParams p, unsigned words) {
   const bool single = (ALG == kBFS || ALG == kSSSP) && !c.srcs;
-  const bool whole = single || (ALG == kCC && p.uf_start);
+  const bool whole = single || ALG == kMIS || (ALG == kCC && p.uf_start);
   const int V = c.g.nodes;
   const int src = single ? p.src : -1;
   const int deg = single ? c.g.nindex[src + 1] - c.g.nindex[src] : 0;
@@ -210,12 +211,13 @@ __global__ void __launch_bounds__(kBlock) k_start(const __grid_constant__ Ctx c,
     int4* d4 = reinterpret_cast<int4*>(c.dist);
     for (unsigned q = tid; q < quads; q += stride) {
       const int v = (int)(q << 2);
-      d4[q] = ALG == kCC ? make_int4(v, v + 1, v + 2, v + 3)
+      d4[q] = ALG == kMIS  ? make_int4(kMisUndecided, kMisUndecided, kMisUndecided, kMisUndecided)
+              : ALG == kCC ? make_int4(v, v + 1, v + 2, v + 3)
                          : make_int4(v == src ? 0 : kInf, v + 1 == src ? 0 : kInf, v + 2 == src ? 0 : kInf,
                                      v + 3 == src ? 0 : kInf);
     }
     for (unsigned v = (quads << 2) + tid; v < (unsigned)V; v += stride)
-      c.dist[v] = ALG == kCC ? (int)v : (int)v == src ? 0 : kInf;
+      c.dist[v] = ALG == kMIS ? (int)kMisUndecided : ALG == kCC ? (int)v : (int)v == src ? 0 : kInf;
   }
   if (blockIdx.x != 0) return;
   __shared__ SelectHead S;
@@ -1260,7 +1262,7 @@ static int launch_resident(i2_graph* g, int algo, int mode, int variant, bool mu
   const long long units = (long long)g->g.nodes / 4 + words;
   const int start_grid = (int)std::max(1LL, std::min(8LL * sm_count(), units / (4 * kBlock)));
   start_kernel(algo)<<<start_grid, kBlock, 0, s>>>(c, rp, words);
-  const bool frontier = algo == I2_MIS || (algo == I2_CC && !rp.uf_start);
+  const bool frontier = algo == I2_CC && !rp.uf_start;
   if (frontier) {
     KernelFn ff = fill_kernel(algo);
     auto fi = g->grids.find(ff);
@@ -1526,6 +1528,12 @@ int run_traversal(i2_graph* g, int algo, int src, const int* srcs_host, int nsrc
   // Resident traversal where the device takes the cooperative launch; a graph
   // with one launch per iteration otherwise.
   bool resident = o.loop_mode == I2_LOOP_GRAPH && g->resident_ok;
+  // a stream under capture gets the graph, whose launch it refuses
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (resident && (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)) {
+    cudaGetLastError();
+    resident = false;
+  }
   if (graph_loop && !resident) {
     st = build_exec(g, algo, mode, variant, multi, rp, &ex);
     if (st) return st;

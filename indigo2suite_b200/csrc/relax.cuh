@@ -1757,9 +1757,13 @@ __device__ __forceinline__ bool body_union(const Ctx& c, H& S, Stage& s) {
 // its second entry (a random neighbour outranks v half the time), so the work
 // is far below the graph's edges: random status reads bound it. One thread
 // scans the first kMisProbe entries, a warp goes on, and lists of
-// kMisBlockDegree entries or more take the whole block. (A warp per vertex
-// rescanning the list in every iteration left a hub to one warp: RMAT 2^20 took
-// 2,642 us, 2,122 of them in the first iteration; now 482 and 186.)
+// kMisBlockDegree entries or more take the whole block after the warps are done.
+// The first iteration takes every vertex without a list (building one was 60 of
+// 195 us on RMAT 3 x 10^5), and each warp stages its own waiting vertices. RMAT
+// with 1,000,003 vertices 2,625-3,129 -> 468-560 us, ER 10^6 796 -> 175, grid
+// 10^6 699 -> 119; the form before, a warp per vertex that rescanned the list in
+// every iteration, left a hub to one warp (2,122 us of its first iteration).
+enum { kMisNone, kMisWait, kMisJoin, kMisLeave, kMisMore };  // what an iteration finds for a vertex
 constexpr int kMisProbe = 16;          // entries a thread scans (or writes) by itself
 constexpr int kMisBlockDegree = 2048;  // entries from which the whole block does
 
@@ -1786,26 +1790,21 @@ __device__ __forceinline__ bool mis_probe(const Ctx& c, int v, int pv, const int
   return in;
 }
 
-// Publish the staged waiting vertices (block-uniform call): s.q the vertices,
-// s.qd their cursors, s.m their entries still to scan.
-__device__ __forceinline__ void mis_flush(const Ctx& c, Stage& s, int nxt) {
-  __syncthreads();
-  const int n = s.n;
-  if (n == 0) return;
-  if (threadIdx.x == 0)
-    s.base = atomicAdd(&c.ctl->slot[nxt].packed, ((unsigned long long)n << 32) | (unsigned)s.m);
-  __syncthreads();
-  const int b = (int)(s.base >> 32);
-  for (int j = threadIdx.x; j < n; j += kBlock) {
-    c.wl[nxt][b + j] = s.q[j];
-    c.woff[nxt][b + j] = (unsigned)s.qd[j];
+// Publish a warp's n staged waiting vertices (warp-uniform call): q the
+// vertices, cur their cursors, `left` the lane's share of their entries still
+// to scan.
+__device__ __forceinline__ void mis_flush(const Ctx& c, const int* q, const int* cur, int n, int left, int nxt) {
+  __syncwarp();
+  const int lane = threadIdx.x & 31;
+  left = __reduce_add_sync(0xffffffffu, left);
+  unsigned long long base = 0;
+  if (lane == 0) base = atomicAdd(&c.ctl->slot[nxt].packed, ((unsigned long long)n << 32) | (unsigned)left);
+  const int b = slot_size(__shfl_sync(0xffffffffu, base, 0));
+  for (int j = lane; j < n; j += kWarp) {
+    c.wl[nxt][b + j] = q[j];
+    c.woff[nxt][b + j] = (unsigned)cur[j];
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    s.n = 0;
-    s.m = 0;
-  }
-  __syncthreads();
+  __syncwarp();
 }
 
 template <class H>
@@ -1817,55 +1816,61 @@ __device__ __forceinline__ bool body_mis(const Ctx& c, H& S, Stage& s) {
   const int active = (int)min((long long)gridDim.x, ((long long)n + kBlock - 1) / kBlock);
   if (blockIdx.x >= active) return idle_epilogue(c, S, s, i, cur, nxt, old);
   stage_init(s);
-  if (threadIdx.x == 0) s.m = 0;
   Acc a;
   acc_init(a);
   __syncthreads();
   const int* wl = c.wl[cur];
+  // the first iteration's frontier may be every vertex, without a list (a
+  // vertex without neighbours joins the set at once)
+  const bool all = i == 0 && n == c.g.nodes;
   const unsigned* cursor = c.woff[cur];
   volatile int* st = c.dist;
   const int* __restrict__ nl = c.g.nlist;
   const int lane = threadIdx.x & 31;
+  // each warp stages its waiting vertices; no warp waits for another
+  constexpr int kStage = kQueue / kWarpsPerBlock;
+  int* const wq = s.q + (threadIdx.x >> 5) * kStage;
+  int* const wcur = s.qd + (threadIdx.x >> 5) * kStage;
+  int qn = 0, qleft = 0;
   for (long long base = (long long)blockIdx.x * kBlock; base < n; base += (long long)active * kBlock) {
     const long long idx = base + threadIdx.x;
-    enum { kNone, kWait, kIn, kOut, kMore };
-    int state = kNone, v = 0, pv = 0, k = 0, end = 0;
+    int state = kMisNone, v = 0, pv = 0, k = 0, end = 0;
     if (idx < n) {
-      v = wl[idx];
-      state = kMore;
+      v = all ? (int)idx : wl[idx];
+      state = kMisMore;
       if (st[v] != kMisUndecided) {  // a neighbour joined the set meanwhile
-        state = kNone;
+        state = kMisNone;
         a.visited++;
       } else {
         k = i == 0 ? c.g.nindex[v] : (int)cursor[idx];
         end = c.g.nindex[v + 1];
         pv = mis_priority(v);
-        for (int t = 0; t < kMisProbe && state == kMore; t += 4) {
+        for (int t = 0; t < kMisProbe && state == kMisMore; t += 4) {
           const int cnt = min(4, end - k);
           const int ks[4] = {k, k + 1, k + 2, k + 3};
           unsigned w = 0;
           if (cnt <= 0) {
-            state = kIn;
+            state = kMisJoin;
           } else if (mis_probe(c, v, pv, ks, cnt, &w)) {
-            state = kOut;
+            state = kMisLeave;
           } else if (w) {
             k += __ffs(w) - 1;
-            state = kWait;
+            state = kMisWait;
           } else {
             k += cnt;
           }
         }
-        if (state == kMore && k >= end) state = kIn;
+        if (state == kMisMore && k >= end) state = kMisJoin;
       }
     }
     // longer lists: the block's (deferred to after the pass), else the warp's
-    bool mine = state == kMore;
+    bool mine = state == kMisMore;
     if (mine && end - k >= kMisBlockDegree) {
       const int p = atomicAdd(&s.hn, 1);
       if (p < kHQueue) {
         s.hq[p] = v;
         s.ht[p] = k;
-        state = kNone;
+        state = kMisNone;
         mine = false;
       }
     }
@@ -1873,7 +1878,7 @@ __device__ __forceinline__ bool body_mis(const Ctx& c, H& S, Stage& s) {
       const int l = __ffs(todo) - 1;
       const int wv = __shfl_sync(0xffffffffu, v, l), wpv = __shfl_sync(0xffffffffu, pv, l);
       const int we = __shfl_sync(0xffffffffu, end, l);
-      int wk = __shfl_sync(0xffffffffu, k, l), out = kIn;
+      int wk = __shfl_sync(0xffffffffu, k, l), out = kMisJoin;
       for (; wk < we; wk += 4 * kWarp) {
         int ks[4];
 #pragma unroll
@@ -1882,13 +1887,13 @@ __device__ __forceinline__ bool body_mis(const Ctx& c, H& S, Stage& s) {
         unsigned w = 0;
         const bool in = mis_probe(c, wv, wpv, ks, cnt, &w);
         if (__any_sync(0xffffffffu, in)) {
-          out = kOut;
+          out = kMisLeave;
           break;
         }
         const int first = __reduce_min_sync(0xffffffffu, w ? (__ffs(w) - 1) * kWarp + lane : INT_MAX);
         if (first != INT_MAX) {
           wk += first;
-          out = kWait;
+          out = kMisWait;
           break;
         }
       }
@@ -1897,13 +1902,13 @@ __device__ __forceinline__ bool body_mis(const Ctx& c, H& S, Stage& s) {
         k = wk;
       }
     }
-    if (state == kOut) {
+    if (state == kMisLeave) {
       st[v] = kMisOut;
       a.visited++;
     }
     // joined: neighbours are out
     bool wide = false;
-    if (state == kIn) {
+    if (state == kMisJoin) {
       st[v] = kMisIn;
       a.visited++;
       const int b = c.g.nindex[v];
@@ -1926,79 +1931,73 @@ __device__ __forceinline__ bool body_mis(const Ctx& c, H& S, Stage& s) {
         if (u != wv) st[u] = kMisOut;
       }
     }
-    // waiting vertices into the block's queue
-    const unsigned waiting = __ballot_sync(0xffffffffu, state == kWait);
-    if (waiting) {
-      const int left = __reduce_add_sync(0xffffffffu, state == kWait ? end - k : 0);
-      int p = 0;
-      if (lane == 0) {
-        p = atomicAdd(&s.n, __popc(waiting));
-        atomicAdd(&s.m, left);
-      }
-      p = __shfl_sync(0xffffffffu, p, 0) + __popc(waiting & ((1u << lane) - 1u));
-      if (state == kWait) {
-        s.q[p] = v;
-        s.qd[p] = k;
-      }
+    // waiting vertices into the warp's queue
+    const unsigned waiting = __ballot_sync(0xffffffffu, state == kMisWait);
+    if (state == kMisWait) {
+      const int p = qn + __popc(waiting & ((1u << lane) - 1u));
+      wq[p] = v;
+      wcur[p] = k;
+      qleft += end - k;
     }
-    __syncthreads();
-    // lists for the whole block
-    const int nb = min(s.hn, kHQueue);
-    for (int x = 0; x < nb; ++x) {
-      const int bv = s.hq[x], be = c.g.nindex[bv + 1], bpv = mis_priority(bv);
-      int bk = s.ht[x], out = kIn;
-      for (; bk < be; bk += 4 * kBlock) {
-        if (threadIdx.x == 0) {
-          s.j0 = INT_MAX;
-          s.chunk = 0;
-        }
-        __syncthreads();
-        int ks[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) ks[r] = bk + r * kBlock + threadIdx.x;
-        const int t = threadIdx.x;
-        const int cnt = be - bk > t ? min(4, (be - bk - t + kBlock - 1) / kBlock) : 0;
-        unsigned w = 0;
-        if (mis_probe(c, bv, bpv, ks, cnt, &w)) s.chunk = 1;
-        if (w) atomicMin(&s.j0, (__ffs(w) - 1) * kBlock + t);
-        __syncthreads();
-        const int found = s.chunk, first = s.j0;
-        __syncthreads();  // read before the next step resets them
-        if (found) {
-          out = kOut;
-          break;
-        }
-        if (first != INT_MAX) {
-          bk += first;
-          out = kWait;
-          break;
-        }
-      }
-      if (out == kIn) {
-        for (int j = c.g.nindex[bv] + (int)threadIdx.x; j < be; j += kBlock) {
-          const int u = ld_adj(nl + j);
-          if (u != bv) st[u] = kMisOut;
-        }
-      }
-      if (threadIdx.x == 0) {
-        if (out == kWait) {
-          s.q[s.n] = bv;
-          s.qd[s.n] = bk;
-          s.n += 1;
-          s.m += be - bk;
-        } else {
-          st[bv] = out == kIn ? kMisIn : kMisOut;
-          a.visited++;
-        }
-      }
+    qn += __popc(waiting);
+    if (qn > kStage - kWarp) {
+      mis_flush(c, wq, wcur, qn, qleft, nxt);
+      qn = 0;
+      qleft = 0;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) s.hn = 0;
-    // a pass adds at most kBlock entries
-    if (s.n > kQueue - kBlock) mis_flush(c, s, nxt);
-    __syncthreads();
   }
-  mis_flush(c, s, nxt);
+  if (qn) mis_flush(c, wq, wcur, qn, qleft, nxt);
+  __syncthreads();
+  // the lists for the whole block
+  const int nb = min(s.hn, kHQueue);
+  for (int x = 0; x < nb; ++x) {
+    const int bv = s.hq[x], be = c.g.nindex[bv + 1], bpv = mis_priority(bv);
+    int bk = s.ht[x], out = kMisJoin;
+    for (; bk < be; bk += 4 * kBlock) {
+      if (threadIdx.x == 0) {
+        s.j0 = INT_MAX;
+        s.chunk = 0;
+      }
+      __syncthreads();
+      int ks[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) ks[r] = bk + r * kBlock + threadIdx.x;
+      const int t = threadIdx.x;
+      const int cnt = be - bk > t ? min(4, (be - bk - t + kBlock - 1) / kBlock) : 0;
+      unsigned w = 0;
+      if (mis_probe(c, bv, bpv, ks, cnt, &w)) s.chunk = 1;
+      if (w) atomicMin(&s.j0, (__ffs(w) - 1) * kBlock + t);
+      __syncthreads();
+      const int found = s.chunk, first = s.j0;
+      __syncthreads();  // read before the next step resets them
+      if (found) {
+        out = kMisLeave;
+        break;
+      }
+      if (first != INT_MAX) {
+        bk += first;
+        out = kMisWait;
+        break;
+      }
+    }
+    if (out == kMisJoin) {
+      for (int j = c.g.nindex[bv] + (int)threadIdx.x; j < be; j += kBlock) {
+        const int u = ld_adj(nl + j);
+        if (u != bv) st[u] = kMisOut;
+      }
+    }
+    if (threadIdx.x == 0) {
+      if (out == kMisWait) {
+        const unsigned long long p =
+            atomicAdd(&c.ctl->slot[nxt].packed, (1ull << 32) | (unsigned)(be - bk));
+        c.wl[nxt][slot_size(p)] = bv;
+        c.woff[nxt][slot_size(p)] = (unsigned)bk;
+      } else {
+        st[bv] = out == kMisJoin ? kMisIn : kMisOut;
+        a.visited++;
+      }
+    }
+  }
   __syncthreads();
   return block_epilogue(c, S, s, a, i, cur, nxt, old);
 }
