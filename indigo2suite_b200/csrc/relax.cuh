@@ -2089,7 +2089,7 @@ union AnyShared {
 // releases the others. Every wait is bounded by Ctl::stall_ns: a block that
 // waits longer sets kStatusStall and leaves, and every other block leaves at
 // its next wait, so the launch always ends. All blocks must be resident at
-// once, which the cooperative launch attribute of the graph node guarantees.
+// once, which the cooperative launch guarantees.
 // Data written in one iteration is read by other blocks in the next, so the
 // bodies read the frontier lists, bitmaps and values with coherent loads only
 // (the read-only path is used for the graph arrays alone).
@@ -2162,7 +2162,11 @@ __global__ void __launch_bounds__(kBlock, MINB) relax_resident(const __grid_cons
     s_hold = c.ctl->hold;
   }
   __syncthreads();
-  if (!s_ok) {  // an earlier launch of this traversal gave up: end the graph's loop
+  // Blocks of this traversal have given up already: end the loop of a graph it
+  // may run in. (Measured: without this branch the compiler hoists into the
+  // bodies' registers, 100 instead of 60 bytes of spills in the near/far form,
+  // RMAT-22 2,047 instead of 1,933 us.)
+  if (!s_ok) {
     if (blockIdx.x == 0 && threadIdx.x == 0 && c.use_loop)
       cudaGraphSetConditional((cudaGraphConditionalHandle)c.loop_h, 0u);
     return;
