@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(kBlock) k_fill(Ctx c) {
   }
   for (long long base = (long long)blockIdx.x * kBlock; base < V; base += (long long)gridDim.x * kBlock) {
     const int v = (int)base + threadIdx.x;
-    const bool in = v < V;
+    const bool in = base + threadIdx.x < V;
     constexpr bool kAll = ALG == kCC || ALG == kMIS;  // every vertex starts in F_0
     const int deg = (kAll && in) ? c.g.nindex[v + 1] - c.g.nindex[v] : 0;
     // MIS: a vertex without neighbours is in the set at once

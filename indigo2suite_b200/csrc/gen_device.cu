@@ -20,6 +20,7 @@
 #include <cub/device/device_select.cuh>
 #include "engine.h"
 #include "gen_rng.h"
+#include "list_walk.h"
 
 namespace i2 {
 
@@ -525,16 +526,15 @@ namespace i2 {
 namespace {
 
 __global__ void k_degree_ids(const int* __restrict__ nindex, int n, int* __restrict__ deg, int* __restrict__ ids) {
-  const int stride = gridDim.x * blockDim.x;
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
+  walk_list(0, n, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, [&](unsigned v) {
     deg[v] = nindex[v + 1] - nindex[v];
-    ids[v] = v;
-  }
+    ids[v] = (int)v;
+  });
 }
 
 __global__ void k_invert(const int* __restrict__ perm, int n, int* __restrict__ inv) {
-  const int stride = gridDim.x * blockDim.x;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) inv[perm[i]] = i;
+  walk_list(0, n, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x,
+            [&](unsigned i) { inv[perm[i]] = (int)i; });
 }
 
 // One warp per vertex (grid-stride): every CSR entry e of old vertex u becomes
@@ -547,12 +547,11 @@ __global__ void k_relabel_keys(const int* __restrict__ nindex, const int* __rest
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
   for (long long u = warp; u < n; u += nwarps) {
     const int iu = inv[u];
-    const int beg = nindex[u], end = nindex[u + 1];
-    for (int e = beg + lane; e < end; e += 32) {
+    walk_list(nindex[u], nindex[u + 1], lane, 32, [&](unsigned e) {
       const int v = nlist[e];  // in range in every graph handle; dropped if not
       keys[e] = (unsigned)v < (unsigned)n ? kb.key(iu, inv[v]) : kb.drop;
       if (w) wk[e] = w[e];
-    }
+    });
   }
 }
 

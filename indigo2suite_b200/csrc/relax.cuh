@@ -30,6 +30,7 @@
 #include <cub/block/block_scan.cuh>
 #include <type_traits>
 #include "common.cuh"
+#include "list_walk.h"
 
 namespace i2 {
 
@@ -127,7 +128,7 @@ __device__ __forceinline__ void stage_init(Stage& s) {
   }
 }
 
-__device__ __forceinline__ int heavy_tiles(int deg) { return (deg + kHeavyTile - 1) / kHeavyTile; }
+__device__ __forceinline__ int heavy_tiles(int deg) { return (int)(((unsigned)deg + kHeavyTile - 1) / kHeavyTile); }
 
 // Block-wide reduction of the per-thread statistics into s.red[0] (thread 0).
 // S is any shared struct with `Acc red[kBlock / kWarp]` and `int last`.
@@ -520,7 +521,7 @@ __device__ void heavy_path(const Ctx& c, const CtlHead& S, Stage& s, Acc& a, int
     const int beg = c.g.nindex[u];
     const int end = c.g.nindex[u + 1];
     const int lo = beg + (int)(t - toff[j]) * kHeavyTile;
-    const int hi = min(end, lo + kHeavyTile);
+    const int hi = end - lo > kHeavyTile ? lo + kHeavyTile : end;  // lo + kHeavyTile may pass INT_MAX
     if (Op<ALG>::valid(du)) relax_range<ALG>(c, s, a, nxt, du, lo, hi, threadIdx.x, blockDim.x);
     stage_flush_if_half(c, s, nxt);
   }
@@ -1237,12 +1238,12 @@ __device__ __forceinline__ bool body_edge_balanced(const Ctx& c, H& S, EBSharedT
       bool ok[kEdgesPerThread];
       if (LONG && e1 <= lend) {  // warp-uniform
         const int d = ALG == kBFS ? i : __ldcg(&c.dist[lv]);  // may have fallen since the last tile
-        const int b = lbase + (int)e0 + lane;
+        const unsigned b = (unsigned)lbase + e0 + (unsigned)lane;
 #pragma unroll
         for (int r = 0; r < kEdgesPerThread; ++r) {
           ok[r] = e0 + lane + r * kWarp < e1;
-          nv[r] = ok[r] ? ld_adj(nl + b + r * kWarp) : 0;
-          wv[r] = Op<ALG>::kWeighted && ok[r] ? ld_adj(ew + b + r * kWarp) : 0;
+          nv[r] = ok[r] ? ld_adj(nl + (b + r * kWarp)) : 0;
+          wv[r] = Op<ALG>::kWeighted && ok[r] ? ld_adj(ew + (b + r * kWarp)) : 0;
           du[r] = d;
         }
 #pragma unroll
@@ -1332,7 +1333,7 @@ __device__ __forceinline__ bool body_push_topo(const Ctx& c, H& S, Stage& s) {
   const int V = c.g.nodes;
   for (long long base = (long long)blockIdx.x * kBlock; base < V; base += (long long)gridDim.x * kBlock) {
     const int v = (int)base + threadIdx.x;
-    if (v < V && ((bmc[v >> 5] >> (v & 31)) & 1u)) {
+    if (base + threadIdx.x < V && ((bmc[v >> 5] >> (v & 31)) & 1u)) {
       const int beg = c.g.nindex[v];
       const int end = c.g.nindex[v + 1];
       const int du = c.dist[v];
@@ -1431,7 +1432,7 @@ __device__ __forceinline__ bool body_pull(const Ctx& c, H& S, Stage& s) {
     const int v = (int)base + threadIdx.x;
     bool improved = false;
     int best = kInf, dv = kInf, deg = 0;
-    if (v < V) {
+    if (base + threadIdx.x < V) {
       dv = c.dist[v];
       best = dv;
       if (!FRONTIER || dv > bound) {
@@ -1673,10 +1674,10 @@ __device__ __forceinline__ bool body_union(const Ctx& c, H& S, Stage& s) {
     const bool in = v < (unsigned)V;
     if (phase == 0) {
       if (!in) continue;
-      const int b = ni[v], e = ni[v + 1];
+      const unsigned b = ni[v], e = ni[v + 1];
       int u[kAfforestLinks], pu[kAfforestLinks];
 #pragma unroll
-      for (int r = 0; r < kAfforestLinks; ++r) u[r] = b + r < e ? ld_adj(nl + b + r) : (int)v;
+      for (int r = 0; r < kAfforestLinks; ++r) u[r] = b + r < e ? ld_adj(nl + (b + r)) : (int)v;
       int pv = p[v];
 #pragma unroll
       for (int r = 0; r < kAfforestLinks; ++r) pu[r] = climb ? p[u[r]] : 0;
@@ -1686,9 +1687,9 @@ __device__ __forceinline__ bool body_union(const Ctx& c, H& S, Stage& s) {
         else if (u[r] != (int)v) uf_union(p, (int)v, u[r]);
       }
     } else if (phase == 1) {
-      int b = 0, e = 0;
+      unsigned b = 0, e = 0;
       if (in) {
-        b = ni[v] + kAfforestLinks;
+        b = (unsigned)ni[v] + kAfforestLinks;
         e = ni[v + 1];
       }
       if (b < e) {
@@ -1700,7 +1701,7 @@ __device__ __forceinline__ bool body_union(const Ctx& c, H& S, Stage& s) {
         }
       }
       // short lists by their thread, longer ones by the warp, the hubs' by the block
-      int left = e - b;
+      int left = b < e ? (int)(e - b) : 0;
       if (left > kUfBlockDegree) {
         const int q = atomicAdd(&s.hn, 1);
         if (q < kHQueue) {
@@ -1709,14 +1710,14 @@ __device__ __forceinline__ bool body_union(const Ctx& c, H& S, Stage& s) {
         }
       }
       if (left > 0 && left <= kWarp) {
-        for (int j = b; j < e; ++j) uf_edge(p, (int)v, ld_adj(nl + j), climb);
+        walk_list(b, e, 0, 1, [&](unsigned j) { uf_edge(p, (int)v, ld_adj(nl + j), climb); });
         left = 0;
       }
       for (unsigned todo = __ballot_sync(0xffffffffu, left > 0); todo; todo &= todo - 1) {
         const int l = __ffs(todo) - 1;
-        const int wv = __shfl_sync(0xffffffffu, (int)v, l), we = __shfl_sync(0xffffffffu, e, l);
-        for (int j = __shfl_sync(0xffffffffu, b, l) + lane; j < we; j += kWarp)
-          uf_edge(p, wv, ld_adj(nl + j), climb);
+        const int wv = __shfl_sync(0xffffffffu, (int)v, l);
+        const unsigned wb = __shfl_sync(0xffffffffu, b, l), we = __shfl_sync(0xffffffffu, e, l);
+        walk_list(wb, we, lane, kWarp, [&](unsigned j) { uf_edge(p, wv, ld_adj(nl + j), climb); });
       }
     } else if (in) {
       // compress: read-only finds (a shortening write could replace a finished
@@ -1732,9 +1733,9 @@ __device__ __forceinline__ bool body_union(const Ctx& c, H& S, Stage& s) {
     __syncthreads();
     const int nh = min(s.hn, kHQueue);
     for (int q = 0; q < nh; ++q) {
-      const int hv = s.hq[q], he = ni[hv + 1];
-      for (int j = ni[hv] + kAfforestLinks + (int)threadIdx.x; j < he; j += kBlock)
-        uf_edge(p, hv, ld_adj(nl + j), climb);
+      const int hv = s.hq[q];
+      walk_list((unsigned)ni[hv] + kAfforestLinks, ni[hv + 1], threadIdx.x, kBlock,
+                [&](unsigned j) { uf_edge(p, hv, ld_adj(nl + j), climb); });
     }
   }
   return block_epilogue(c, S, s, a, i, cur, nxt, old);
@@ -1770,7 +1771,7 @@ constexpr int kMisBlockDegree = 2048;  // entries from which the whole block doe
 // Outcome of `count` (<= 4) consecutive entries from k on, loaded together:
 // bit r of *wait: entry r outranks v and is undecided; returns whether one
 // that outranks v is in the set.
-__device__ __forceinline__ bool mis_probe(const Ctx& c, int v, int pv, const int* k, int count, unsigned* wait) {
+__device__ __forceinline__ bool mis_probe(const Ctx& c, int v, int pv, const unsigned* k, int count, unsigned* wait) {
   volatile int* st = c.dist;
   const int* __restrict__ nl = c.g.nlist;
   int u[4], su[4];
@@ -1834,7 +1835,8 @@ __device__ __forceinline__ bool body_mis(const Ctx& c, H& S, Stage& s) {
   int qn = 0, qleft = 0;
   for (long long base = (long long)blockIdx.x * kBlock; base < n; base += (long long)active * kBlock) {
     const long long idx = base + threadIdx.x;
-    int state = kMisNone, v = 0, pv = 0, k = 0, end = 0;
+    int state = kMisNone, v = 0, pv = 0;
+    unsigned k = 0, end = 0;
     if (idx < n) {
       v = all ? (int)idx : wl[idx];
       state = kMisMore;
@@ -1842,12 +1844,12 @@ __device__ __forceinline__ bool body_mis(const Ctx& c, H& S, Stage& s) {
         state = kMisNone;
         a.visited++;
       } else {
-        k = i == 0 ? c.g.nindex[v] : (int)cursor[idx];
+        k = i == 0 ? (unsigned)c.g.nindex[v] : cursor[idx];
         end = c.g.nindex[v + 1];
         pv = mis_priority(v);
         for (int t = 0; t < kMisProbe && state == kMisMore; t += 4) {
-          const int cnt = min(4, end - k);
-          const int ks[4] = {k, k + 1, k + 2, k + 3};
+          const int cnt = min(4, (int)(end - k));
+          const unsigned ks[4] = {k, k + 1, k + 2, k + 3};
           unsigned w = 0;
           if (cnt <= 0) {
             state = kMisJoin;
@@ -1865,11 +1867,11 @@ __device__ __forceinline__ bool body_mis(const Ctx& c, H& S, Stage& s) {
     }
     // longer lists: the block's (deferred to after the pass), else the warp's
     bool mine = state == kMisMore;
-    if (mine && end - k >= kMisBlockDegree) {
+    if (mine && (int)(end - k) >= kMisBlockDegree) {
       const int p = atomicAdd(&s.hn, 1);
       if (p < kHQueue) {
         s.hq[p] = v;
-        s.ht[p] = k;
+        s.ht[p] = (int)k;
         state = kMisNone;
         mine = false;
       }
@@ -1877,13 +1879,14 @@ __device__ __forceinline__ bool body_mis(const Ctx& c, H& S, Stage& s) {
     for (unsigned todo = __ballot_sync(0xffffffffu, mine); todo; todo &= todo - 1) {
       const int l = __ffs(todo) - 1;
       const int wv = __shfl_sync(0xffffffffu, v, l), wpv = __shfl_sync(0xffffffffu, pv, l);
-      const int we = __shfl_sync(0xffffffffu, end, l);
-      int wk = __shfl_sync(0xffffffffu, k, l), out = kMisJoin;
+      const unsigned we = __shfl_sync(0xffffffffu, end, l);
+      unsigned wk = __shfl_sync(0xffffffffu, k, l);
+      int out = kMisJoin;
       for (; wk < we; wk += 4 * kWarp) {
-        int ks[4];
+        unsigned ks[4];
 #pragma unroll
         for (int r = 0; r < 4; ++r) ks[r] = wk + r * kWarp + lane;
-        const int cnt = we - wk > lane ? min(4, (we - wk - lane + kWarp - 1) / kWarp) : 0;
+        const int cnt = window_share(wk, we, lane, kWarp);
         unsigned w = 0;
         const bool in = mis_probe(c, wv, wpv, ks, cnt, &w);
         if (__any_sync(0xffffffffu, in)) {
@@ -1911,12 +1914,12 @@ __device__ __forceinline__ bool body_mis(const Ctx& c, H& S, Stage& s) {
     if (state == kMisJoin) {
       st[v] = kMisIn;
       a.visited++;
-      const int b = c.g.nindex[v];
+      const unsigned b = c.g.nindex[v];
       if (end - b <= kMisProbe) {
-        for (int j = b; j < end; ++j) {
+        walk_list(b, end, 0, 1, [&](unsigned j) {
           const int u = ld_adj(nl + j);
           if (u != v) st[u] = kMisOut;
-        }
+        });
       } else {
         k = b;
         wide = true;
@@ -1924,20 +1927,20 @@ __device__ __forceinline__ bool body_mis(const Ctx& c, H& S, Stage& s) {
     }
     for (unsigned todo = __ballot_sync(0xffffffffu, wide); todo; todo &= todo - 1) {
       const int l = __ffs(todo) - 1;
-      const int wv = __shfl_sync(0xffffffffu, v, l), we = __shfl_sync(0xffffffffu, end, l);
-#pragma unroll 4
-      for (int j = __shfl_sync(0xffffffffu, k, l) + lane; j < we; j += kWarp) {
+      const int wv = __shfl_sync(0xffffffffu, v, l);
+      const unsigned wb = __shfl_sync(0xffffffffu, k, l), we = __shfl_sync(0xffffffffu, end, l);
+      walk_list(wb, we, lane, kWarp, [&](unsigned j) {
         const int u = ld_adj(nl + j);
         if (u != wv) st[u] = kMisOut;
-      }
+      });
     }
     // waiting vertices into the warp's queue
     const unsigned waiting = __ballot_sync(0xffffffffu, state == kMisWait);
     if (state == kMisWait) {
       const int p = qn + __popc(waiting & ((1u << lane) - 1u));
       wq[p] = v;
-      wcur[p] = k;
-      qleft += end - k;
+      wcur[p] = (int)k;
+      qleft += (int)(end - k);
     }
     qn += __popc(waiting);
     if (qn > kStage - kWarp) {
@@ -1951,19 +1954,21 @@ __device__ __forceinline__ bool body_mis(const Ctx& c, H& S, Stage& s) {
   // the lists for the whole block
   const int nb = min(s.hn, kHQueue);
   for (int x = 0; x < nb; ++x) {
-    const int bv = s.hq[x], be = c.g.nindex[bv + 1], bpv = mis_priority(bv);
-    int bk = s.ht[x], out = kMisJoin;
+    const int bv = s.hq[x], bpv = mis_priority(bv);
+    const unsigned be = c.g.nindex[bv + 1];
+    unsigned bk = s.ht[x];
+    int out = kMisJoin;
     for (; bk < be; bk += 4 * kBlock) {
       if (threadIdx.x == 0) {
         s.j0 = INT_MAX;
         s.chunk = 0;
       }
       __syncthreads();
-      int ks[4];
+      unsigned ks[4];
 #pragma unroll
       for (int r = 0; r < 4; ++r) ks[r] = bk + r * kBlock + threadIdx.x;
       const int t = threadIdx.x;
-      const int cnt = be - bk > t ? min(4, (be - bk - t + kBlock - 1) / kBlock) : 0;
+      const int cnt = window_share(bk, be, t, kBlock);
       unsigned w = 0;
       if (mis_probe(c, bv, bpv, ks, cnt, &w)) s.chunk = 1;
       if (w) atomicMin(&s.j0, (__ffs(w) - 1) * kBlock + t);
@@ -1981,17 +1986,17 @@ __device__ __forceinline__ bool body_mis(const Ctx& c, H& S, Stage& s) {
       }
     }
     if (out == kMisJoin) {
-      for (int j = c.g.nindex[bv] + (int)threadIdx.x; j < be; j += kBlock) {
+      walk_list(c.g.nindex[bv], be, threadIdx.x, kBlock, [&](unsigned j) {
         const int u = ld_adj(nl + j);
         if (u != bv) st[u] = kMisOut;
-      }
+      });
     }
     if (threadIdx.x == 0) {
       if (out == kMisWait) {
         const unsigned long long p =
-            atomicAdd(&c.ctl->slot[nxt].packed, (1ull << 32) | (unsigned)(be - bk));
+            atomicAdd(&c.ctl->slot[nxt].packed, (1ull << 32) | (be - bk));
         c.wl[nxt][slot_size(p)] = bv;
-        c.woff[nxt][slot_size(p)] = (unsigned)bk;
+        c.woff[nxt][slot_size(p)] = bk;
       } else {
         st[bv] = out == kMisJoin ? kMisIn : kMisOut;
         a.visited++;
