@@ -1606,6 +1606,8 @@ static int sweep(i2_graph* g, int algo, int src, int follow, int reps, i2_iter_r
   if (st) return st;
   st = ensure_symmetry(g);
   if (st) return st;
+  st = ensure_sp(g);  // every style is timed, the edge sweep too
+  if (st) return st;
   const long long V = g->g.nodes;
   if (!g->snap_dist) {
     I2_CK(dev_alloc(&g->snap_dist, sizeof(int) * V));
@@ -2117,7 +2119,10 @@ int i2_sweep(i2_graph* g, int algo, int src, int follow, int reps, i2_iter_recor
   if (algo != I2_CC && (src < 0 || src >= g->g.nodes)) return I2_ERR_ARG;
   if (algo == I2_SSSP && !g->g.eweight) return I2_ERR_ARG;
   if (follow >= 0) {
+    I2_CK(cudaSetDevice(g->device));
     int st = ensure_symmetry(g);
+    if (st) return st;
+    st = ensure_sp(g);
     if (st) return st;
     if (!((allowed_mask(g, algo) >> follow) & 1)) return I2_ERR_UNSUPPORTED;
   }
