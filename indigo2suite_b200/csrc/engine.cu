@@ -1614,8 +1614,12 @@ static int sweep(i2_graph* g, int algo, int src, int follow, int reps, i2_iter_r
     I2_CK(dev_alloc(&g->snap_bm, sizeof(unsigned) * 3ull * g->bm_words));
   }
   cudaStream_t s = g->stream;
-  const int mode = follow == I2_AUTO_LEARNED ? 2 : (follow < 0 ? 1 : 0);
-  st = prepare_run(g, s, make_params(g, algo, mode, follow < 0 ? 0 : follow, src, 1, 0));
+  // a followed style runs as a switch to itself: the states that the other
+  // styles are timed from are those of a run whose style may change
+  const int mode = follow == I2_AUTO_LEARNED ? 2 : (follow < 0 ? 1 : 3);
+  RunParams rp = make_params(g, algo, mode, follow < 0 ? 0 : follow, src, 1, 0);
+  rp.then_variant = rp.fixed_variant;
+  st = prepare_run(g, s, rp);
   if (st) return st;
   Ctx c = make_ctx(g);
   KernelFn ff = fill_kernel(algo);
