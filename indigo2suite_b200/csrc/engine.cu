@@ -636,7 +636,7 @@ struct i2_graph {
   int* h_stage = nullptr;  // pinned, kStageInts ints (results of small graphs on their way to the caller)
   bool staged = false;     // the last run's result has reached the caller's array
   std::map<ExecKey, ExecEntry> execs;
-  std::map<KernelFn, int> grids;  // launch grids of the resident kernels
+  std::map<const void*, int> grids;  // launch grids of the resident traversals' kernels
   std::vector<cudaGraph_t> graphs;
   int last_iters = 0;
   // sweep scratch
@@ -1247,32 +1247,60 @@ static StartFn start_kernel(int algo) {
   return k_start<kMIS>;
 }
 
+// The kernels of a resident traversal and their grids.
+struct ResidentPlan {
+  KernelFn loop = nullptr;   // every iteration, one cooperative launch
+  KernelFn fill = nullptr;   // a first frontier of many vertices (else null)
+  KernelFn seed = nullptr;   // its seeding, or that of many sources (else null)
+  StartFn start = nullptr;
+  int loop_grid = 0, fill_grid = 0, start_grid = 0;
+};
+
+// Looks the kernels up before the traversal's first event: a kernel's first use
+// in a process loads it (0.5-15 ms), which the report's device time must not hold.
+static ResidentPlan plan_resident(i2_graph* g, int algo, int mode, int variant, bool multi, const RunParams& rp) {
+  const auto grid = [g](const void* fn, int max_per_sm) {
+    auto it = g->grids.find(fn);
+    if (it == g->grids.end()) it = g->grids.emplace(fn, grid_for((KernelFn)fn, max_per_sm)).first;
+    return it->second;
+  };
+  const auto load = [g](const void* fn) {
+    if (!g->grids.emplace(fn, 0).second) return;
+    cudaFuncAttributes a;
+    if (cudaFuncGetAttributes(&a, fn) != cudaSuccess) cudaGetLastError();  // its launch reports it
+  };
+  ResidentPlan p;
+  const int v = mode == 0 ? variant : -1;
+  p.loop = resident_kernel(algo, v, rp.delta != 0, wide_form(g, v));
+  p.loop_grid = grid((const void*)p.loop, g->blocks_per_sm);
+  p.start = start_kernel(algo);
+  load((const void*)p.start);
+  const long long units = (long long)g->g.nodes / 4 + (long long)bm_block_words(g);
+  p.start_grid = (int)std::max(1LL, std::min(8LL * sm_count(), units / (4 * kBlock)));
+  const bool frontier = algo == I2_CC && !rp.uf_start;
+  if (frontier) {
+    p.fill = fill_kernel(algo);
+    p.fill_grid = grid((const void*)p.fill, 8);
+  }
+  if (frontier || multi) {
+    p.seed = seed_kernel(algo);
+    load((const void*)p.seed);
+  }
+  return p;
+}
+
 // A resident traversal: its start (one kernel; with the frontier's own kernels
 // where many vertices are in it), and one cooperative launch that runs every
 // iteration.
-static int launch_resident(i2_graph* g, int algo, int mode, int variant, bool multi, const RunParams& rp,
-                           cudaStream_t s) {
+static int launch_resident(i2_graph* g, const ResidentPlan& p, bool multi, const RunParams& rp, cudaStream_t s) {
   Ctx c = make_ctx(g);
   c.srcs = multi ? g->srcs : nullptr;
-  const int v = mode == 0 ? variant : -1;
-  KernelFn fn = resident_kernel(algo, v, rp.delta != 0, wide_form(g, v));
-  auto it = g->grids.find(fn);
-  if (it == g->grids.end()) it = g->grids.emplace(fn, grid_for(fn, g->blocks_per_sm)).first;
-  const unsigned words = (unsigned)bm_block_words(g);
-  const long long units = (long long)g->g.nodes / 4 + words;
-  const int start_grid = (int)std::max(1LL, std::min(8LL * sm_count(), units / (4 * kBlock)));
-  start_kernel(algo)<<<start_grid, kBlock, 0, s>>>(c, rp, words);
-  const bool frontier = algo == I2_CC && !rp.uf_start;
-  if (frontier) {
-    KernelFn ff = fill_kernel(algo);
-    auto fi = g->grids.find(ff);
-    if (fi == g->grids.end()) fi = g->grids.emplace(ff, grid_for(ff, 8)).first;
-    ff<<<fi->second, kBlock, 0, s>>>(c);
-  }
-  if (frontier || multi) seed_kernel(algo)<<<1, kBlock, 0, s>>>(c);
+  p.start<<<p.start_grid, kBlock, 0, s>>>(c, rp, (unsigned)bm_block_words(g));
+  if (p.fill) p.fill<<<p.fill_grid, kBlock, 0, s>>>(c);
+  if (p.seed) p.seed<<<1, kBlock, 0, s>>>(c);
   I2_CK(cudaGetLastError());
   void* args[1] = {&c};
-  I2_CK(cudaLaunchCooperativeKernel((const void*)fn, dim3(it->second), dim3(kBlock), args, 0, s));
+  I2_CK(cudaLaunchCooperativeKernel((const void*)p.loop, dim3(p.loop_grid), dim3(kBlock), args, 0, s));
   return I2_OK;
 }
 
@@ -1538,10 +1566,12 @@ int run_traversal(i2_graph* g, int algo, int src, const int* srcs_host, int nsrc
     st = build_exec(g, algo, mode, variant, multi, rp, &ex);
     if (st) return st;
   }
+  ResidentPlan plan;
+  if (resident) plan = plan_resident(g, algo, mode, variant, multi, rp);
   double host_relax_ms = -1.0;
   if (rep) I2_CK(cudaEventRecord(g->ev0, s));
   if (resident) {
-    st = launch_resident(g, algo, mode, variant, multi, rp, s);
+    st = launch_resident(g, plan, multi, rp, s);
     if (st) {  // refused: this graph's traversals relaunch from here on
       cudaGetLastError();
       g->resident_ok = false;
