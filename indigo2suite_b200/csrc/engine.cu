@@ -14,6 +14,7 @@
 // the next style on the device, so there is no host round trip per iteration.
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -539,11 +540,14 @@ static int sm_count() {
 
 // Preferred shared-memory carveout (percent of the unified L1/shared storage)
 // for the relax kernels; -1 leaves the choice to the driver. A large carveout
-// costs L1 capacity, which the adjacency reads use.
-static int g_carveout = -1;
+// costs L1 capacity, which the adjacency reads use. It is an attribute of the
+// kernels, which all graphs share, and decides how many blocks of one fit an SM:
+// a change invalidates the grids that every graph has kept (g_carveout_set).
+static std::atomic<int> g_carveout{-1};
+static std::atomic<unsigned> g_carveout_set{0};  // changes so far
 
 int grid_for(KernelFn fn, int max_per_sm) {
-  cudaFuncSetAttribute((const void*)fn, cudaFuncAttributePreferredSharedMemoryCarveout, g_carveout);
+  cudaFuncSetAttribute((const void*)fn, cudaFuncAttributePreferredSharedMemoryCarveout, g_carveout.load());
   int per = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)fn, kBlock, 0);
   per = std::max(1, std::min(per, max_per_sm));
@@ -637,6 +641,7 @@ struct i2_graph {
   bool staged = false;     // the last run's result has reached the caller's array
   std::map<ExecKey, ExecEntry> execs;
   std::map<const void*, int> grids;  // launch grids of the resident traversals' kernels
+  unsigned grids_of = 0;             // g_carveout_set they belong to
   std::vector<cudaGraph_t> graphs;
   int last_iters = 0;
   // sweep scratch
@@ -1259,6 +1264,9 @@ struct ResidentPlan {
 // Looks the kernels up before the traversal's first event: a kernel's first use
 // in a process loads it (0.5-15 ms), which the report's device time must not hold.
 static ResidentPlan plan_resident(i2_graph* g, int algo, int mode, int variant, bool multi, const RunParams& rp) {
+  const unsigned set = g_carveout_set.load();
+  if (g->grids_of != set) g->grids.clear();
+  g->grids_of = set;
   const auto grid = [g](const void* fn, int max_per_sm) {
     auto it = g->grids.find(fn);
     if (it == g->grids.end()) it = g->grids.emplace(fn, grid_for((KernelFn)fn, max_per_sm)).first;
@@ -1292,16 +1300,24 @@ static ResidentPlan plan_resident(i2_graph* g, int algo, int mode, int variant, 
 // A resident traversal: its start (one kernel; with the frontier's own kernels
 // where many vertices are in it), and one cooperative launch that runs every
 // iteration.
-static int launch_resident(i2_graph* g, const ResidentPlan& p, bool multi, const RunParams& rp, cudaStream_t s) {
+static cudaError_t launch_resident(i2_graph* g, const ResidentPlan& p, bool multi, const RunParams& rp,
+                                   cudaStream_t s) {
   Ctx c = make_ctx(g);
   c.srcs = multi ? g->srcs : nullptr;
   p.start<<<p.start_grid, kBlock, 0, s>>>(c, rp, (unsigned)bm_block_words(g));
   if (p.fill) p.fill<<<p.fill_grid, kBlock, 0, s>>>(c);
   if (p.seed) p.seed<<<1, kBlock, 0, s>>>(c);
-  I2_CK(cudaGetLastError());
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
   void* args[1] = {&c};
-  I2_CK(cudaLaunchCooperativeKernel((const void*)p.loop, dim3(p.loop_grid), dim3(kBlock), args, 0, s));
-  return I2_OK;
+  e = cudaLaunchCooperativeKernel((const void*)p.loop, dim3(p.loop_grid), dim3(kBlock), args, 0, s);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {  // another thread changed the carveout meanwhile
+    cudaGetLastError();
+    const int grid = g->grids[(const void*)p.loop] = grid_for(p.loop, g->blocks_per_sm);
+    e = cudaLaunchCooperativeKernel((const void*)p.loop, dim3(grid), dim3(kBlock), args, 0, s);
+  }
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
 }
 
 // Reset the bitmaps and the control block on the stream (host-driven paths).
@@ -1571,15 +1587,15 @@ int run_traversal(i2_graph* g, int algo, int src, const int* srcs_host, int nsrc
   double host_relax_ms = -1.0;
   if (rep) I2_CK(cudaEventRecord(g->ev0, s));
   if (resident) {
-    st = launch_resident(g, plan, multi, rp, s);
-    if (st) {  // refused: this graph's traversals relaunch from here on
-      cudaGetLastError();
-      g->resident_ok = false;
+    const cudaError_t e = launch_resident(g, plan, multi, rp, s);
+    if (e != cudaSuccess) {  // refused: one launch per iteration, for good where the device has no such launch
+      if (e == cudaErrorNotSupported) g->resident_ok = false;
+      resident = false;
       st = build_exec(g, algo, mode, variant, multi, rp, &ex);
       if (st) return st;
     }
   }
-  if (graph_loop && (!resident || !g->resident_ok)) {
+  if (graph_loop && !resident) {
     st = launch_exec(g, ex, rp, s);
     if (st) return st;
   } else if (!graph_loop) {
@@ -2000,7 +2016,7 @@ int i2_graph_download(const i2_graph* g, i2_eclgraph* out) {
 int i2_graph_tune(i2_graph* g, int heavy_threshold, int blocks_per_sm, int smem_carveout) {
   if (!g || heavy_threshold < 0 || blocks_per_sm < 0 || blocks_per_sm > 32) return I2_ERR_ARG;
   if (smem_carveout < -1 || smem_carveout > 100) return I2_ERR_ARG;
-  g_carveout = smem_carveout;
+  if (g_carveout.exchange(smem_carveout) != smem_carveout) ++g_carveout_set;
   I2_CK(cudaSetDevice(g->device));
   if (g->stream) I2_CK(cudaStreamSynchronize(g->stream));
   drop_execs(g);
@@ -2081,7 +2097,7 @@ int i2_graph_reorder(i2_graph* g, int order) {
   }
   // the copy launches like the original (settings of i2_graph_tune; the
   // heavy lists are sized for the threshold by the tune call)
-  st = i2_graph_tune(twin, g->heavy, g->blocks_per_sm, g_carveout);
+  st = i2_graph_tune(twin, g->heavy, g->blocks_per_sm, g_carveout.load());
   if (st) {
     i2_graph_free(twin);
     dev_free(inv);
