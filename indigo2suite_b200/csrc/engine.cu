@@ -747,7 +747,7 @@ static void dev_free_all(void* const* ptrs, int n) {
 
 void dev_free(void* ptr) { dev_free_all(&ptr, 1); }
 
-static int trim_pool() {
+int dev_trim() {
   DevPool* p = dev_pool();
   if (!p) return I2_ERR_NO_DEVICE;
   I2_CK(cudaStreamSynchronize(p->s));
@@ -2111,7 +2111,7 @@ int i2_graph_reorder(i2_graph* g, int order) {
 
 int i2_trim_device_memory(void) {
   if (i2_device_count() < 1) return I2_ERR_NO_DEVICE;
-  return trim_pool();
+  return dev_trim();
 }
 
 static int run_host_out(i2_graph* g, int algo, int src, int* out, const i2_opts* opts, i2_report* rep) {

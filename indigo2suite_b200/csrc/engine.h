@@ -68,6 +68,7 @@ int graph_copy_result(i2_graph* g, int* host_out, const i2_opts* opts);
 // dev_alloc.
 cudaError_t dev_alloc_bytes(void** p, size_t bytes);
 void dev_free(void* p);
+int dev_trim();  // the pool's unused blocks back to the driver; a status
 template <class T>
 inline cudaError_t dev_alloc(T** p, size_t bytes) {
   return dev_alloc_bytes(reinterpret_cast<void**>(p), bytes);

@@ -104,39 +104,52 @@ struct MinOp {
   __device__ __forceinline__ int operator()(int a, int b) const { return a < b ? a : b; }
 };
 
-// Scratch of a build, freed on every path. Up to kPooled bytes come from the
-// engine's pool, so that builds of ordinary graphs pay no cudaMalloc and
-// cudaFree (16 M keys: 3.4 of 4.6 ms); what is beyond them (tens of GB at RMAT
-// scale 26) is a plain allocation, which the pool never keeps.
+// Scratch of a build, freed on every path. Up to kPooled bytes at a time come
+// from the engine's pool, so that builds of ordinary graphs pay no cudaMalloc
+// and cudaFree (16 M keys: 3.4 of 4.6 ms); what is beyond them (tens of GB at
+// RMAT scale 26) is a plain allocation, which the pool never keeps. The parts of
+// a build (`outer`: the scratch that is alive around this one) share the bytes.
 struct Scratch {
   static constexpr int kMax = 16;
   static constexpr size_t kPooled = (size_t)2 << 30;
-  void* p[kMax] = {nullptr};
-  bool pooled[kMax] = {false};
-  int n = 0;
-  size_t total = 0;
+  explicit Scratch(Scratch* outer = nullptr) : total(outer ? outer->total : &own) {}
+  Scratch(const Scratch&) = delete;
+  Scratch& operator=(const Scratch&) = delete;
   template <class T>
   cudaError_t get(T** out, size_t bytes) {
     *out = nullptr;
     if (n == kMax) return cudaErrorMemoryAllocation;  // more buffers than one build takes
     bytes = bytes > 0 ? bytes : 1;
     void* q = nullptr;
-    const bool pool = total + bytes <= kPooled;
-    const cudaError_t e = pool ? dev_alloc(&q, bytes) : cudaMalloc(&q, bytes);
+    const bool pool = *total + bytes <= kPooled;
+    cudaError_t e = pool ? dev_alloc(&q, bytes) : cudaMalloc(&q, bytes);
+    if (e == cudaErrorMemoryAllocation && !pool) {  // what the pool holds unused may be enough
+      cudaGetLastError();
+      dev_trim();
+      e = cudaMalloc(&q, bytes);
+    }
     if (e == cudaSuccess) {
-      pooled[n] = pool;
+      pooled[n] = pool ? bytes : 0;
       p[n++] = q;
-      if (pool) total += bytes;
+      *total += pool ? bytes : 0;
     }
     *out = static_cast<T*>(q);
     return e;
   }
   ~Scratch() {
     for (int k = 0; k < n; ++k) {
+      *total -= pooled[k];
       if (pooled[k]) dev_free(p[k]);
       else cudaFree(p[k]);
     }
   }
+
+ private:
+  void* p[kMax] = {nullptr};
+  size_t pooled[kMax] = {0};  // bytes from the pool, 0: a plain allocation
+  int n = 0;
+  size_t own = 0;
+  size_t* const total;  // pooled bytes of the whole build
 };
 
 // CSR of `nodes` vertices from nkeys keys in k0 (k1: a buffer of the same
@@ -144,9 +157,9 @@ struct Scratch {
 // with the same weights. Weights: cw.mode 1 seeded; cw.mode 2 given per
 // key in w0 (w1: a buffer of the same size), duplicates keeping the smallest.
 static int csr_from_keys(unsigned long long* k0, unsigned long long* k1, int* w0, int* w1, long long nkeys,
-                         int nodes, CutWeights cw, bool symmetric, i2_graph** out) {
+                         int nodes, CutWeights cw, bool symmetric, Scratch& outer, i2_graph** out) {
   const KeyBits kb = key_bits(nodes);
-  Scratch sc;
+  Scratch sc(&outer);
   long long* d_num = nullptr;
   void* tmp = nullptr;
   size_t tb = 0, tb2 = 0;
@@ -326,10 +339,10 @@ __global__ void k_both_directions(const unsigned long long* __restrict__ pairs, 
 // passed `limit` without enough of them, or a CUDA status.
 template <class Make>
 static int first_distinct(long long want, long long start, long long limit, KeyBits kb, Make make,
-                          unsigned long long* out) {
+                          Scratch& outer, unsigned long long* out) {
   long long C = start;
   for (;;) {
-    Scratch sc;
+    Scratch sc(&outer);
     unsigned long long *k0, *k1, *i0, *i1;
     long long* d_num;
     cudaError_t e = sc.get(&k0, sizeof(unsigned long long) * C);
@@ -391,7 +404,8 @@ static int generate_rmat(long long n, int scale, long long samples, double a, do
   if (e != cudaSuccess) return cuda_status(e);
   k_rmat_keys<<<4096, 256>>>(seed, scale, make_thresholds(a, b, c), make_perm(seed, scale), samples, (int)n,
                              key_bits((int)n), k0);
-  return csr_from_keys(k0, k1, nullptr, nullptr, nkeys, (int)n, CutWeights{weighted ? 1 : 0, seed, nullptr}, true, out);
+  return csr_from_keys(k0, k1, nullptr, nullptr, nkeys, (int)n, CutWeights{weighted ? 1 : 0, seed, nullptr}, true, sc,
+                       out);
 }
 
 extern "C" int i2_graph_generate_rmat(int scale, int edge_factor, double a, double b, double c, uint64_t seed,
@@ -432,13 +446,14 @@ extern "C" int i2_graph_generate_er(int n, long long m, uint64_t seed, int weigh
                           [&](long long C, unsigned long long* keys, unsigned long long* idx) {
                             k_er_candidates<<<4096, 256>>>(seed, n, 0, C, kb, keys, idx);
                           },
-                          pairs);
+                          sc, pairs);
   if (st) return st;
   e = sc.get(&k0, sizeof(unsigned long long) * std::max(1LL, 2 * m));
   if (e == cudaSuccess) e = sc.get(&k1, sizeof(unsigned long long) * std::max(1LL, 2 * m));
   if (e != cudaSuccess) return cuda_status(e);
   k_both_directions<<<4096, 256>>>(pairs, m, kb, k0);
-  return csr_from_keys(k0, k1, nullptr, nullptr, 2 * m, n, CutWeights{weighted ? 1 : 0, seed, nullptr}, true, out);
+  return csr_from_keys(k0, k1, nullptr, nullptr, 2 * m, n, CutWeights{weighted ? 1 : 0, seed, nullptr}, true, sc,
+                       out);
 }
 
 extern "C" int i2_graph_generate_grid(int side, double remove_frac, double add_frac, uint64_t seed, int weighted,
@@ -478,11 +493,12 @@ extern "C" int i2_graph_generate_grid(int side, double remove_frac, double add_f
                             [&](long long C, unsigned long long* keys, unsigned long long* idx) {
                               k_grid_extra_candidates<<<4096, 256>>>(seed, side, drop, C, kb, keys, idx);
                             },
-                            extra);
+                            sc, extra);
     if (st) return st;
     k_both_directions<<<4096, 256>>>(extra, K, kb, k0 + 2 * G);
   }
-  return csr_from_keys(k0, k1, nullptr, nullptr, nkeys, (int)V, CutWeights{weighted ? 1 : 0, seed, nullptr}, true, out);
+  return csr_from_keys(k0, k1, nullptr, nullptr, nkeys, (int)V, CutWeights{weighted ? 1 : 0, seed, nullptr}, true, sc,
+                       out);
 }
 
 extern "C" int i2_graph_from_coo_device(int nodes, long long m, const int* src, const int* dst, const int* w,
@@ -511,7 +527,7 @@ extern "C" int i2_graph_from_coo_device(int nodes, long long m, const int* src, 
   e = cudaMemcpy(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return cuda_status(e);
   if (hbad) return I2_ERR_FORMAT;
-  return csr_from_keys(k0, k1, w0, w1, nkeys, nodes, CutWeights{w ? 2 : 0, 0, nullptr}, symmetrize != 0, out);
+  return csr_from_keys(k0, k1, w0, w1, nkeys, nodes, CutWeights{w ? 2 : 0, 0, nullptr}, symmetrize != 0, sc, out);
 }
 
 // ---------------------------------------------------------------------------
@@ -597,7 +613,8 @@ int degree_ordered_copy(const i2_graph* g, i2_graph** twin, int** inv_out) {
     dev_free(inv);
     return cuda_status(e);
   }
-  st = csr_from_keys(k0, k1, w0, w1, E, n, CutWeights{w ? 2 : 0, 0, nullptr}, graph_known_symmetric(g), twin);
+  st = csr_from_keys(k0, k1, w0, w1, E, n, CutWeights{w ? 2 : 0, 0, nullptr}, graph_known_symmetric(g), sc,
+                     twin);
   if (st) {
     dev_free(inv);
     return st;
