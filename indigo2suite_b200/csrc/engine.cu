@@ -477,11 +477,13 @@ static KernelFn dispatch_kernel(int algo, bool wide) {
   return dispatch_fn<kCC>(wide);  // MIS never dispatches
 }
 
-KernelFn relax_kernel(int algo, int v, bool near_far) {
+// One launch per iteration in style v: in a run of that style alone (mode 0), or
+// in one whose style may change.
+static KernelFn relax_kernel(int algo, int mode, int v, bool near_far, bool wide) {
   if (near_far && algo == kSSSP && v == kVPCta) return near_far_kernel(false);
-  if (algo == kBFS) return relax_fn<kBFS>(v);
-  if (algo == kSSSP) return relax_fn<kSSSP>(v);
-  if (algo == kCC) return relax_fn<kCC>(v);
+  if (algo == kBFS) return relax_fn<kBFS>(v, mode != 0, wide);
+  if (algo == kSSSP) return relax_fn<kSSSP>(v, mode != 0, wide);
+  if (algo == kCC) return relax_fn<kCC>(v, mode != 0, wide);
   return mis_kernel(false);  // one style
 }
 
@@ -1211,7 +1213,8 @@ static int build_exec(i2_graph* g, int algo, int mode, int variant, bool multi, 
   // iteration selected.
   {
     cudaGraphNode_t n;
-    KernelFn fn = mode == 0 ? relax_kernel(algo, variant, rp.delta != 0) : dispatch_kernel(algo, wide_selector(g));
+    KernelFn fn = mode == 0 ? relax_kernel(algo, 0, variant, rp.delta != 0, wide_form(g, variant))
+                            : dispatch_kernel(algo, wide_selector(g));
     st = add_kernel_node(body, &n, nullptr, 0, fn, grid_for(fn, g->blocks_per_sm), &c);
     if (st) return st;
   }
@@ -1345,7 +1348,7 @@ static int run_host_loop(i2_graph* g, cudaStream_t s, int algo, bool multi, doub
     // the last launch's decision: another frontier, a near/far split, the
     // compress launch of union-find, or the end (including the iteration cap)
     if (!h->go || (h->status & kStatusIterCap)) break;
-    KernelFn fn = relax_kernel(algo, h->variant, h->delta != 0);
+    KernelFn fn = relax_kernel(algo, h->mode, h->variant, h->delta != 0, wide_form(g, h->variant));
     I2_CK(cudaEventRecord(g->ev2, s));
     fn<<<grid_for(fn, g->blocks_per_sm), kBlock, 0, s>>>(c);
     I2_CK(cudaGetLastError());
@@ -2326,7 +2329,7 @@ extern "C" int i2_run_noalloc(int algo, const i2_eclgraph* dev, int src, int* di
   KernelFn ff = fill_kernel(algo);
   ff<<<grid_for(ff, 8), kBlock, 0, s>>>(c);
   seed_kernel(algo)<<<1, kBlock, 0, s>>>(c);
-  KernelFn fn = relax_kernel(algo, kVPCta, false);
+  KernelFn fn = relax_kernel(algo, 0, kVPCta, false, false);
   const int grid = grid_for(fn, 8);
   Ctl h;
   for (;;) {

@@ -12,12 +12,14 @@ int cuda_status(cudaError_t e);
 int grid_for(KernelFn fn, int max_per_sm);
 // Relax kernels of one algorithm, each set instantiated in a translation unit
 // of its own (relax_*.cu, resident_*.cu: they compile in parallel).
-// relax_fn: one launch per iteration in style v; dispatch_fn: one launch per
-// iteration in the style the selectors picked; resident_fn: every iteration in
-// one launch, in style v or (v < 0) the selectors' per-iteration pick. `wide`:
-// the selectors' form compiled for more resident blocks per SM (I2_FIXED_MIN_BLOCKS).
+// relax_fn: one launch per iteration in style v, whose last block picks the next
+// style (`select`) or stays with v; dispatch_fn: one launch per iteration in the
+// style the selectors picked; resident_fn: every iteration in one launch, in
+// style v or (v < 0) the selectors' per-iteration pick. `wide`: the form compiled
+// for more resident blocks per SM (I2_FIXED_MIN_BLOCKS), which the selectors'
+// kernels and the edge-balanced style have (engine.cu: wide_form).
 template <int ALG>
-KernelFn relax_fn(int v);
+KernelFn relax_fn(int v, bool select, bool wide);
 template <int ALG>
 KernelFn dispatch_fn(bool wide);
 template <int ALG>

@@ -8,22 +8,29 @@
 
 namespace i2 {
 
-template <int ALG>
-KernelFn relax_fn(int v) {
+template <int ALG, class H>
+KernelFn relax_fn_of(int v) {
   switch (v) {
-    case kVPThread: return relax_push<ALG, kVPThread>;
-    case kVPWarp: return relax_push<ALG, kVPWarp>;
-    case kVPCta: return relax_edge_balanced<ALG>;
-    case kVPBlock: return relax_push<ALG, kVPBlock>;
-    case kPullFrontier: return relax_pull<ALG, true>;
-    case kPullTopo: return relax_pull<ALG, false>;
-    case kEdgeTopo: return relax_edge_topo<ALG>;
-    case kPushTopo: return relax_push_topo<ALG>;
+    case kVPThread: return relax_push<ALG, kVPThread, H>;
+    case kVPWarp: return relax_push<ALG, kVPWarp, H>;
+    case kVPCta: return relax_edge_balanced<ALG, H>;
+    case kVPBlock: return relax_push<ALG, kVPBlock, H>;
+    case kPullFrontier: return relax_pull<ALG, true, H>;
+    case kPullTopo: return relax_pull<ALG, false, H>;
+    case kEdgeTopo: return relax_edge_topo<ALG, H>;
+    case kPushTopo: return relax_push_topo<ALG, H>;
     case kUnionFind:
-      if constexpr (ALG == kCC) return relax_union<ALG>;
+      if constexpr (ALG == kCC) return relax_union<ALG, H>;
       return nullptr;
   }
   return nullptr;
+}
+
+template <int ALG>
+KernelFn relax_fn(int v, bool select, bool wide) {
+  if (select) return relax_fn_of<ALG, SelectHead>(v);
+  if (v == kVPCta && wide) return relax_edge_balanced<ALG, FixedHead, true>;
+  return relax_fn_of<ALG, FixedHead>(v);
 }
 
 template <int ALG>

@@ -2014,28 +2014,33 @@ __device__ __forceinline__ bool body_mis(const Ctx& c, H& S, Stage& s) {
 }
 
 // ---------------------------------------------------------------------------
-// Kernel wrappers.
-template <int ALG, int VAR>
+// Kernel wrappers, one launch per iteration. H: what the end of an iteration may
+// have to do (common.cuh); with the selector's network in it the pull kernels
+// took 69-78 registers and lost the fourth block per SM (BFS pull_frontier,
+// launched per iteration, us, before / with the network / FixedHead: RMAT-20
+// 1,132 / 1,464 / 1,059, grid 6000^2 83.7 / 108 / 81.8 ms).
+template <int ALG, int VAR, class H>
 __global__ void __launch_bounds__(kBlock) relax_push(const __grid_constant__ Ctx c) {
   __shared__ Stage s;
-  __shared__ SelectHead S;
+  __shared__ H S;
   load_head(c, S);
   __syncthreads();
   body_push<ALG, VAR>(c, S, s);
 }
 
-template <int ALG>
-__global__ void __launch_bounds__(kBlock, I2_EB_MIN_BLOCKS) relax_edge_balanced(const __grid_constant__ Ctx c) {
+template <int ALG, class H, bool LONG = false>
+__global__ void __launch_bounds__(kBlock, LONG ? I2_FIXED_MIN_BLOCKS : I2_EB_MIN_BLOCKS)
+    relax_edge_balanced(const __grid_constant__ Ctx c) {
   __shared__ EBShared sh;
-  __shared__ SelectHead S;
+  __shared__ H S;
   load_head(c, S);
   __syncthreads();
-  body_edge_balanced<ALG>(c, S, sh);
+  body_edge_balanced<ALG, false, LONG>(c, S, sh);
 }
 
 static __global__ void __launch_bounds__(kBlock, I2_FIXED_MIN_BLOCKS) relax_mis(const __grid_constant__ Ctx c) {
   __shared__ Stage s;
-  __shared__ SelectHead S;
+  __shared__ FixedHead S;
   load_head(c, S);
   __syncthreads();
   body_mis(c, S, s);
@@ -2044,43 +2049,43 @@ static __global__ void __launch_bounds__(kBlock, I2_FIXED_MIN_BLOCKS) relax_mis(
 // Edge-balanced SSSP push with near/far ordering (Ctl::delta != 0).
 static __global__ void __launch_bounds__(kBlock, I2_EB_MIN_BLOCKS) relax_near_far(const __grid_constant__ Ctx c) {
   __shared__ EBSharedFar sh;
-  __shared__ SelectHead S;
+  __shared__ FixedHead S;
   load_head(c, S);
   __syncthreads();
   body_edge_balanced<kSSSP, true>(c, S, sh);
 }
 
-template <int ALG>
+template <int ALG, class H>
 __global__ void __launch_bounds__(kBlock) relax_push_topo(const __grid_constant__ Ctx c) {
   __shared__ Stage s;
-  __shared__ SelectHead S;
+  __shared__ H S;
   load_head(c, S);
   __syncthreads();
   body_push_topo<ALG>(c, S, s);
 }
 
-template <int ALG>
+template <int ALG, class H>
 __global__ void __launch_bounds__(kBlock) relax_edge_topo(const __grid_constant__ Ctx c) {
   __shared__ Stage s;
-  __shared__ SelectHead S;
+  __shared__ H S;
   load_head(c, S);
   __syncthreads();
   body_edge_topo<ALG>(c, S, s);
 }
 
-template <int ALG>
+template <int ALG, class H>
 __global__ void __launch_bounds__(kBlock) relax_union(const __grid_constant__ Ctx c) {
   __shared__ Stage s;
-  __shared__ SelectHead S;
+  __shared__ H S;
   load_head(c, S);
   __syncthreads();
   body_union<ALG>(c, S, s);
 }
 
-template <int ALG, bool FRONTIER>
-__global__ void __launch_bounds__(kBlock) relax_pull(const __grid_constant__ Ctx c) {
+template <int ALG, bool FRONTIER, class H>
+__global__ void __launch_bounds__(kBlock, 4) relax_pull(const __grid_constant__ Ctx c) {
   __shared__ Stage s;
-  __shared__ SelectHead S;
+  __shared__ H S;
   load_head(c, S);
   __syncthreads();
   body_pull<ALG, FRONTIER>(c, S, s);

@@ -3,7 +3,7 @@
 
 namespace i2 {
 
-template KernelFn relax_fn<kBFS>(int);
+template KernelFn relax_fn<kBFS>(int, bool, bool);
 template KernelFn dispatch_fn<kBFS>(bool);
 
 }  // namespace i2

@@ -3,7 +3,7 @@
 
 namespace i2 {
 
-template KernelFn relax_fn<kCC>(int);
+template KernelFn relax_fn<kCC>(int, bool, bool);
 template KernelFn dispatch_fn<kCC>(bool);
 
 }  // namespace i2

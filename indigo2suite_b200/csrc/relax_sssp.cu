@@ -3,7 +3,7 @@
 
 namespace i2 {
 
-template KernelFn relax_fn<kSSSP>(int);
+template KernelFn relax_fn<kSSSP>(int, bool, bool);
 template KernelFn dispatch_fn<kSSSP>(bool);
 KernelFn near_far_launch() { return relax_near_far; }
 
