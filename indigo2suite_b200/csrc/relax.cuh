@@ -1430,9 +1430,13 @@ __device__ __forceinline__ bool body_pull(const Ctx& c, H& S, Stage& s) {
   // edge-balanced push takes F_i for level i), so a neighbour reached in this
   // iteration waits. A run of this style alone uses it at once: it recomputes
   // every vertex until none falls, so levels reached early and too large are
-  // corrected. Fewer iterations where neighbours are visited late in a sweep
-  // (us, at once / level by level: RMAT-20 17,632 / 22,739, RMAT-14 730 / 902).
+  // corrected. It takes fewer iterations where neighbours are visited late in a
+  // sweep (RMAT-18 4-5 instead of 5, grid 1024^2 without long edges 1,793 of 2,045).
+  // One test of the neighbour's value covers this and an unreached neighbour: with
+  // a second one the loop's loads are no longer issued together (RMAT-18, an
+  // iteration of the hub's thread 1,450 instead of 1,082 us).
   const bool by_level = ALG == kBFS && !FRONTIER && S.mode != 0;
+  const int last = by_level ? i : kInf - 1;  // values above it are no use to BFS
   // Smallest candidate any frontier vertex can produce.
   const int bound = FRONTIER ? (fmin == kInf ? kInf : Op<ALG>::cand(fmin, c.gs.wmin)) : INT_MIN;
   for (long long base = (long long)blockIdx.x * kBlock; base < V; base += (long long)gridDim.x * kBlock) {
@@ -1450,8 +1454,7 @@ __device__ __forceinline__ bool body_pull(const Ctx& c, H& S, Stage& s) {
           const int u = ld_adj(nl + k);
           if (FRONTIER && !((bmc[u >> 5] >> (u & 31)) & 1u)) continue;
           const int du = c.dist[u];
-          if (!Op<ALG>::valid(du)) continue;
-          if (by_level && du > i) continue;
+          if (ALG == kBFS && !FRONTIER ? du > last : !Op<ALG>::valid(du)) continue;
           const int cd = Op<ALG>::cand(du, Op<ALG>::kWeighted ? ld_adj(ew + k) : 0);
           if (cd < best) {
             best = cd;
