@@ -189,13 +189,18 @@ struct CtlHead {
   alignas(128) unsigned done;  // blocks finished in the current launch
 };
 // A block's copy of the head, by what the end of an iteration may have to do:
-// pick the next style (every kernel but the resident ones of one fixed style,
-// which leave the network's code and its registers out).
+// pick the next style, by the network too (SelectHead) or by the rule and fixed
+// switches alone (RuleHead: graphs larger than any the network was trained on,
+// where it is never asked), or stay with the one style (FixedHead). The
+// network's weights are loaded up front, so its code sets a kernel's registers.
 struct SelectHead : CtlHead {
-  static constexpr bool kSelect = true;
+  static constexpr bool kSelect = true, kNetwork = true;
+};
+struct RuleHead : CtlHead {
+  static constexpr bool kSelect = true, kNetwork = false;
 };
 struct FixedHead : CtlHead {
-  static constexpr bool kSelect = false;
+  static constexpr bool kSelect = false, kNetwork = false;
 };
 constexpr int kHeadWords = sizeof(CtlHead) / 4;
 static_assert(kHeadWords <= kBlock, "one word of the head per thread");

@@ -62,14 +62,19 @@ static __device__ void select_next(const Ctx& c, H& S, int next_iter, int nxt, b
   const unsigned e = slot_edges(p);
   int v = S.fixed_variant;
   if constexpr (H::kSelect) {
-    __shared__ float h1[kHidden], h2[kHidden], y[kOut];
     const int mode = S.mode;
-    const bool learned = c.mlp && c.gs.nodes <= kMaxTrainedNodes;
-    const long long sn = S.sel_n, se = S.sel_e;
-    const bool moved = next_iter == 0 || 2LL * n > 3LL * sn || 3LL * n < 2LL * sn || 2LL * e > 3LL * se ||
-                       3LL * e < 2LL * se || next_iter - S.sel_iter >= 16;
-    const bool infer = mode == 2 && learned && cond && moved && force < 0;
-    if (infer) mlp_forward_block(c.mlp, S.feat, h1, h2, y);
+    [[maybe_unused]] const float* y = nullptr;
+    bool learned = false, infer = false;
+    if constexpr (H::kNetwork) {
+      __shared__ float h1[kHidden], h2[kHidden], out[kOut];
+      learned = c.mlp && c.gs.nodes <= kMaxTrainedNodes;
+      const long long sn = S.sel_n, se = S.sel_e;
+      const bool moved = next_iter == 0 || 2LL * n > 3LL * sn || 3LL * n < 2LL * sn || 2LL * e > 3LL * se ||
+                         3LL * e < 2LL * se || next_iter - S.sel_iter >= 16;
+      infer = mode == 2 && learned && cond && moved && force < 0;
+      if (infer) mlp_forward_block(c.mlp, S.feat, h1, h2, out);
+      y = out;
+    }
     if (threadIdx.x == 0) {
       if (mode == 3) {
         v = next_iter >= S.then_at ? S.then_variant : S.fixed_variant;

@@ -2168,7 +2168,10 @@ template <int ALG, int VAR, bool DEFER = false,
                                           : I2_FIXED_MIN_BLOCKS)>
 __global__ void __launch_bounds__(kBlock, MINB) relax_resident(const __grid_constant__ Ctx c) {
   __shared__ AnyShared<DEFER> sh;
-  __shared__ typename std::conditional<(VAR < 0), SelectHead, FixedHead>::type S;
+  // the selectors' form for more blocks runs on the largest graphs only
+  static_assert(kWideSelectorNodes > kMaxTrainedNodes, "no network in the wide forms");
+  using Pick = typename std::conditional<(MINB > I2_SEL_MIN_BLOCKS), RuleHead, SelectHead>::type;
+  __shared__ typename std::conditional<(VAR < 0), Pick, FixedHead>::type S;
   constexpr bool LONG = DEFER || (VAR == kVPCta && MINB == I2_FIXED_MIN_BLOCKS);  // skewed graphs' forms
   // thread 0's: barrier generation, whether to go on, the test hook (kept in
   // shared memory: the bodies have no register to spare)
@@ -2214,7 +2217,7 @@ __global__ void __launch_bounds__(kBlock, MINB) relax_resident(const __grid_cons
 template <int ALG, int MINB = I2_SEL_MIN_BLOCKS>
 __global__ void __launch_bounds__(kBlock, MINB) relax_dispatch(const __grid_constant__ Ctx c) {
   __shared__ AnyShared<> sh;
-  __shared__ SelectHead S;
+  __shared__ typename std::conditional<(MINB > I2_SEL_MIN_BLOCKS), RuleHead, SelectHead>::type S;
   load_head(c, S);
   __syncthreads();
   switch (S.variant) {
