@@ -1027,6 +1027,20 @@ static bool wide_form(const i2_graph* g, int variant) {
   return variant == kVPCta ? g->gs.degcv > 1.f : wide_selector(g);
 }
 
+// Most resident blocks per SM of a style's kernel on this graph. The
+// edge-balanced push of BFS and SSSP takes 4 of the 5 it is compiled for on
+// sparse graphs of even degrees (average below 6: grids, road networks), where
+// the blocks wait on the same few cache lines and, from 2^25 vertices, push one
+// another's out of L2. 5 / 4 blocks: SSSP grid 7000^2 70.5 / 65.8 ms, 6000^2
+// 52.2 / 48.6, 2000^2 4.47 / 4.31, ER 4 x 10^7 with 4 entries a vertex 21.9 /
+// 21.2, BFS grid 2000^2 1,709 / 1,600 us; ER with 8 entries a vertex gains
+// nothing (8 x 10^6 BFS 918 / 952 us) and CC, whose first iteration holds every
+// vertex, loses (ER 4 x 10^7 with 4 entries 39.8 / 41.9 ms).
+static int style_blocks(const i2_graph* g, int algo, int variant) {
+  const bool sparse = variant == kVPCta && (algo == I2_BFS || algo == I2_SSSP) && g->gs.degcv <= 1.f && g->gs.avgdeg < 6.f;
+  return sparse ? std::min(g->blocks_per_sm, 4) : g->blocks_per_sm;
+}
+
 static int allowed_mask(const i2_graph* g, int algo) {
   int m = 0;
   for (int v = 0; v < kNumVariants; ++v) m |= 1 << v;
@@ -1223,7 +1237,7 @@ static int build_exec(i2_graph* g, int algo, int mode, int variant, bool multi, 
     cudaGraphNode_t n;
     KernelFn fn = mode == 0 ? relax_kernel(algo, 0, variant, rp.delta != 0, wide_form(g, variant))
                             : dispatch_kernel(algo, wide_selector(g));
-    st = add_kernel_node(body, &n, nullptr, 0, fn, grid_for(fn, g->blocks_per_sm), &c);
+    st = add_kernel_node(body, &n, nullptr, 0, fn, grid_for(fn, style_blocks(g, algo, mode == 0 ? variant : -1)), &c);
     if (st) return st;
   }
   ExecEntry e;
@@ -1269,7 +1283,7 @@ struct ResidentPlan {
   KernelFn fill = nullptr;   // a first frontier of many vertices (else null)
   KernelFn seed = nullptr;   // its seeding, or that of many sources (else null)
   StartFn start = nullptr;
-  int loop_grid = 0, fill_grid = 0, start_grid = 0;
+  int loop_grid = 0, loop_blocks = 0, fill_grid = 0, start_grid = 0;
 };
 
 // Looks the kernels up before the traversal's first event: a kernel's first use
@@ -1291,7 +1305,8 @@ static ResidentPlan plan_resident(i2_graph* g, int algo, int mode, int variant, 
   ResidentPlan p;
   const int v = mode == 0 ? variant : -1;
   p.loop = resident_kernel(algo, v, rp.delta != 0, wide_form(g, v));
-  p.loop_grid = grid((const void*)p.loop, g->blocks_per_sm);
+  p.loop_blocks = style_blocks(g, algo, v);
+  p.loop_grid = grid((const void*)p.loop, p.loop_blocks);
   p.start = start_kernel(algo);
   load((const void*)p.start);
   const long long units = (long long)g->g.nodes / 4 + (long long)bm_block_words(g);
@@ -1324,7 +1339,7 @@ static cudaError_t launch_resident(i2_graph* g, const ResidentPlan& p, bool mult
   e = cudaLaunchCooperativeKernel((const void*)p.loop, dim3(p.loop_grid), dim3(kBlock), args, 0, s);
   if (e == cudaErrorCooperativeLaunchTooLarge) {  // another thread changed the carveout meanwhile
     cudaGetLastError();
-    const int grid = g->grids[(const void*)p.loop] = grid_for(p.loop, g->blocks_per_sm);
+    const int grid = g->grids[(const void*)p.loop] = grid_for(p.loop, p.loop_blocks);
     e = cudaLaunchCooperativeKernel((const void*)p.loop, dim3(grid), dim3(kBlock), args, 0, s);
   }
   if (e != cudaSuccess) cudaGetLastError();
@@ -1358,7 +1373,7 @@ static int run_host_loop(i2_graph* g, cudaStream_t s, int algo, bool multi, doub
     if (!h->go || (h->status & kStatusIterCap)) break;
     KernelFn fn = relax_kernel(algo, h->mode, h->variant, h->delta != 0, wide_form(g, h->variant));
     I2_CK(cudaEventRecord(g->ev2, s));
-    fn<<<grid_for(fn, g->blocks_per_sm), kBlock, 0, s>>>(c);
+    fn<<<grid_for(fn, style_blocks(g, algo, h->variant)), kBlock, 0, s>>>(c);
     I2_CK(cudaGetLastError());
     I2_CK(cudaEventRecord(g->ev3, s));
     I2_CK(cudaEventSynchronize(g->ev3));
