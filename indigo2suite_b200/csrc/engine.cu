@@ -1036,7 +1036,20 @@ static bool wide_form(const i2_graph* g, int variant) {
 // 21.2, BFS grid 2000^2 1,709 / 1,600 us; ER with 8 entries a vertex gains
 // nothing (8 x 10^6 BFS 918 / 952 us) and CC, whose first iteration holds every
 // vertex, loses (ER 4 x 10^7 with 4 entries 39.8 / 41.9 ms).
+// Union-find takes about one block per SM for every 2^11 vertices an SM has, 8
+// chunks a warp: more warps link trees that the others have not joined yet, and
+// meet at the same roots. us, 1 / 2 / 3 / 4 / 6 blocks: RMAT-17 110 / 122 / 153 /
+// 193 / 204, RMAT-18 117 / 172 / 198 / 215 / 305, RMAT-20 171 / 140 / 144 / 168 /
+// 187, RMAT-22 473 / 295 / 235 / 213 / 186, ER 3 x 10^5 139 / 138 / 200 / 255 /
+// 371, 6 x 10^5 175 / 170 / 163 / 192 / 301, 2 x 10^6 304 / 219 / 200 / 192 / 195,
+// grid 300^2 121 / 108 / 112 / 134 / 116, 1000^2 223 / 159 / 136 / 149 / 146,
+// 2000^2 705 / 408 / 312 / 262 / 224.
 static int style_blocks(const i2_graph* g, int algo, int variant) {
+  if (variant == kUnionFind) {
+    const long long per_block = 8LL * kWarp * kWarpsPerBlock, sms = sm_count();
+    const long long blocks = (g->g.nodes + per_block * sms / 2) / (per_block * sms);
+    return (int)std::min<long long>(std::max(1LL, blocks), std::min(g->blocks_per_sm, I2_UF_MIN_BLOCKS));
+  }
   const bool sparse = variant == kVPCta && (algo == I2_BFS || algo == I2_SSSP) && g->gs.degcv <= 1.f && g->gs.avgdeg < 6.f;
   return sparse ? std::min(g->blocks_per_sm, 4) : g->blocks_per_sm;
 }

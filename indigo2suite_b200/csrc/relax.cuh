@@ -959,7 +959,7 @@ struct EpiStage {
 #ifndef I2_FIXED_MIN_BLOCKS
 #define I2_FIXED_MIN_BLOCKS 6
 #endif
-// ... and union-find's (4, 6 and 8 within the noise of its links).
+// ... and union-find's: the most that it is launched with (style_blocks).
 #ifndef I2_UF_MIN_BLOCKS
 #define I2_UF_MIN_BLOCKS 6
 #endif
@@ -2077,7 +2077,7 @@ __global__ void __launch_bounds__(kBlock) relax_edge_topo(const __grid_constant_
 }
 
 template <int ALG, class H>
-__global__ void __launch_bounds__(kBlock) relax_union(const __grid_constant__ Ctx c) {
+__global__ void __launch_bounds__(kBlock, I2_UF_MIN_BLOCKS) relax_union(const __grid_constant__ Ctx c) {
   __shared__ Stage s;
   __shared__ H S;
   load_head(c, S);
