@@ -98,6 +98,8 @@ struct GStats {
   int edges;
   int maxdeg;
   int nheavy;       // vertices with degree >= heavy threshold
+  int linked;       // vertices with edges
+  int first;        // the smallest of them (kInf: none)
   int wmin;         // minimum edge weight (1 for BFS)
   int symmetric;    // 1 when every (u,v,w) has a (v,u,w) partner
   float avgdeg;
@@ -170,7 +172,7 @@ struct CtlHead {
   int pcur;                 // current far pile
   int uf_phase;             // union-find CC: 1 after the hook launch (the compress launch follows)
   int uf_giant;             // union-find CC: root of the sampled largest tree
-  int uf_start;             // union-find CC from the first iteration: no frontier is built
+  int whole;                // the first iteration takes every vertex, without a frontier list (union-find CC, MIS)
   unsigned uf_step;         // union-find CC: order of the vertices (body_union)
   int then_at;              // mode 3: iteration from which then_variant runs
   int then_variant;

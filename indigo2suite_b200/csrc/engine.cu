@@ -39,9 +39,18 @@ static_assert((int)kNumVariants == (int)I2_NUM_VARIANTS, "variant count");
 // ---------------------------------------------------------------------------
 // Init kernels.
 
+// Counts of a frontier that is not listed: every vertex with edges (records and
+// features show what a listed one would).
+static __device__ __forceinline__ void whole_slot(const Ctx& c, Slot& s) {
+  s.packed = ((unsigned long long)c.gs.linked << 32) | (unsigned)c.g.edges;
+  s.hpacked = (unsigned long long)c.gs.nheavy << 32;
+  s.maxdeg = c.gs.maxdeg;
+  s.mindist = c.gs.first;
+}
+
 // dist[v] = INF (BFS/SSSP) or v (CC). For CC every vertex enters F_0, unless
-// union-find runs from the first iteration (uf_start): it reads no frontier, so
-// none is built.
+// union-find runs from the first iteration (CtlHead::whole): it reads no
+// frontier, so none is built.
 template <int ALG>
 __global__ void __launch_bounds__(kBlock) k_fill(Ctx c) {
   __shared__ Stage s;
@@ -50,14 +59,10 @@ __global__ void __launch_bounds__(kBlock) k_fill(Ctx c) {
   acc_init(a);
   __syncthreads();
   const int V = c.g.nodes;
-  if (ALG == kCC && c.ctl->uf_start) {
+  if (ALG == kCC && c.ctl->whole) {
     const unsigned stride = gridDim.x * kBlock;
     for (unsigned v = blockIdx.x * kBlock + threadIdx.x; v < (unsigned)V; v += stride) c.dist[v] = (int)v;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {  // the record's frontier: every vertex
-      c.ctl->slot[0].packed = ((unsigned long long)V << 32) | (unsigned)c.g.edges;
-      c.ctl->slot[0].maxdeg = c.gs.maxdeg;
-      c.ctl->slot[0].mindist = 0;
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) whole_slot(c, c.ctl->slot[0]);
     return;
   }
   for (long long base = (long long)blockIdx.x * kBlock; base < V; base += (long long)gridDim.x * kBlock) {
@@ -148,7 +153,7 @@ __global__ void __launch_bounds__(kBlock) k_seed(Ctx c) {
 // Per-run parameters, passed by value to k_reset so that queued runs never
 // share a host buffer.
 struct RunParams {
-  int algo, mode, fixed_variant, allowed, src, nsrc, iter_cap, delta, hold, stall_ms, then_at, then_variant, hshift, uf_start;
+  int algo, mode, fixed_variant, allowed, src, nsrc, iter_cap, delta, hold, stall_ms, then_at, then_variant, hshift, whole;
   unsigned uf_step;
   bool operator!=(const RunParams& o) const { return std::memcmp(this, &o, sizeof(RunParams)) != 0; }
 };
@@ -170,7 +175,7 @@ static __device__ __forceinline__ void reset_head(CtlHead& S, const RunParams& p
   S.then_at = p.then_at;
   S.then_variant = p.then_variant;
   S.hold = p.hold;
-  S.uf_start = p.uf_start;
+  S.whole = p.whole;
   S.uf_step = p.uf_step;
   S.stall_ns = (unsigned long long)p.stall_ms * 1000000ull;
   S.threshold = p.delta > 0 ? p.delta : kInf;  // sources start at 0
@@ -197,7 +202,7 @@ __global__ void k_reset(Ctl* ctl, RunParams p) {
 template <int ALG>
 __global__ void __launch_bounds__(kBlock) k_start(const __grid_constant__ Ctx c, RunParams p, unsigned words) {
   const bool single = (ALG == kBFS || ALG == kSSSP) && !c.srcs;
-  const bool whole = single || ALG == kMIS || (ALG == kCC && p.uf_start);
+  const bool whole = single || ALG == kMIS || (ALG == kCC && p.whole);
   const int V = c.g.nodes;
   const int src = single ? p.src : -1;
   const int deg = single ? c.g.nindex[src + 1] - c.g.nindex[src] : 0;
@@ -243,11 +248,10 @@ __global__ void __launch_bounds__(kBlock) k_start(const __grid_constant__ Ctx c,
           c.htoff[0][0] = 0;
         }
       }
-    } else if (whole) {  // the record's frontier: every vertex
+    } else if (whole) {
+      S.whole = 1;
       S.visited = V;
-      sl.packed = ((unsigned long long)V << 32) | (unsigned)c.g.edges;
-      sl.maxdeg = c.gs.maxdeg;
-      sl.mindist = 0;
+      whole_slot(c, sl);
     }
   }
   __syncthreads();
@@ -280,6 +284,8 @@ __global__ void k_validate(DGraph g, int* bad) {
 struct DevStats {
   unsigned long long hub;  // largest degree << 32 | ~vertex: the lowest ID on ties
   int nheavy;
+  int linked;              // vertices with edges
+  unsigned firstinv;       // INT_MAX - the smallest of them (0: none)
   unsigned winv;           // INT_MAX - smallest weight (0: no weights)
   int unsorted;
   int asym;
@@ -292,13 +298,18 @@ __global__ void k_degree_stats(DGraph g, int heavy, DevStats* st) {
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
   unsigned long long hub = 0;
-  int nh = 0;
+  int nh = 0, nl = 0;
+  unsigned firstinv = 0;
   double s2 = 0.0;
   for (long long v = tid; v < g.nodes; v += stride) {
     const int b = g.nindex[v], e = g.nindex[v + 1];
     const int d = e - b;
     hub = max(hub, ((unsigned long long)d << 32) | (unsigned)~v);
     nh += d >= heavy;
+    if (d > 0) {
+      ++nl;
+      firstinv = max(firstinv, (unsigned)INT_MAX - (unsigned)v);
+    }
     s2 += (double)d * d;
   }
   unsigned winv = 0;
@@ -311,20 +322,24 @@ __global__ void k_degree_stats(DGraph g, int heavy, DevStats* st) {
     }
   // one set of atomics per block: from every thread they were 0.4 ms on one line
   nh = __reduce_add_sync(0xffffffffu, nh);
+  nl = __reduce_add_sync(0xffffffffu, nl);
+  firstinv = __reduce_max_sync(0xffffffffu, firstinv);
   winv = __reduce_max_sync(0xffffffffu, winv);
   for (int o = 16; o > 0; o >>= 1) {
     hub = max(hub, __shfl_down_sync(0xffffffffu, hub, o));
     s2 += __shfl_down_sync(0xffffffffu, s2, o);
     ws += __shfl_down_sync(0xffffffffu, ws, o);
   }
-  __shared__ int snh[kWarp];
-  __shared__ unsigned swi[kWarp];
+  __shared__ int snh[kWarp], snl[kWarp];
+  __shared__ unsigned swi[kWarp], sfi[kWarp];
   __shared__ unsigned long long shub[kWarp];
   __shared__ double ss2[kWarp], sws[kWarp];
   const int wid = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   if ((threadIdx.x & 31) == 0) {
     shub[wid] = hub;
     snh[wid] = nh;
+    snl[wid] = nl;
+    sfi[wid] = firstinv;
     swi[wid] = winv;
     ss2[wid] = s2;
     sws[wid] = ws;
@@ -334,12 +349,16 @@ __global__ void k_degree_stats(DGraph g, int heavy, DevStats* st) {
   for (int k = 1; k < nwarp; ++k) {
     hub = max(hub, shub[k]);
     nh += snh[k];
+    nl += snl[k];
+    firstinv = max(firstinv, sfi[k]);
     winv = max(winv, swi[k]);
     s2 += ss2[k];
     ws += sws[k];
   }
   atomicMax(&st->hub, hub);
   atomicAdd(&st->nheavy, nh);
+  atomicAdd(&st->linked, nl);
+  atomicMax(&st->firstinv, firstinv);
   atomicMax(&st->winv, winv);
   atomicAdd(&st->sumsq, s2);
   if (g.eweight) atomicAdd(&st->wsum, ws);
@@ -869,6 +888,8 @@ static int compute_stats(i2_graph* g) {
   s.maxdeg = (int)(h.hub >> 32);
   g->hub = (int)~(unsigned)h.hub;
   s.nheavy = h.nheavy;
+  s.linked = h.linked;
+  s.first = h.linked ? INT_MAX - (int)h.firstinv : kInf;
   s.wmin = g->g.eweight && h.winv ? (int)((unsigned)INT_MAX - h.winv) : 1;
   s.symmetric = -1;  // decided on first need (ensure_symmetry)
   const double mean = (double)g->g.edges / (double)g->g.nodes;
@@ -1324,7 +1345,7 @@ static ResidentPlan plan_resident(i2_graph* g, int algo, int mode, int variant, 
   load((const void*)p.start);
   const long long units = (long long)g->g.nodes / 4 + (long long)bm_block_words(g);
   p.start_grid = (int)std::max(1LL, std::min(8LL * sm_count(), units / (4 * kBlock)));
-  const bool frontier = algo == I2_CC && !rp.uf_start;
+  const bool frontier = algo == I2_CC && !rp.whole;
   if (frontier) {
     p.fill = fill_kernel(algo);
     p.fill_grid = grid((const void*)p.fill, 8);
@@ -1603,7 +1624,7 @@ int run_traversal(i2_graph* g, int algo, int src, const int* srcs_host, int nsrc
     rp.then_variant = o.then_variant;
   }
   // union-find from the first iteration: fixed, or by the selectors' rule
-  rp.uf_start = algo == I2_CC && ((mode == 0 && variant == kUnionFind) ||
+  rp.whole = algo == I2_CC && ((mode == 0 && variant == kUnionFind) ||
                                   ((mode == 1 || mode == 2) && ((rp.allowed >> kUnionFind) & 1) &&
                                    union_find_pays(g->g.nodes, g->gs.avgdeg)));
   ExecEntry* ex = nullptr;

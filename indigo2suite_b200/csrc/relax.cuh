@@ -1822,7 +1822,10 @@ __device__ __forceinline__ bool body_mis(const Ctx& c, H& S, Stage& s) {
   block_prologue(c);
   const int i = S.iter;
   const int cur = i % 3, nxt = (i + 1) % 3, old = (i + 2) % 3;
-  const int n = slot_size(S.slot[cur].packed);
+  // the first iteration may take every vertex, without a list (a vertex without
+  // neighbours joins the set at once)
+  const bool all = i == 0 && S.whole;
+  const int n = all ? c.g.nodes : slot_size(S.slot[cur].packed);
   const int active = (int)min((long long)gridDim.x, ((long long)n + kBlock - 1) / kBlock);
   if (blockIdx.x >= active) return idle_epilogue(c, S, s, i, cur, nxt, old);
   stage_init(s);
@@ -1830,9 +1833,6 @@ __device__ __forceinline__ bool body_mis(const Ctx& c, H& S, Stage& s) {
   acc_init(a);
   __syncthreads();
   const int* wl = c.wl[cur];
-  // the first iteration's frontier may be every vertex, without a list (a
-  // vertex without neighbours joins the set at once)
-  const bool all = i == 0 && n == c.g.nodes;
   const unsigned* cursor = c.woff[cur];
   volatile int* st = c.dist;
   const int* __restrict__ nl = c.g.nlist;
