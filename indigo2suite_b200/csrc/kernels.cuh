@@ -35,7 +35,7 @@ KernelFn relax_fn(int v, bool select, bool wide) {
 
 template <int ALG>
 KernelFn dispatch_fn(bool wide) {
-  return wide ? relax_dispatch<ALG, I2_FIXED_MIN_BLOCKS> : relax_dispatch<ALG>;
+  return wide ? relax_dispatch<ALG, true> : relax_dispatch<ALG>;
 }
 
 template <int ALG>
@@ -43,7 +43,7 @@ KernelFn resident_fn(int v, bool wide) {
   switch (v) {
     case kVPThread: return relax_resident<ALG, kVPThread>;
     case kVPWarp: return relax_resident<ALG, kVPWarp>;
-    case kVPCta: return wide ? relax_resident<ALG, kVPCta, false, I2_FIXED_MIN_BLOCKS> : relax_resident<ALG, kVPCta>;
+    case kVPCta: return wide ? relax_resident<ALG, kVPCta, false, true> : relax_resident<ALG, kVPCta>;
     case kVPBlock: return relax_resident<ALG, kVPBlock>;
     case kPullFrontier: return relax_resident<ALG, kPullFrontier>;
     case kPullTopo: return relax_resident<ALG, kPullTopo>;
@@ -54,7 +54,7 @@ KernelFn resident_fn(int v, bool wide) {
       return nullptr;
   }
   // per-iteration pick
-  return wide ? relax_resident<ALG, -1, false, I2_FIXED_MIN_BLOCKS> : relax_resident<ALG, -1>;
+  return wide ? relax_resident<ALG, -1, false, true> : relax_resident<ALG, -1>;
 }
 
 }  // namespace i2

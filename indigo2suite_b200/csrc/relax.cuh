@@ -2160,19 +2160,23 @@ __device__ __forceinline__ bool run_body(const Ctx& c, H& S, AnyShared<DEFER>& s
 }
 
 // VAR >= 0: that style every iteration; VAR < 0: the style picked for each
-// iteration by the previous one (heuristic or learned selector).
-template <int ALG, int VAR, bool DEFER = false,
-          int MINB = (VAR < 0                 ? I2_SEL_MIN_BLOCKS
-                      : VAR == kVPCta     ? I2_EB_MIN_BLOCKS
-                      : VAR == kUnionFind ? I2_UF_MIN_BLOCKS
-                                          : I2_FIXED_MIN_BLOCKS)>
+// iteration by the previous one (heuristic or learned selector). WIDE: the form
+// for more resident blocks (selectors: the largest graphs; edge-balanced push:
+// graphs of skewed degrees, with long tiles too).
+template <int VAR, bool WIDE>
+constexpr int kResidentMinBlocks = WIDE                ? I2_FIXED_MIN_BLOCKS
+                                   : VAR < 0           ? I2_SEL_MIN_BLOCKS
+                                   : VAR == kVPCta     ? I2_EB_MIN_BLOCKS
+                                   : VAR == kUnionFind ? I2_UF_MIN_BLOCKS
+                                                       : I2_FIXED_MIN_BLOCKS;
+template <int ALG, int VAR, bool DEFER = false, bool WIDE = false, int MINB = kResidentMinBlocks<VAR, WIDE>>
 __global__ void __launch_bounds__(kBlock, MINB) relax_resident(const __grid_constant__ Ctx c) {
   __shared__ AnyShared<DEFER> sh;
   // the selectors' form for more blocks runs on the largest graphs only
   static_assert(kWideSelectorNodes > kMaxTrainedNodes, "no network in the wide forms");
-  using Pick = typename std::conditional<(MINB > I2_SEL_MIN_BLOCKS), RuleHead, SelectHead>::type;
+  using Pick = typename std::conditional<WIDE, RuleHead, SelectHead>::type;
   __shared__ typename std::conditional<(VAR < 0), Pick, FixedHead>::type S;
-  constexpr bool LONG = DEFER || (VAR == kVPCta && MINB == I2_FIXED_MIN_BLOCKS);  // skewed graphs' forms
+  constexpr bool LONG = DEFER || (VAR == kVPCta && WIDE);  // skewed graphs' forms
   // thread 0's: barrier generation, whether to go on, the test hook (kept in
   // shared memory: the bodies have no register to spare)
   __shared__ unsigned s_gen;
@@ -2184,13 +2188,13 @@ __global__ void __launch_bounds__(kBlock, MINB) relax_resident(const __grid_cons
     s_hold = c.ctl->hold;
   }
   __syncthreads();
-  // Blocks of this traversal have given up already: end the loop of a graph it
-  // may run in. (Measured: without this branch the compiler hoists into the
-  // bodies' registers, 100 instead of 60 bytes of spills in the near/far form,
-  // RMAT-22 2,047 instead of 1,933 us.)
+  // Blocks of this traversal have given up already, before this one began: it
+  // leaves and says so, like a block whose wait ran out. (With a bare return here
+  // nvcc 12.9 keeps the kernel's parameters in registers across the loop and
+  // spills them in the bodies: 88 instead of 56 bytes in the near/far form, 92
+  // instead of 24 in vp_thread's.)
   if (!s_ok) {
-    if (blockIdx.x == 0 && threadIdx.x == 0 && c.use_loop)
-      cudaGraphSetConditional((cudaGraphConditionalHandle)c.loop_h, 0u);
+    if (threadIdx.x == 0) atomicOr(&c.ctl->status, kStatusStall);
     return;
   }
   for (;;) {
@@ -2214,10 +2218,11 @@ __global__ void __launch_bounds__(kBlock, MINB) relax_resident(const __grid_cons
   }
 }
 
-template <int ALG, int MINB = I2_SEL_MIN_BLOCKS>
-__global__ void __launch_bounds__(kBlock, MINB) relax_dispatch(const __grid_constant__ Ctx c) {
+template <int ALG, bool WIDE = false>
+__global__ void __launch_bounds__(kBlock, WIDE ? I2_FIXED_MIN_BLOCKS : I2_SEL_MIN_BLOCKS)
+    relax_dispatch(const __grid_constant__ Ctx c) {
   __shared__ AnyShared<> sh;
-  __shared__ typename std::conditional<(MINB > I2_SEL_MIN_BLOCKS), RuleHead, SelectHead>::type S;
+  __shared__ typename std::conditional<WIDE, RuleHead, SelectHead>::type S;
   load_head(c, S);
   __syncthreads();
   switch (S.variant) {
