@@ -109,9 +109,12 @@ struct MinOp {
 // and cudaFree (16 M keys: 3.4 of 4.6 ms); what is beyond them (tens of GB at
 // RMAT scale 26) is a plain allocation, which the pool never keeps. The parts of
 // a build (`outer`: the scratch that is alive around this one) share the bytes.
+// Buffers of up to kSmall (counters, the sorts' temporaries) come from the pool
+// whatever the large ones took: as plain allocations they cost a build at the
+// bound 3.6 ms (RMAT-22, whose two key buffers are 2 GB: 13.7 -> 17.3 ms).
 struct Scratch {
   static constexpr int kMax = 16;
-  static constexpr size_t kPooled = (size_t)2 << 30;
+  static constexpr size_t kPooled = (size_t)2 << 30, kSmall = (size_t)32 << 20;
   explicit Scratch(Scratch* outer = nullptr) : total(outer ? outer->total : &own) {}
   Scratch(const Scratch&) = delete;
   Scratch& operator=(const Scratch&) = delete;
@@ -121,7 +124,7 @@ struct Scratch {
     if (n == kMax) return cudaErrorMemoryAllocation;  // more buffers than one build takes
     bytes = bytes > 0 ? bytes : 1;
     void* q = nullptr;
-    const bool pool = *total + bytes <= kPooled;
+    const bool pool = bytes <= kSmall || *total + bytes <= kPooled;
     cudaError_t e = pool ? dev_alloc(&q, bytes) : cudaMalloc(&q, bytes);
     if (e == cudaErrorMemoryAllocation && !pool) {  // what the pool holds unused may be enough
       cudaGetLastError();
