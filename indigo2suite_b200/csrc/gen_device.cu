@@ -20,36 +20,10 @@
 #include <cub/device/device_select.cuh>
 #include "engine.h"
 #include "gen_rng.h"
+#include "key_bits.h"
 #include "list_walk.h"
 
 namespace i2 {
-
-// Keys of the vertex pairs of a graph of n vertices: `shift` bits hold an ID
-// (those of n, which marks dropped pairs), and keys sort over `bits` bits.
-struct KeyBits {
-  int shift;
-  int bits;
-  unsigned long long drop;
-  __host__ __device__ unsigned long long key(unsigned long long u, unsigned long long v) const {
-    return (u << shift) | v;
-  }
-  __host__ __device__ unsigned long long hi(unsigned long long k) const { return k >> shift; }
-  __host__ __device__ unsigned long long lo(unsigned long long k) const { return k & ((1ull << shift) - 1); }
-};
-
-static int bit_length(unsigned long long x) {
-  int b = 0;
-  for (; x; x >>= 1) ++b;
-  return b;
-}
-
-static KeyBits key_bits(int n) {
-  KeyBits k;
-  k.shift = std::max(1, bit_length((unsigned long long)n - 1));
-  k.bits = k.shift + bit_length((unsigned long long)n);
-  k.drop = (unsigned long long)n << k.shift;
-  return k;
-}
 
 __global__ void k_rmat_keys(uint64_t seed, int scale, RmatThresholds t, RmatPerm p, long long samples, int n,
                             KeyBits kb, unsigned long long* keys) {

@@ -6,12 +6,7 @@
 // the array. Positions are unsigned here; with ends of at most 2^31 - 1 and
 // steps far below 2^31 they never wrap.
 #pragma once
-
-#ifdef __CUDACC__
-#define I2_HOST_DEVICE __host__ __device__ __forceinline__
-#else
-#define I2_HOST_DEVICE inline
-#endif
+#include "host_device.h"
 
 namespace i2 {
 
