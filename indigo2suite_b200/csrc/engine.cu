@@ -1050,13 +1050,15 @@ static bool wide_form(const i2_graph* g, int variant) {
 
 // Most resident blocks per SM of a style's kernel on this graph. The
 // edge-balanced push of BFS and SSSP takes 4 of the 5 it is compiled for on
-// sparse graphs of even degrees (average below 6: grids, road networks), where
-// the blocks wait on the same few cache lines and, from 2^25 vertices, push one
-// another's out of L2. 5 / 4 blocks: SSSP grid 7000^2 70.5 / 65.8 ms, 6000^2
-// 52.2 / 48.6, 2000^2 4.47 / 4.31, ER 4 x 10^7 with 4 entries a vertex 21.9 /
-// 21.2, BFS grid 2000^2 1,709 / 1,600 us; ER with 8 entries a vertex gains
-// nothing (8 x 10^6 BFS 918 / 952 us) and CC, whose first iteration holds every
-// vertex, loses (ER 4 x 10^7 with 4 entries 39.8 / 41.9 ms).
+// sparse graphs of even degrees (average below 6: grids, road networks) of 2^24
+// vertices and more, where the blocks push one another's lines out of L2. 5 / 4
+// blocks: SSSP grid 7000^2 70.5 / 65.8 ms, 6000^2 52.2 / 48.6, 5000^2 28.7 / 26.8,
+// ER 4 x 10^7 with 4 entries a vertex 21.9 / 21.2, BFS grid 6000^2 5.76 / 5.56. ER
+// with 8 entries a vertex gains nothing (2^24 BFS 2.35 / 2.40) and CC, whose first
+// iteration holds every vertex, loses (ER 4 x 10^7 with 4 entries 39.8 / 41.9).
+// Smaller sparse graphs would gain too (grid 2000^2 SSSP 4.47 / 4.31, BFS 1.71 /
+// 1.60); there the line is with the learned selector, which would then lose to the
+// rule on grids (its picks are from times at 5 blocks).
 // Union-find takes about one block per SM for every 2^11 vertices an SM has, 8
 // chunks a warp: more warps link trees that the others have not joined yet, and
 // meet at the same roots. us, 1 / 2 / 3 / 4 / 6 blocks: RMAT-17 110 / 122 / 153 /
@@ -1071,7 +1073,8 @@ static int style_blocks(const i2_graph* g, int algo, int variant) {
     const long long blocks = (g->g.nodes + per_block * sms / 2) / (per_block * sms);
     return (int)std::min<long long>(std::max(1LL, blocks), std::min(g->blocks_per_sm, I2_UF_MIN_BLOCKS));
   }
-  const bool sparse = variant == kVPCta && (algo == I2_BFS || algo == I2_SSSP) && g->gs.degcv <= 1.f && g->gs.avgdeg < 6.f;
+  const bool sparse = variant == kVPCta && (algo == I2_BFS || algo == I2_SSSP) && g->g.nodes >= (1 << 24) &&
+                      g->gs.degcv <= 1.f && g->gs.avgdeg < 6.f;
   return sparse ? std::min(g->blocks_per_sm, 4) : g->blocks_per_sm;
 }
 
