@@ -1029,8 +1029,15 @@ constexpr long long kUnionFindKernelNodes = 1LL << 22;
 // the whole traversal (no parameters, or a graph larger than any it was trained
 // on) the traversal is the rule's, by the rule's kernels (SSSP on a grid of
 // 6000^2, ms: 52.4 as the rule's, 59.7 in the selectors' kernel).
-static bool learned_here(const i2_graph* g) {
-  return mlp_device_params() && (long long)g->g.nodes <= kMaxTrainedNodes;
+// SSSP on graphs of skewed degrees is the rule's too: the network mostly picks
+// the rule's style there, whose own kernel has more blocks and the long tiles, and
+// where it picks another it loses. us, by the network / the rule: RMAT-20 786 / 658,
+// RMAT-18 307 / 282, RMAT-12 184 / 144, RMAT-20 with edge factor 4 2,942 / 385, 32
+// 1,282 / 944, power-law pairs on 10^6 vertices 1,462 / 987; of 33 graphs of 2^10 to
+// 2^21 vertices none was faster by the network.
+static bool learned_here(const i2_graph* g, int algo) {
+  return mlp_device_params() && (long long)g->g.nodes <= kMaxTrainedNodes &&
+         !(algo == I2_SSSP && g->gs.degcv > 1.f);
 }
 
 // Whether the selectors run in the form compiled for more resident blocks.
@@ -1543,7 +1550,7 @@ int run_traversal(i2_graph* g, int algo, int src, const int* srcs_host, int nsrc
   }
   int mode = 0, variant = o.variant;
   if (variant == I2_AUTO_HEURISTIC) mode = 1;
-  else if (variant == I2_AUTO_LEARNED) mode = learned_here(g) ? 2 : 1;
+  else if (variant == I2_AUTO_LEARNED) mode = learned_here(g, algo) ? 2 : 1;
   else if (variant < 0 || variant >= kNumVariants) return I2_ERR_ARG;
   if (o.then_at < 0) return I2_ERR_ARG;
   if (o.then_at > 0) {  // a fixed switch of style: per-iteration dispatch
