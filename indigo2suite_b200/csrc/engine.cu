@@ -283,8 +283,7 @@ __global__ void k_validate(DGraph g, int* bad) {
 
 struct DevStats {
   unsigned long long hub;  // largest degree << 32 | ~vertex: the lowest ID on ties
-  int nheavy;
-  int linked;              // vertices with edges
+  unsigned long long counts;  // heavy vertices << 32 | vertices with edges
   unsigned firstinv;       // INT_MAX - the smallest of them (0: none)
   unsigned winv;           // INT_MAX - smallest weight (0: no weights)
   int unsorted;
@@ -356,10 +355,10 @@ __global__ void k_degree_stats(DGraph g, int heavy, DevStats* st) {
     ws += sws[k];
   }
   atomicMax(&st->hub, hub);
-  atomicAdd(&st->nheavy, nh);
-  atomicAdd(&st->linked, nl);
-  atomicMax(&st->firstinv, firstinv);
-  atomicMax(&st->winv, winv);
+  atomicAdd(&st->counts, ((unsigned long long)(unsigned)nh << 32) | (unsigned)nl);
+  // most blocks find these two no further on than others have
+  if (firstinv > *(volatile unsigned*)&st->firstinv) atomicMax(&st->firstinv, firstinv);
+  if (winv > *(volatile unsigned*)&st->winv) atomicMax(&st->winv, winv);
   atomicAdd(&st->sumsq, s2);
   if (g.eweight) atomicAdd(&st->wsum, ws);
 }
@@ -887,9 +886,9 @@ static int compute_stats(i2_graph* g) {
   s.edges = g->g.edges;
   s.maxdeg = (int)(h.hub >> 32);
   g->hub = (int)~(unsigned)h.hub;
-  s.nheavy = h.nheavy;
-  s.linked = h.linked;
-  s.first = h.linked ? INT_MAX - (int)h.firstinv : kInf;
+  s.nheavy = (int)(h.counts >> 32);
+  s.linked = (int)(unsigned)h.counts;
+  s.first = s.linked ? INT_MAX - (int)h.firstinv : kInf;
   s.wmin = g->g.eweight && h.winv ? (int)((unsigned)INT_MAX - h.winv) : 1;
   s.symmetric = -1;  // decided on first need (ensure_symmetry)
   const double mean = (double)g->g.edges / (double)g->g.nodes;
@@ -1342,7 +1341,8 @@ static ResidentPlan plan_resident(i2_graph* g, int algo, int mode, int variant, 
     return it->second;
   };
   const auto load = [g](const void* fn) {
-    if (!g->grids.emplace(fn, 0).second) return;
+    if (g->grids.count(fn)) return;
+    g->grids.emplace(fn, 0);
     cudaFuncAttributes a;
     if (cudaFuncGetAttributes(&a, fn) != cudaSuccess) cudaGetLastError();  // its launch reports it
   };
