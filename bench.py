@@ -839,7 +839,7 @@ def main():
                     help="rmat26 workload: vertex numbering BFS, SSSP and CC run under (degree: a copy "
                          "renumbered by descending degree, results in original IDs)")
     ap.add_argument("--loop", choices=["graph", "host", "relaunch"], default="graph",
-                    help="graph: one CUDA graph whose resident kernel runs every iteration (default); "
+                    help="graph: a start kernel and one resident launch that runs every iteration (default); "
                          "host: one host launch per iteration; relaunch: one launch per iteration "
                          "from the graph's device-side loop")
     args = ap.parse_args()

@@ -131,12 +131,13 @@ typedef struct {
 typedef struct {
   int iter;
   int variant;
-  int size;                /* light frontier entries consumed */
-  int hsize;               /* heavy frontier entries consumed */
+  int size;                /* frontier vertices consumed (those with edges) */
+  int hsize;               /* the heavy ones among them */
   unsigned long long edges;/* frontier edges consumed */
   int maxdeg;
   int mindist;
-  long long visited;       /* vertices reached before this launch */
+  long long visited;       /* vertices reached by the end of this launch (MIS: all of
+                              them, and once more each vertex decided) */
   unsigned long long t_ns; /* launch duration (device timer) */
   float feat[16];          /* selector features of the consumed frontier */
   int kind;                /* SSSP near/far ordering: 0 relaxation, 1 move from the far pile,
@@ -270,8 +271,8 @@ int i2_cc(i2_graph* g, int* label, const i2_opts* opts, i2_report* rep);
    and GPUmis_edge, include/mis_edge_cuda.h:54): status[v] = 1 in the set, 2 not,
    the set the reference's deterministic CUDA MIS variants converge to (priority
    hash(v + 712313887) as int, ties to the larger ID). Symmetric graphs only
-   (I2_ERR_UNSUPPORTED otherwise); opts->variant is ignored (one style: a warp
-   per frontier vertex). */
+   (I2_ERR_UNSUPPORTED otherwise); opts->variant is ignored (one style: each
+   undecided vertex keeps a cursor into its list). */
 int i2_mis(i2_graph* g, int* status, const i2_opts* opts, i2_report* rep);
 /* Same, with the result left in (or copied to) DEVICE memory; out_dev may be NULL
    to keep the result only inside the engine. src is ignored for I2_CC and I2_MIS. */

@@ -4,10 +4,9 @@
 // vertices at offset voff[k], its CSR entries at offset eoff[k]). A traversal
 // of the union from one source per graph is the same as one traversal per
 // graph: no edge crosses two graphs, so every graph reaches the same fixed point
-// as on its own. One persistent relax launch per iteration then drains frontier
-// chunks of all graphs from the same device-side chunk counter, and the whole
-// loop is one CUDA graph, instead of one launch sequence (with a host round trip
-// per iteration) per graph.
+// as on its own. The relax kernels then drain the frontier work of all graphs at
+// once, in the one resident launch of a traversal, instead of one launch sequence
+// (with a host round trip per iteration) per graph.
 #include <cuda_runtime.h>
 #include <cstring>
 #include <vector>

@@ -15,8 +15,13 @@
 //                        the frontier's edges form one index space [0, edges),
 //     hwl[s][0..hsize)   the subset of degree >= the heavy threshold, with
 //     htoff[s][0..hsize) the exclusive prefix of their tile counts,
-//     bm[s]              a bitmap with the bits of F_i set (vertices of
-//                        degree 0 are never kept: they have nothing to relax);
+//     bm[s]              a bitmap with the bits of F_i set. Other bits may be
+//                        set too, of vertices without edges only, and may
+//                        outlive their iteration: the edge-balanced push leaves
+//                        the bit of such a vertex it lowers, which keeps its
+//                        visit counted once, and a slot cleared by its list
+//                        never sees it. Readers that relax from the bitmap find
+//                        no edges there; the list never holds such a vertex;
 //   every vertex outside F_i has already relaxed all of its out-edges against
 //   the current dist[]. Iteration i propagates at least F_i and builds F_{i+1}
 //   in slot (i+1) % 3 from every vertex whose value it lowered. It also clears
@@ -216,11 +221,15 @@ struct Ctl : CtlHead {
   unsigned long long reached[2];  // reached vertices and the sum of their degrees (k_reached)
 };
 
-// Union-find CC pays on graphs of 2^19 vertices or more, or of average degree
-// below 6 (measured 2.5-23x faster than the best propagation style on RMAT,
-// ER and grid graphs of 2^22 vertices and more; propagation up to 1.7x faster
-// on RMAT and ER of 2^18 vertices with higher degrees). Both selectors take it
-// before the first iteration on symmetric graphs.
+// Where the selectors take union-find for CC, before the first iteration, on
+// symmetric graphs: 2^19 vertices or more, or an average degree below 6. The line
+// was drawn for an earlier union-find, to which propagation was up to 1.7x faster
+// on RMAT and ER of 2^18 vertices with higher degrees. With links by climbing and
+// blocks by the graph's size, union-find by name is the faster one below the line
+// too (us, union-find / what the selectors run: RMAT-12 46 / 95, RMAT-16 111 / 129,
+// RMAT-18 114 / 185, ER 60,000 128 / 183, ER 300,000 122 / 250): the line has not
+// been moved. Above it, against the edge-balanced push: RMAT-22 186 / 1,894, ER
+// 2 x 10^6 199 / 949, grid 4096^2 654 / 36,000 (pull_topo 31,764).
 __host__ __device__ inline bool union_find_pays(long long nodes, float avgdeg) {
   return nodes >= (1LL << 19) || avgdeg < 6.f;
 }

@@ -796,7 +796,11 @@ static void ctl_host_put(Ctl* c) {
 // Results of up to kStageInts values go to the caller through a pinned block,
 // copied with the report before its one wait for the device; a copy into
 // pageable memory waits by itself after that. Blocks of freed graphs are kept
-// for the next ones, at most kStageKept of them.
+// for the next ones, at most kStageKept of them. Host BFS call, us, pinned /
+// pageable: ER 1,000 106 / 115, 16,000 143 / 154, 65,000 175 / 186, 131,072 208 /
+// 225, 262,144 275 / 288, 524,288 412 / 380, 10^6 631 / 545 (the host's copy out
+// of the block is then the longer one). The limit keeps a graph's block at 256
+// KB; up to 2^18 values would gain the same 10-16 us for four times that.
 constexpr int kStageInts = 1 << 16;
 constexpr size_t kStageKept = 16;
 static std::mutex g_stage_mu;
@@ -1021,7 +1025,10 @@ static int ensure_symmetry(i2_graph* g) {
 // vertex's out-list as its in-list (symmetric graphs only), the edge sweeps
 // need sp[], and union-find computes CC labels only.
 // Smallest graph (vertices) on which the selectors' union-find CC runs as
-// union-find's own kernel (run_traversal).
+// union-find's own kernel (run_traversal). The line was drawn before that kernel
+// chose its blocks by the graph's size; below it, us, own kernel / the selectors':
+// RMAT-20 145 / 168, ER 600,000 159 / 176, ER 2 x 10^6 199 / 200, grid 300^2 85 /
+// 135, 1000^2 135 / 141, 2000^2 231 / 268. It has not been moved.
 constexpr long long kUnionFindKernelNodes = 1LL << 22;
 
 // Whether the learned selector picks styles here. Where it defers to the rule for
@@ -1172,7 +1179,11 @@ static int budget_shift(const i2_graph* g) {
 // degree-ordered copies among them), where the first vertices' links already
 // tie most of the graph to the smallest IDs. First launch, us, ascending /
 // spread, on degree-ordered copies: RMAT 10^6 33 / 294, 9 x 10^6 123 / 362,
-// 25 x 10^6 253 / 511.
+// 25 x 10^6 253 / 511. Whole run: degree-ordered RMAT-18 84 / 174, RMAT-20 140 /
+// 336; pairs whose ends' IDs fall like a power p of a uniform number, 2 x 10^6
+// vertices: p = 4 154 / 290, p = 2 187 / 258, p = 1.7 194 / 355, p = 1.3 289-382 /
+// 187-289. A hub in the first 64th by chance (RMAT-16 to 20, within the noise;
+// RMAT-20 up to 1.4x for spread) is why the line lies as low as 1/256.
 static bool union_in_order(const i2_graph* g) {
   return g->gs.avgdeg < 6.f || g->hub < g->g.nodes / 256;
 }
@@ -1561,15 +1572,15 @@ int run_traversal(i2_graph* g, int algo, int src, const int* srcs_host, int nsrc
   // 2^26 CSR entries or more, from one source: both selectors run the
   // edge-balanced push in the budgeted near/far ordering for the whole
   // traversal (the per-iteration styles cannot take part in its moves and
-  // trims). Measured against plain frontier-driven relaxation: 1.13x faster on
-  // RMAT-22 and 1.31x on RMAT-26; 5-28% slower on ER, grid and RMAT graphs of
-  // up to 2^21 vertices and 2^25 entries, which keep the per-iteration rule.
+  // trims). us, plain / budgeted: RMAT-22 2,120 / 1,901, RMAT-23 4,367 / 3,403,
+  // RMAT-26 in degree order 45,829 / 29,035, RMAT-21 1,144 / 1,131; but RMAT-20 654 /
+  // 772, RMAT-18 283 / 328, ER 2^22 2,405 / 2,787, grid 2048^2 4,242 / 4,895, which
+  // keep the per-iteration rule. (At a budget of 10^6 edges ER 2^22 takes 2,027 and
+  // 2^23 3,741 for 4,860: the rule has no budget for such graphs.)
   // CC on a symmetric graph of 2^22 vertices or more where union-find pays:
   // both selectors take it before the first iteration, so it runs as
-  // union-find's own kernel (grid 4096²: 1.37-1.47 ms against 1.79-1.89 in the
-  // selectors' kernel at 4 blocks per SM). On smaller graphs the selectors'
-  // kernel, with its 64 registers, measured faster (ER 2^20: 0.25 against
-  // 0.33 ms; grid 2^18: 0.14 against 0.22-0.28).
+  // union-find's own kernel; on smaller graphs in the selectors' kernel
+  // (kUnionFindKernelNodes).
   if (algo == I2_CC && (mode == 1 || mode == 2) && (long long)g->g.nodes >= kUnionFindKernelNodes) {
     st = ensure_symmetry(g);
     if (st) return st;

@@ -11,18 +11,14 @@ namespace i2 {
 // ---------------------------------------------------------------------------
 // Selection of the next variant.
 
-// Fixed frontier-size rule: union-find for CC on symmetric graphs (measured
-// 2.5-23x faster than the best propagation style on RMAT, ER and grid graphs
-// of 2^22 vertices and more, within 2x either way on 2^18), bottom-up pull for BFS levels whose frontier
-// carries more than 1/16 of the edges (direction-optimising BFS), otherwise the
-// edge-balanced push, which measured fastest of the push styles on every
-// family tried.
+// Fixed frontier-size rule: union-find for CC on symmetric graphs where
+// union_find_pays (common.cuh, with both sides measured), bottom-up pull for BFS
+// levels whose frontier carries more than 1/16 of the edges
+// (direction-optimising BFS), otherwise the edge-balanced push, which measured
+// fastest of the push styles on every family tried.
 // Union-find replaces the whole traversal, so it is a choice made once, before
 // the first iteration, by both selectors; the per-iteration picks are among the
-// propagation styles. On graphs below 2^19 vertices with an average degree of
-// 6 or more (RMAT and ER of 2^18 vertices) propagation measured up to 1.7x
-// faster than union-find; on grids and on every graph of 2^20 vertices and
-// more, union-find was the fastest.
+// propagation styles.
 static __device__ bool union_find_first(const GStats& gs, int algo, int allowed, int next_iter) {
   return algo == kCC && next_iter == 0 && ((allowed >> kUnionFind) & 1) && union_find_pays(gs.nodes, gs.avgdeg);
 }

@@ -947,7 +947,7 @@ struct EpiStage {
 };
 
 // Resident blocks per SM that the edge-balanced kernels are compiled for: 5
-// leaves them 48 registers, no spills but 48 bytes in the near/far form (6: 40
+// leaves them 48 registers, no spills but 56 bytes in the near/far form (6: 40
 // registers, 192 bytes there). ER 2M SSSP 1,318 us (6 blocks 1,367; 4 blocks
 // 1,323), RMAT-22 near/far 2,007 (2,238; 2,057), RMAT-25 ordered 16,213
 // (17,455; 17,664); 3 edges per lane at 5 and 4 blocks 1,396 and 1,342, 2,025
@@ -955,7 +955,9 @@ struct EpiStage {
 #ifndef I2_EB_MIN_BLOCKS
 #define I2_EB_MIN_BLOCKS 5
 #endif
-// ... and the other fixed styles' kernels, and the selectors' on the largest graphs.
+// ... and the other fixed styles' kernels, and the wide forms. The other styles at
+// 5 blocks, us, against 6: ER 2 x 10^6 vp_warp SSSP 6,877 / 6,000, RMAT-18 vp_block
+// CC 1,518 / 840, RMAT-20 push_topo SSSP 11,440 / 10,500.
 #ifndef I2_FIXED_MIN_BLOCKS
 #define I2_FIXED_MIN_BLOCKS 6
 #endif
@@ -1498,7 +1500,7 @@ __device__ __forceinline__ bool body_pull(const Ctx& c, H& S, Stage& s) {
 // smallest ID of a component is therefore never linked and ends as the root of
 // the whole component; the compress launch sets every label to its root. The
 // result is the minimum-ID labelling that label propagation converges to,
-// reached from any propagation state in two launches.
+// reached from any propagation state in three launches (below).
 
 // Reads of parents may be served from this SM's L1 and so be stale: a stale
 // parent is still an ancestor (links are never undone), and a vertex wrongly
@@ -1536,10 +1538,13 @@ __device__ __forceinline__ void uf_union(int* p, int a, int b) {
   }
 }
 
-// The same without finding the roots first: pa and pb are ancestors of a and b;
-// climb from the larger of the two until the ancestors meet or the larger is a
-// root, which is then linked below the smaller. Two vertices whose parents are
-// the same are done after those two reads. Returns an ancestor of both.
+// The same without finding the roots first (the link step of Sutton et al.,
+// "Optimizing parallel graph connectivity computation via subgraph sampling",
+// IPDPS 2018, with the path halved on the way and an early end where the larger's
+// parent is the smaller): pa and pb are ancestors of a and b; climb from the
+// larger of the two until the ancestors meet or the larger is a root, which is
+// then linked below the smaller. Two vertices whose parents are the same are done
+// after those two reads. Returns an ancestor of both.
 __device__ __forceinline__ int uf_climb(int* p, int pa, int pb) {
   while (pa != pb) {
     const int high = max(pa, pb), low = min(pa, pb);
@@ -1573,7 +1578,10 @@ __device__ __forceinline__ void uf_edge(int* p, int v, int u, bool climb) {
 
 // List length from which launch 1 gives a vertex to the whole block. (One thread
 // per vertex left the hubs outside the largest tree, as in a batch of RMAT
-// graphs, to one thread each: 23 graphs of 10^3 to 10^6 vertices 16,181 us, now 969.)
+// graphs, to one thread each: 23 graphs of 10^3 to 10^6 vertices 16,181 us, now
+// 751.) From 512 / 2,048 / 8,192 entries, us: that batch 680 / 751 / 852, 23 RMAT
+// graphs 774 / 829 / 1,118, 48 graphs of up to 10^5 vertices 325 / 367 / 379;
+// single RMAT graphs the same.
 constexpr int kUfBlockDegree = 2048;
 
 // Neighbours each vertex is linked with before the largest tree is sampled.
@@ -1770,12 +1778,17 @@ __device__ __forceinline__ bool body_union(const Ctx& c, H& S, Stage& s) {
 // kMisBlockDegree entries or more take the whole block after the warps are done.
 // The first iteration takes every vertex without a list (building one was 60 of
 // 195 us on RMAT 3 x 10^5), and each warp stages its own waiting vertices. RMAT
-// with 1,000,003 vertices 2,625-3,129 -> 468-560 us, ER 10^6 796 -> 175, grid
+// with 1,000,003 vertices 2,625-3,129 -> 396-587 us, ER 10^6 796 -> 175, grid
 // 10^6 699 -> 119; the form before, a warp per vertex that rescanned the list in
 // every iteration, left a hub to one warp (2,122 us of its first iteration).
 enum { kMisNone, kMisWait, kMisJoin, kMisLeave, kMisMore };  // what an iteration finds for a vertex
-constexpr int kMisProbe = 16;          // entries a thread scans (or writes) by itself
-constexpr int kMisBlockDegree = 2048;  // entries from which the whole block does
+// Entries a thread scans (or writes) by itself: 8 / 16 / 32, us: RMAT-22 1,902 /
+// 1,776 / 1,730, RMAT 1,000,003 394 / 396 / 411, ER 10^6 180 / 174 / 173, ER with 64
+// entries a vertex 235 / 233 / 242.
+constexpr int kMisProbe = 16;
+// Entries from which the whole block does: 512, 2,048 and 8,192 within 1% on the
+// same graphs (after the first iteration few long lists are scanned far).
+constexpr int kMisBlockDegree = 2048;
 
 // Outcome of `count` (<= 4) consecutive entries from k on, loaded together:
 // bit r of *wait: entry r outranks v and is undecided; returns whether one
