@@ -10,10 +10,15 @@
 
 namespace i2 {
 
-// f(j) for the positions begin + first, + step, + 2 step, ... below end.
+// f(j) for the positions begin + first, + step, + 2 step, ... below end. Counted,
+// not compared with the end: a loop over unsigned positions may wrap as far as the
+// compiler knows, and it would then not issue the loads of several steps together
+// (union-find on a star whose hub comes last, us: 64 by comparison, 54 counted).
 template <class F>
 I2_HOST_DEVICE void walk_list(unsigned begin, unsigned end, unsigned first, unsigned step, F f) {
-  for (unsigned j = begin + first; j < end; j += step) f(j);
+  const unsigned from = begin + first;
+  const unsigned n = from < end ? (end - from + step - 1) / step : 0;
+  for (unsigned i = 0; i < n; ++i) f(from + i * step);
 }
 
 // A group of `width` threads reads a list in windows of 4 * width entries,

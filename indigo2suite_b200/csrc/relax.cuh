@@ -1244,8 +1244,8 @@ __device__ __forceinline__ bool body_edge_balanced(const Ctx& c, H& S, EBSharedT
 #pragma unroll
         for (int r = 0; r < kEdgesPerThread; ++r) {
           ok[r] = e0 + lane + r * kWarp < e1;
-          nv[r] = ok[r] ? ld_adj(nl + (b + r * kWarp)) : 0;
-          wv[r] = Op<ALG>::kWeighted && ok[r] ? ld_adj(ew + (b + r * kWarp)) : 0;
+          nv[r] = ok[r] ? ld_adj(nl + b + r * kWarp) : 0;
+          wv[r] = Op<ALG>::kWeighted && ok[r] ? ld_adj(ew + b + r * kWarp) : 0;
           du[r] = d;
         }
 #pragma unroll
@@ -1335,7 +1335,7 @@ __device__ __forceinline__ bool body_push_topo(const Ctx& c, H& S, Stage& s) {
   const int V = c.g.nodes;
   for (long long base = (long long)blockIdx.x * kBlock; base < V; base += (long long)gridDim.x * kBlock) {
     const int v = (int)base + threadIdx.x;
-    if (base + threadIdx.x < V && ((bmc[v >> 5] >> (v & 31)) & 1u)) {
+    if ((unsigned)v < (unsigned)V && ((bmc[v >> 5] >> (v & 31)) & 1u)) {  // v may pass INT_MAX
       const int beg = c.g.nindex[v];
       const int end = c.g.nindex[v + 1];
       const int du = c.dist[v];
@@ -1445,7 +1445,7 @@ __device__ __forceinline__ bool body_pull(const Ctx& c, H& S, Stage& s) {
     const int v = (int)base + threadIdx.x;
     bool improved = false;
     int best = kInf, dv = kInf, deg = 0;
-    if (base + threadIdx.x < V) {
+    if ((unsigned)v < (unsigned)V) {  // v may pass INT_MAX
       dv = c.dist[v];
       best = dv;
       if (!FRONTIER || dv > bound) {
@@ -1694,7 +1694,7 @@ __device__ __forceinline__ bool body_union(const Ctx& c, H& S, Stage& s) {
       const unsigned b = ni[v], e = ni[v + 1];
       int u[kAfforestLinks], pu[kAfforestLinks];
 #pragma unroll
-      for (int r = 0; r < kAfforestLinks; ++r) u[r] = b + r < e ? ld_adj(nl + (b + r)) : (int)v;
+      for (int r = 0; r < kAfforestLinks; ++r) u[r] = b + r < e ? ld_adj(nl + b + r) : (int)v;
       int pv = p[v];
 #pragma unroll
       for (int r = 0; r < kAfforestLinks; ++r) pu[r] = climb ? p[u[r]] : 0;
@@ -2034,7 +2034,9 @@ __device__ __forceinline__ bool body_mis(const Ctx& c, H& S, Stage& s) {
 // have to do (common.cuh); with the selector's network in it the pull kernels
 // took 69-78 registers and lost the fourth block per SM (BFS pull_frontier,
 // launched per iteration, us, before / with the network / FixedHead: RMAT-20
-// 1,132 / 1,464 / 1,059, grid 6000^2 83.7 / 108 / 81.8 ms).
+// 1,132 / 1,464 / 1,059, grid 6000^2 83.7 / 108 / 81.8 ms). pull_topo, whose time on
+// hubs is one thread's list, needs the 64 registers of the 4 blocks to issue its
+// loads together: left to itself the compiler takes 54 (RMAT-20 BFS 23.6 ms).
 template <int ALG, int VAR, class H>
 __global__ void __launch_bounds__(kBlock) relax_push(const __grid_constant__ Ctx c) {
   __shared__ Stage s;
