@@ -29,7 +29,11 @@ KernelFn relax_fn_of(int v) {
 template <int ALG>
 KernelFn relax_fn(int v, bool select, bool wide) {
   if (select) return relax_fn_of<ALG, SelectHead>(v);
-  if (v == kVPCta && wide) return relax_edge_balanced<ALG, FixedHead, true>;
+  // the wide form spills here; BFS, whose tiles do least, does not gain (RMAT-20,
+  // us, wide / not: BFS 297 / 285, SSSP 736 / 732, CC 521 / 547; RMAT-25 in degree
+  // order, ms: 8.4 / 8.2, 17.8 / 18.8, 22.2 / 24.3)
+  if constexpr (ALG != kBFS)
+    if (v == kVPCta && wide) return relax_edge_balanced<ALG, FixedHead, true>;
   return relax_fn_of<ALG, FixedHead>(v);
 }
 
