@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(kBlock) k_fill(Ctx c) {
   }
   for (long long base = (long long)blockIdx.x * kBlock; base < V; base += (long long)gridDim.x * kBlock) {
     const int v = (int)base + threadIdx.x;
-    const bool in = base + threadIdx.x < V;
+    const bool in = (unsigned)v < (unsigned)V;  // v may pass INT_MAX
     constexpr bool kAll = ALG == kCC || ALG == kMIS;  // every vertex starts in F_0
     const int deg = (kAll && in) ? c.g.nindex[v + 1] - c.g.nindex[v] : 0;
     // MIS: a vertex without neighbours is in the set at once
@@ -1027,8 +1027,8 @@ static int ensure_symmetry(i2_graph* g) {
 // Smallest graph (vertices) on which the selectors' union-find CC runs as
 // union-find's own kernel (run_traversal). The line was drawn before that kernel
 // chose its blocks by the graph's size; below it, us, own kernel / the selectors':
-// RMAT-20 145 / 168, ER 600,000 159 / 176, ER 2 x 10^6 199 / 200, grid 300^2 85 /
-// 135, 1000^2 135 / 141, 2000^2 231 / 268. It has not been moved.
+// RMAT-20 145 / 168, ER 600,000 159 / 176, ER 2 x 10^6 199 / 200, grid 300^2 116 /
+// 122, 1000^2 146 / 142, 2000^2 224 / 266. It has not been moved.
 constexpr long long kUnionFindKernelNodes = 1LL << 22;
 
 // Whether the learned selector picks styles here. Where it defers to the rule for
@@ -1072,19 +1072,21 @@ static bool wide_form(const i2_graph* g, int variant) {
 // Smaller sparse graphs would gain too (grid 2000^2 SSSP 4.47 / 4.31, BFS 1.71 /
 // 1.60); there the line is with the learned selector, which would then lose to the
 // rule on grids (its picks are from times at 5 blocks).
-// Union-find takes about one block per SM for every 2^11 vertices an SM has, 8
-// chunks a warp: more warps link trees that the others have not joined yet, and
-// meet at the same roots. us, 1 / 2 / 3 / 4 / 6 blocks: RMAT-17 110 / 122 / 153 /
+// Union-find on graphs of average degree 6 or more takes about one block per SM
+// for every 2^11 vertices an SM has, 8 chunks a warp: more warps link trees that the
+// others have not joined yet, and meet at the same roots. Sparser graphs have few
+// links at a time and keep every block (a caterpillar of 4 x 10^5 vertices 92, 125-168
+// by size). us, 1 / 2 / 3 / 4 / 6 blocks: RMAT-17 110 / 122 / 153 /
 // 193 / 204, RMAT-18 117 / 172 / 198 / 215 / 305, RMAT-20 171 / 140 / 144 / 168 /
 // 187, RMAT-22 473 / 295 / 235 / 213 / 186, ER 3 x 10^5 139 / 138 / 200 / 255 /
-// 371, 6 x 10^5 175 / 170 / 163 / 192 / 301, 2 x 10^6 304 / 219 / 200 / 192 / 195,
-// grid 300^2 121 / 108 / 112 / 134 / 116, 1000^2 223 / 159 / 136 / 149 / 146,
-// 2000^2 705 / 408 / 312 / 262 / 224.
+// 371, 6 x 10^5 175 / 170 / 163 / 192 / 301, 2 x 10^6 304 / 219 / 200 / 192 / 195;
+// grid 300^2 121 / 108 / 112 / 134 / 116, 2000^2 705 / 408 / 312 / 262 / 224.
 static int style_blocks(const i2_graph* g, int algo, int variant) {
   if (variant == kUnionFind) {
     const long long per_block = 8LL * kWarp * kWarpsPerBlock, sms = sm_count();
     const long long blocks = (g->g.nodes + per_block * sms / 2) / (per_block * sms);
-    return (int)std::min<long long>(std::max(1LL, blocks), std::min(g->blocks_per_sm, I2_UF_MIN_BLOCKS));
+    const long long most = std::min(g->blocks_per_sm, I2_UF_MIN_BLOCKS);
+    return (int)(g->gs.avgdeg < 6.f ? most : std::min(std::max(1LL, blocks), most));
   }
   const bool sparse = variant == kVPCta && (algo == I2_BFS || algo == I2_SSSP) && g->g.nodes >= (1 << 24) &&
                       g->gs.degcv <= 1.f && g->gs.avgdeg < 6.f;
